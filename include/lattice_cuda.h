@@ -511,6 +511,10 @@ LC_API int lc_lb_commit(lc_lb_key *key, const uint64_t *witness, uint32_t r, uin
 /* the same over host buffers, synchronous */
 LC_API int lc_lb_commit_host(lc_lb_key *key, const uint64_t *witness, uint32_t r, uint32_t *raw, int16_t *matrix,
                              uint32_t *batches);
+/* Wait for `stream` and report (and clear) a device-side error of this key's
+ * commitments (LC_ERR_TIMEOUT: a bounded wait expired; the outputs of that
+ * call are not valid).  lc_lb_commit_host reports it itself. */
+LC_API int lc_lb_key_check(lc_lb_key *key, lc_stream stream);
 /* random_elems (binfield.rs:177-189): n F162 elements [n][3] u64 into host memory */
 LC_API int lc_lb_random_elems(size_t n, uint64_t seed, uint64_t *out);
 

@@ -132,6 +132,7 @@ def _declare(L):
         "lc_lb_key_info": (i32, [P, P, P, P, P]),
         "lc_lb_ntt": (i32, [P, u32, P, P, sz, P]),
         "lc_lb_commit": (i32, [P, P, u32, P, P, P, P]),
+        "lc_lb_key_check": (i32, [P, P]),
         "lc_lb_commit_host": (i32, [P, P, u32, P, P, P]),
         "lc_lb_random_elems": (i32, [sz, C.c_uint64, P]),
     }

@@ -13,16 +13,16 @@
 // scalar.rs:229-243).  The raw commitment yc = y mod q is decomposed into four
 // R_162 slot elements (ring.rs:193-319).
 //
-// GPU mapping: one warp per lifted ring element (648 residues in shared
-// memory, __syncwarp between tree levels), grid (chunk split, chunk, limb);
-// each lane accumulates its 21 slots (11 leaf pairs) over the warp's ring
-// elements in u64 registers, the CTA sums its warps, and a finish kernel adds
-// the splits, reduces mod q and decomposes.  Every transform value is
-// canonical in [0, q) and every product is exact, so the results equal the
-// scalar reference bit for bit.
+// GPU mapping: the commitment transforms the binary elements on the INT8
+// tensor cores (lb_commit_kernel, below) and a finish kernel reduces the
+// column sums mod q and decomposes them; the general-input transform of the
+// key derivation runs one warp per ring element on the tree itself.  Every
+// transform value is reduced exactly and every product is exact, so the
+// results equal the scalar reference bit for bit.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -31,6 +31,7 @@
 #include "../../include/lattice_cuda.h"
 #include "common.cuh"
 #include "internal.h"
+#include "tcgen05.cuh"
 
 namespace lc {
 
@@ -38,9 +39,27 @@ constexpr int kLbN = 648, kLbN162 = 162, kLbQSlots = 324;
 constexpr int kLbCond = 1944, kLbCondQ = 972;
 constexpr int kLbTw = 326;  // twiddles of levels 1..6 of the split tree (2+4+8+24+72+216)
 constexpr int kLbWarps = 8;
-constexpr int kLbSlotsPerLane = (kLbN + 31) / 32;       // 21
-constexpr int kLbPairsPerLane = (kLbQSlots + 31) / 32;  // 11
-static_assert(2 * kLbPairsPerLane >= kLbSlotsPerLane, "accumulators");
+
+// Tensor-core transform of a binary ring element a = E(X^2) + X O(X^2): the
+// 324 leaves j of either kind of prime need E(g_j) and O(g_j) for one node
+// g_j -- a quadratic prime's leaf X^2 - g_j holds (E(g_j), O(g_j)) in slots
+// 2j, 2j + 1; a splitting prime's roots come in pairs +-w_j with w_j^2 = g_j
+// and values E(g_j) +- w_j O(g_j).
+constexpr int kLbLeaves = kLbQSlots;
+constexpr int kLbTiles = 3;            // leaf tiles, MMA M = 128 each
+constexpr int kLbTileLeaves = kLbLeaves / kLbTiles;  // 108: equal tiles keep the CTAs in step
+constexpr int kLbK = 352;              // K: 2 x 5 words x 32 bits, then the two elements' last 2 bits
+constexpr int kLbElems = 64;           // ring elements per tile; MMA N = 128 rows (E then O)
+constexpr int kLbImg = 128 * kLbK;     // one byte limb of one leaf tile; also one stage of digit rows
+constexpr uint32_t kLbStoreWeight = 7;  // a tile of the kept limb takes about 7/4 of another's (measured 5.7 and 2.9 k cycles before its
+                                        // reductions were cut)
+constexpr int kLbEpiWarps = 16, kLbProdWarps = 4;
+constexpr int kLbTcThreads = 32 * (kLbEpiWarps + kLbProdWarps + 1);
+constexpr int kLbOffB = 2 * kLbImg, kLbOffBar = kLbOffB + 2 * kLbImg;
+constexpr size_t kLbSmem = 1024 + kLbOffBar + 128;
+static_assert(kLbSmem <= 227 * 1024, "shared memory");
+// D = s32, A = B = u8, both K-major, N = 128, M = 128
+constexpr uint32_t kLbIdesc = (2u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 
 // Per-limb constants: Shoup pairs (w, floor(w 2^32 / q)) for every twiddle.
 struct LbLimb {
@@ -50,6 +69,9 @@ struct LbLimb {
   uint32_t leaf[kLbQSlots];                                // quadratic leaves: psi'^QUAD_SLOT_EXP[j]
   uint32_t dtw[4][kLbN162];                                // decomposition factors
   uint32_t i_root, inv2;
+  // per leaf of the tensor-core form: its node g_j, slots (first | second << 16) and w_j
+  // with its Shoup quotient (splitting primes) or g_j (quadratic primes)
+  uint32_t node[kLbLeaves], pair_slot[kLbLeaves], pair_w[kLbLeaves], pair_ws[kLbLeaves];
 };
 
 // Index maps shared by every prime (params.rs:88-97, ring.rs:68-99, params.rs:318-355).
@@ -67,10 +89,12 @@ struct lc_lb_key {
   uint32_t limbs = 0;
   std::vector<uint16_t> primes;
   std::vector<int16_t> a_host;  // centered rows [limbs][nr][648]
-  uint16_t* d_a = nullptr;      // canonical rows [limbs][nr][648]
+  uint32_t* d_a = nullptr;      // canonical rows by leaf [limbs][nr][324]: first slot | second << 16
   lc::LbLimb* d_limb = nullptr;
-  uint32_t* d_partial = nullptr;
-  size_t partial_bytes = 0;
+  uint8_t* d_img = nullptr;     // transform matrices [limbs][tile][byte limb][128 x 352]
+  uint32_t* d_sums = nullptr;   // column sums [limbs][r][648], zero between calls
+  size_t sums_bytes = 0;
+  uint32_t* d_err = nullptr;
   uint64_t* d_in = nullptr;  // host-API staging
   size_t in_bytes = 0;
   void* d_out = nullptr;
@@ -197,6 +221,33 @@ static void build_limb(uint32_t q, LbLimb& L) {
   }
 }
 
+// The leaves of the tensor-core form and their nodes g_j.
+static void build_pairs(uint32_t q, LbLimb& L) {
+  const bool quad = lb_is_quad(q);
+  const uint32_t psi = find_root(q, quad);
+  if (quad) {
+    for (int j = 0; j < kLbLeaves; ++j) {
+      L.node[j] = L.pair_w[j] = (uint32_t)lb_pow(psi, sub_exp(true, 6, j), q);
+      L.pair_slot[j] = (uint32_t)(2 * j) | (uint32_t)(2 * j + 1) << 16;
+    }
+    return;
+  }
+  // psi^972 = -1: slots whose exponents differ by 972 hold +-w_j
+  uint16_t slot_of[kLbCond] = {};
+  for (int j = 0; j < kLbN; ++j) slot_of[sub_exp(false, 7, j)] = (uint16_t)j;
+  int n = 0;
+  for (int j = 0; j < kLbN; ++j) {
+    const uint32_t e = sub_exp(false, 7, j);
+    const int partner = slot_of[(e + kLbCond / 2) % kLbCond];
+    if (partner < j) continue;  // seen from its partner
+    const uint32_t w = (uint32_t)lb_pow(psi, e, q);
+    L.node[n] = (uint32_t)((uint64_t)w * w % q);
+    L.pair_slot[n] = (uint32_t)j | (uint32_t)partner << 16;
+    L.pair_w[n] = w;
+    L.pair_ws[n++] = shoup32(w, q);
+  }
+}
+
 // c_lb_maps is constant memory of each device: uploaded once per device (one
 // bit per device; devices past 63 upload on every call).
 static std::mutex g_maps_mu;
@@ -255,14 +306,12 @@ LC_D void lb_level(uint32_t* v, const LbTw& T, uint32_t q, uint32_t om, uint32_t
 }
 
 // The whole forward transform of one ring element in warp-private shared
-// memory, canonical residues out.  Inputs are canonical; BINARY inputs
-// (0/1 coefficients) take the Phi_6 split's product a1 * zeta6 as a select.
-template <bool BINARY>
+// memory, canonical residues in and out.
 LC_D void lb_transform(uint32_t* v, const LbTw& T, const LbLimb& L, uint32_t lane) {
   const uint32_t q = L.q;
   for (int i = lane; i < 324; i += 32) {  // Phi_6 split: (a0 + t, a0 + a1 - t), t = zeta6 a1
     const uint32_t a0 = v[i], a1 = v[i + 324];
-    const uint32_t t = BINARY ? (a1 ? L.z6 : 0u) : lb_mulc(a1, L.z6, L.z6s, q);
+    const uint32_t t = lb_mulc(a1, L.z6, L.z6s, q);
     v[i] = a0 + t;
     v[i + 324] = a0 + a1 + 2 * q - t;
   }
@@ -290,115 +339,394 @@ LC_D void lb_transform(uint32_t* v, const LbTw& T, const LbLimb& L, uint32_t lan
   __syncwarp();
 }
 
+// The two byte limbs of the matrices of the three leaf tiles, in the operand's
+// shared-memory order (16-byte K chunk, row, byte).  Digit rows keep each bit
+// in place: K position 32 wd + 4 s + b holds bit 8b + s of 32-bit word wd, as
+// 0 or 2^s, so the matrix entry of coefficient y there is g^y 2^-s mod q.
+// Element h of a parity has the words 5h .. 5h + 4 and holds the coefficients
+// y = 2 m + h (m its bit); K step 10 has both elements' bits 160 and 161.
+__global__ void __launch_bounds__(256) lb_image_kernel(const LbLimb* limbs, uint8_t* img) {
+  const uint32_t e = blockIdx.x * 256 + threadIdx.x;  // position in one byte limb's image
+  const LbLimb& L = limbs[blockIdx.z];
+  const uint32_t q = L.q, kpos = e / 2048 * 16 + e % 16, row = e / 16 % 128;
+  const uint32_t wd = kpos / 32, s = kpos / 4 % 8, b = kpos % 4;
+  const uint32_t h = wd < 10 ? wd / 5 : b, m = wd < 10 ? 32 * (wd % 5) + 8 * b + s : 160 + s;
+  uint32_t v = 0;
+  if (row < (uint32_t)kLbTileLeaves && h < 2 && m < (uint32_t)kLbN162) {
+    uint32_t base = L.node[blockIdx.y * kLbTileLeaves + row];
+    v = 1;
+    for (uint32_t y = 2 * m + h; y; y >>= 1) {
+      if (y & 1) v = v * base % q;  // below 2^15 each
+      base = base * base % q;
+    }
+    for (uint32_t t = 0; t < s; ++t) v = (v & 1 ? v + q : v) / 2;
+  }
+  uint8_t* dst = img + ((size_t)blockIdx.z * kLbTiles + blockIdx.y) * 2 * kLbImg + e;
+  dst[0] = (uint8_t)v;
+  dst[kLbImg] = (uint8_t)(v >> 8);
+}
+
 struct LbCommitParams {
-  const uint64_t* witness;  // [r * len_f162][3]
-  const uint16_t* a;        // [limbs][nr][648] canonical
+  const uint64_t* witness;  // [r * nr][12]
+  const uint32_t* a;        // [limbs][nr][324] leaf pairs
   const LbLimb* limbs;
-  uint32_t* partial;        // [limbs][r][S][648]
+  const uint8_t* img;
+  uint32_t* sums;           // [limbs][r][648]
   uint32_t* batches;        // [r * nr][648] (limb 0) or null
-  uint32_t nr, splits, per_split, r;
-  size_t len_f162;
+  uint32_t* err;
+  uint32_t nr, r, total;    // total = r * nr ring elements
+  uint32_t tiles;           // of 64 ring elements
+  uint32_t runs0, per0;     // runs of limb 0's tiles, tiles in each
+  uint32_t runs, per;       // the other limbs'
 };
 
-__global__ void __launch_bounds__(kLbWarps * 32) lb_commit_kernel(const __grid_constant__ LbCommitParams p) {
-  __shared__ LbTw s_tw;
-  __shared__ uint32_t s_leaf[kLbQSlots];
-  __shared__ uint32_t s_v[kLbWarps][kLbN];
-  __shared__ uint64_t s_w[kLbWarps][12];
-  const uint32_t split = blockIdx.x, c = blockIdx.y, k = blockIdx.z;
-  const LbLimb& L = p.limbs[k];
-  const uint32_t q = L.q;
-  const bool quad = L.quad != 0;
-  for (int e = threadIdx.x; e < kLbTw; e += blockDim.x) {
-    s_tw.tw[e] = L.tw[e];
-    s_tw.tws[e] = L.tws[e];
-    s_tw.tw2[e] = L.tw2[e];
-    s_tw.tw2s[e] = L.tw2s[e];
-  }
-  if (quad)
-    for (int e = threadIdx.x; e < kLbQSlots; e += blockDim.x) s_leaf[e] = L.leaf[e];
-  __syncthreads();
-  const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  uint32_t* v = s_v[warp];
-  uint64_t* w = s_w[warp];
-  // 21 slots per lane (split limbs) or 11 leaf pairs = 22 sums (quadratic limbs)
-  uint64_t acc[2 * kLbPairsPerLane];
+// x mod q in [0, 2q) for any x < 2^32, bm = floor(2^32 / q)
+LC_D uint32_t lb_barrett(uint32_t x, uint32_t q, uint32_t bm) { return x - __umulhi(x, bm) * q; }
+LC_D uint32_t lb_canon(uint32_t x, uint32_t q, uint32_t bm) {
+  const uint32_t r = lb_barrett(x, q, bm);
+  return min(r, r - q);
+}
+// x mod q, canonical, for any x: three 24-bit digits, 2^24 == c24 < 2^15
+LC_D uint32_t lb_canon64(uint64_t x, uint32_t q, uint32_t bm, uint32_t c24) {
+  const uint32_t hi = lb_canon((uint32_t)(x >> 48) * c24 + ((uint32_t)(x >> 24) & 0xFFFFFFu), q, bm);
+  return lb_canon(hi * c24 + ((uint32_t)x & 0xFFFFFFu), q, bm);
+}
+
+// One epilogue warp: leaf 32 (warp & 3) + lane of the CTA's leaf tile, ring
+// elements 16 (warp >> 2) .. + 16 of every tile of the run, eight at a time.
+// STORE: this limb's transform is kept.
+template <bool QUAD, bool STORE, class Wait, class Release>
+LC_D void lb_epilogue(const LbCommitParams& p, const LbLimb& L, uint32_t k, uint32_t lt, uint32_t t0, uint32_t t1,
+                      uint32_t tmem, uint32_t warp, uint32_t lane, Wait&& wait, Release&& release) {
+  const uint32_t q = L.q, bm = 0xFFFFFFFFu / q, q2 = 2 * q, c24 = (1u << 24) % q;
+  const uint32_t quadrant = warp & 3, grp = warp >> 2;
+  const uint32_t leaf = lt * kLbTileLeaves + 32 * quadrant + lane;
+  const bool mine = 32 * quadrant + lane < (uint32_t)kLbTileLeaves;
+  const uint32_t slots = mine ? L.pair_slot[leaf] : 0, w = mine ? L.pair_w[leaf] : 0, ws = mine ? L.pair_ws[leaf] : 0;
+  const uint32_t s0 = slots & 0xFFFFu, s1 = slots >> 16;
+  const uint32_t* ak = p.a + (size_t)k * p.nr * kLbLeaves + (mine ? leaf : 0);
+  const uint32_t nr = p.nr, total = p.total;
+  // Sums over the column's elements.  STORE: of a0 x, a1 y (splitting) or a0 x,
+  // a1 y, a0 y + a1 x (quadratic) of the canonical slots.  Otherwise nothing is
+  // reduced per element: of a0 E, a1 O, a0 O, a1 E (E, O < 2^28, a < 2^15, at
+  // most 2^16 elements: below 2^59), and w and q come in at the flush.
+  uint64_t acc[4] = {};
+  uint32_t cur = 0;      // column of the pending sums
+  bool pending = false;  // warp-uniform
+  auto flush = [&]() {
+    uint32_t r[4];
 #pragma unroll
-  for (int j = 0; j < 2 * kLbPairsPerLane; ++j) acc[j] = 0;
-  const uint32_t i0 = split * p.per_split, i1 = min(p.nr, i0 + p.per_split);
-  const uint64_t* wc = p.witness + (size_t)c * p.len_f162 * 3;
-  const uint16_t* ak = p.a + (size_t)k * p.nr * kLbN;
-  for (uint32_t i = i0 + warp; i < i1; i += kLbWarps) {
-    if (lane < 12) w[lane] = wc[(size_t)12 * i + lane];  // elements 4i..4i+3, 3 words each
-    __syncwarp();
-    for (int x = lane; x < kLbN; x += 32) {  // coefficient 4m + kk = bit m of element 4i + kk
-      const int m = x >> 2, kk = x & 3;
-      v[x] = (uint32_t)(w[3 * kk + (m >> 6)] >> (m & 63)) & 1u;
+    for (int e = 0; e < 4; ++e) r[e] = lb_canon64(acc[e], q, bm, c24);
+    uint32_t r0 = r[0], r1 = r[1];
+    if (QUAD) {  // (a0 + a1 X)(x + y X) mod (X^2 - w)
+      r0 = lb_canon(r[0] + w * r[1], q, bm);
+      r1 = STORE ? r[2] : lb_canon(r[2] + r[3], q, bm);
+    } else if (!STORE) {  // a0 (E + w O) and a1 (E - w O)
+      r0 = lb_canon(r[0] + w * r[2], q, bm);
+      r1 = lb_canon(r[3] + w * (q - r[1]), q, bm);
     }
-    __syncwarp();
-    lb_transform<true>(v, s_tw, L, lane);
-    if (k == 0 && p.batches) {
-      uint32_t* dst = p.batches + ((size_t)c * p.nr + i) * kLbN;
-      for (int x = lane; x < kLbN; x += 32) dst[x] = v[x];
+    if (mine) {
+      uint32_t* dst = p.sums + ((size_t)k * p.r + cur) * kLbN;
+      atomicAdd(dst + s0, r0);
+      atomicAdd(dst + s1, r1);
     }
-    const uint16_t* arow = ak + (size_t)i * kLbN;
-    if (!quad) {
 #pragma unroll
-      for (int j = 0; j < kLbSlotsPerLane; ++j) {
-        const int u = lane + 32 * j;
-        if (u < kLbN) acc[j] += (uint64_t)__ldg(arow + u) * v[u];
+    for (int e = 0; e < 4; ++e) acc[e] = 0;
+    pending = false;
+  };
+  // adds elements [a, e) of the eight
+  auto mac = [&](const uint32_t (&kp)[8], const uint32_t (&x)[8], const uint32_t (&y)[8], uint32_t a, uint32_t e) {
+    uint32_t s0_ = 0, s1_ = 0;
+    uint64_t s2_ = 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const uint32_t pair = (uint32_t)u >= a && (uint32_t)u < e ? kp[u] : 0u;
+      const uint32_t a0 = pair & 0xFFFFu, a1 = pair >> 16;
+      if (STORE) {  // canonical: eight products stay below 8 * 19441^2 < 2^32
+        s0_ += a0 * x[u];
+        s1_ += a1 * y[u];
+        if (QUAD) s2_ += (uint64_t)(a0 * y[u]) + a1 * x[u];
+      } else {
+        acc[0] += (uint64_t)a0 * x[u];
+        acc[1] += (uint64_t)a1 * y[u];
+        acc[2] += (uint64_t)a0 * y[u];
+        acc[3] += (uint64_t)a1 * x[u];
       }
-    } else {
-      // leaf j: (a0 + a1 X)(b0 + b1 X) mod (X^2 - c_j), accumulated without reduction
+    }
+    if (STORE) {
+      acc[0] += s0_;
+      acc[1] += s1_;
+      acc[2] += s2_;
+    }
+  };
+  // Column and element of the first of each eight, advanced by a tile at a time.
+  const uint32_t step_c = kLbElems / nr, step_i = kLbElems % nr;
+  uint32_t col_of[2], at[2];
+  uint32_t kp[2][8];  // this tile's key pairs, loaded while the previous tile is processed
+  auto load_keys = [&](int h) {
+    uint32_t i = at[h];
+    if (i + 8 <= nr) {
+      const uint32_t* src = ak + (size_t)i * kLbLeaves;
 #pragma unroll
-      for (int j = 0; j < kLbPairsPerLane; ++j) {
-        const int s = lane + 32 * j;
-        if (s < kLbQSlots) {
-          const uint32_t a0 = __ldg(arow + 2 * s), a1 = __ldg(arow + 2 * s + 1);
-          const uint32_t b0 = v[2 * s], b1 = v[2 * s + 1];
-          acc[2 * j] += (uint64_t)a0 * b0 + (uint64_t)s_leaf[s] * (a1 * b1);
-          acc[2 * j + 1] += (uint64_t)a0 * b1 + (uint64_t)a1 * b0;
+      for (int u = 0; u < 8; ++u) kp[h][u] = __ldg(src + u * kLbLeaves);
+    } else {  // rows past the last column's are loaded and not used
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        kp[h][u] = __ldg(ak + (size_t)i * kLbLeaves);
+        i = i + 1 == nr ? 0 : i + 1;
+      }
+    }
+  };
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t f = t0 * kLbElems + 16 * grp + 8 * h;
+    col_of[h] = f / nr;
+    at[h] = f - col_of[h] * nr;
+    load_keys(h);
+  }
+  for (uint32_t t = t0; t < t1; ++t) {
+    const uint32_t buf = (t - t0) & 1;
+    if (!wait(t - t0)) break;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t f = t * kLbElems + 16 * grp + 8 * h;
+      const uint32_t lim = f < total ? min(8u, total - f) : 0u;
+      // E and O columns of the tile, low and high byte limb
+      uint32_t x[8], y[8], xh[8], yh[8];
+      const uint32_t col = tmem + ((32 * quadrant) << 16) + buf * 256 + 16 * grp + 8 * h;
+      tmem_ld8(col, x);
+      tmem_ld8(col + 64, y);
+      tmem_ld8(col + 128, xh);
+      tmem_ld8(col + 192, yh);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (h == 1) release(buf);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        x[u] += xh[u] << 8;
+        y[u] += yh[u] << 8;
+        if (STORE) {
+          x[u] = lb_barrett(x[u], q, bm);
+          if (!QUAD) {  // E +- w O in (0, 4q), two conditional subtractions
+            const uint32_t tw = lb_mulc(y[u], w, ws, q);
+            y[u] = x[u] + q2 - tw;
+            x[u] = x[u] + tw;
+            x[u] = min(x[u], x[u] - q2);
+            y[u] = min(y[u], y[u] - q2);
+          } else {
+            y[u] = lb_barrett(y[u], q, bm);
+          }
+          x[u] = min(x[u], x[u] - q);
+          y[u] = min(y[u], y[u] - q);
         }
       }
-    }
-    __syncwarp();
-  }
-  // CTA sum of the warps' accumulators, reduced mod q
-  __syncthreads();
-  if (!quad) {
+      if (STORE && mine) {
+        uint32_t* d0 = p.batches + (size_t)f * kLbN + s0;
+        uint32_t* d1 = p.batches + (size_t)f * kLbN + s1;
+        if (lim == 8) {
 #pragma unroll
-    for (int j = 0; j < kLbSlotsPerLane; ++j) {
-      const int u = lane + 32 * j;
-      if (u < kLbN) s_v[warp][u] = (uint32_t)(acc[j] % q);
-    }
-  } else {
+          for (int u = 0; u < 8; ++u) {
+            d0[u * kLbN] = x[u];
+            d1[u * kLbN] = y[u];
+          }
+        } else {
 #pragma unroll
-    for (int j = 0; j < kLbPairsPerLane; ++j) {
-      const int s = lane + 32 * j;
-      if (s < kLbQSlots) {
-        s_v[warp][2 * s] = (uint32_t)(acc[2 * j] % q);
-        s_v[warp][2 * s + 1] = (uint32_t)(acc[2 * j + 1] % q);
+          for (int u = 0; u < 8; ++u)
+            if ((uint32_t)u < lim) {
+              d0[u * kLbN] = x[u];
+              d1[u * kLbN] = y[u];
+            }
+        }
       }
+      // the eight elements column by column
+      uint32_t c = col_of[h], i = at[h], a = 0;
+      while (a < lim) {
+        const uint32_t e = a + min(lim - a, nr - i);
+        if (pending && c != cur) flush();
+        cur = c;
+        pending = true;
+        if (e - a == 8)
+          mac(kp[h], x, y, 0, 8);
+        else
+          mac(kp[h], x, y, a, e);
+        a = e;
+        i = 0;
+        ++c;
+      }
+      at[h] += step_i;
+      col_of[h] += step_c;
+      if (at[h] >= nr) {
+        at[h] -= nr;
+        ++col_of[h];
+      }
+      if (t + 1 < t1) load_keys(h);
     }
   }
+  if (pending) flush();
+}
+
+// The commitment of all columns under limb k and leaf tile blockIdx.y: a block
+// takes a run of tiles of 64 ring elements of the flat sequence (column,
+// element).  For every tile the two byte limbs of
+//   [E; O](g_j) = sum_y g_j^y [a_2y; a_2y+1]   (u8 x u8 -> s32, K = 352)
+// are exact: |D| <= 44 * 255 * 255 per byte limb (every shift s of the digit
+// rows fills an eighth of K), so low + 256 high < 2^28.  Warp roles: 0-15
+// reduce, store and multiply-accumulate (four per TMEM lane quadrant), 16-19
+// spread the witness bits into digit rows (one thread per row), 20 loads the
+// matrices, owns TMEM and issues the MMAs.  Two digit stages, two
+// accumulators; all waits bounded.
+//
+// As butterflies in shared memory the transform was issue-bound: 427 us for
+// 2^16 elements and two limbs with the base limb's transform kept.  Here a tile
+// is 22 MMAs, and the epilogue is what is left: 106 us (tensor pipe 34 %, issue
+// 51 %), against 27 us for the bytes of the kept transform.  A limb whose
+// transform is not kept skips the reductions per element, so the kept one gets
+// more of the blocks (kLbStoreWeight; equal shares took 138 us).
+__global__ void __launch_bounds__(kLbTcThreads, 1) lb_commit_kernel(const __grid_constant__ LbCommitParams p) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  unsigned char* base =
+      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base + kLbOffBar);
+  uint64_t* a_full = bars;         // matrices landed
+  uint64_t* b_full = bars + 1;     // [2] digit rows written (one arrival per producer warp)
+  uint64_t* b_empty = bars + 3;    // [2] MMAs of the stage done
+  uint64_t* acc_full = bars + 5;   // [2] accumulator complete
+  uint64_t* acc_empty = bars + 7;  // [2] accumulator read (one arrival per epilogue warp)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 10);
+
+  const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  // blocks: limb 0's runs, then the other limbs'
+  const bool first = blockIdx.x < p.runs0;
+  const uint32_t rest = first ? 0 : blockIdx.x - p.runs0;
+  const uint32_t lt = blockIdx.y, k = first ? 0 : 1 + rest / p.runs, per = first ? p.per0 : p.per;
+  const uint32_t t0 = (first ? blockIdx.x : rest % p.runs) * per, t1 = min(p.tiles, t0 + per);
+  const LbLimb& L = p.limbs[k];
+  if (tid == 0) {
+    mbar_init(a_full, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&b_full[s], kLbProdWarps);
+      mbar_init(&b_empty[s], 1);
+      mbar_init(&acc_full[s], 1);
+      mbar_init(&acc_empty[s], kLbEpiWarps);
+    }
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == kLbEpiWarps + kLbProdWarps) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc_fence_before();
   __syncthreads();
-  uint32_t* out = p.partial + (((size_t)k * p.r + c) * p.splits + split) * kLbN;
-  for (int u = threadIdx.x; u < kLbN; u += blockDim.x) {
-    uint32_t sum = 0;
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  auto fail = [&]() {
+    record_error(p.err, LC_DEVERR_TIMEOUT);
+    *abort_flag = 1;
+  };
+  int last_mma = -1;
+
+  if (warp < kLbEpiWarps) {
+    auto wait = [&](uint32_t it) -> bool {  // warp-uniform result: the TMEM loads are .sync.aligned
+      const bool ok = mbar_wait(&acc_full[it & 1], (it >> 1) & 1);
+      if (!ok) fail();
+      if (__any_sync(0xffffffffu, !ok || *abort_flag)) return false;
+      tc_fence_after();
+      return true;
+    };
+    auto release = [&](uint32_t buf) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[buf]);
+    };
+    const bool store = k == 0 && p.batches;
+    if (L.quad) {
+      if (store) lb_epilogue<true, true>(p, L, k, lt, t0, t1, tmem, warp, lane, wait, release);
+      else lb_epilogue<true, false>(p, L, k, lt, t0, t1, tmem, warp, lane, wait, release);
+    } else {
+      if (store) lb_epilogue<false, true>(p, L, k, lt, t0, t1, tmem, warp, lane, wait, release);
+      else lb_epilogue<false, false>(p, L, k, lt, t0, t1, tmem, warp, lane, wait, release);
+    }
+  } else if (warp < kLbEpiWarps + kLbProdWarps) {
+    // digit row: ring element row & 63 of the tile, parity row >> 6 (elements parity and parity + 2 of the four)
+    const uint32_t row = tid - 32 * kLbEpiWarps, parity = row >> 6;
+    for (uint32_t t = t0; t < t1; ++t) {
+      const uint32_t it = t - t0, f = t * kLbElems + (row & 63);
+      uint64_t wv[2][3] = {};
+      if (f < p.total) {
+        const uint64_t* src = p.witness + (size_t)f * 12 + 3 * parity;
 #pragma unroll
-    for (int ww = 0; ww < kLbWarps; ++ww) sum += s_v[ww][u];
-    out[u] = sum % q;
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int e = 0; e < 3; ++e) wv[h][e] = __ldg(src + 6 * h + e);
+      }
+      bool ok = it < 2 || mbar_wait(&b_empty[it & 1], ((it >> 1) - 1) & 1);
+      if (!ok) fail();
+      if (__any_sync(0xffffffffu, !ok || *abort_flag)) break;
+      uint4* dst = reinterpret_cast<uint4*>(base + kLbOffB + (it & 1) * kLbImg + row * 16);
+#pragma unroll
+      for (int wd = 0; wd < 10; ++wd) {
+        const uint64_t x64 = wv[wd / 5][(wd % 5) / 2];
+        const uint32_t x = (uint32_t)(((wd % 5) & 1) ? x64 >> 32 : x64);
+        const uint32_t m = 0x01010101u;
+        dst[(2 * wd) * 128] = make_uint4(x & m, x & (m << 1), x & (m << 2), x & (m << 3));
+        dst[(2 * wd + 1) * 128] = make_uint4(x & (m << 4), x & (m << 5), x & (m << 6), x & (m << 7));
+      }
+      const uint32_t z = ((uint32_t)(wv[0][2] >> 32) & 3u) | ((uint32_t)(wv[1][2] >> 32) & 3u) << 8;
+      dst[20 * 128] = make_uint4(z & 0x0101u, z & 0x0202u, 0u, 0u);
+      dst[21 * 128] = make_uint4(0u, 0u, 0u, 0u);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&b_full[it & 1]);
+    }
+  } else if (lane == 0) {
+    const uint8_t* src = p.img + ((size_t)k * kLbTiles + lt) * 2 * kLbImg;
+    mbar_arrive_expect_tx(a_full, 2 * kLbImg);
+    bulk_g2s(base, src, kLbImg, a_full);
+    bulk_g2s(base + kLbImg, src + kLbImg, kLbImg, a_full);
+    if (!mbar_wait(a_full, 0)) {
+      fail();
+      mbar_wait(a_full, 0);  // nothing may be in flight when shared memory goes
+    }
+    const uint32_t aa = smem_u32(base);
+    for (uint32_t t = t0; t < t1 && !*abort_flag; ++t) {
+      const uint32_t it = t - t0, s = it & 1;
+      if (!mbar_wait(&b_full[s], (it >> 1) & 1) || (it >= 2 && !mbar_wait(&acc_empty[s], ((it >> 1) - 1) & 1))) {
+        fail();
+        break;
+      }
+      tc_fence_after();
+      const uint32_t ba = smem_u32(base + kLbOffB + s * kLbImg);
+#pragma unroll
+      for (int l = 0; l < 2; ++l)
+#pragma unroll
+        for (int ks = 0; ks < kLbK / 32; ++ks)
+          mma_i8(tmem + s * 256 + l * 128, umma_desc_noswz(aa + l * kLbImg + ks * 4096, 2048, 128),
+                 umma_desc_noswz(ba + ks * 4096, 2048, 128), kLbIdesc, ks > 0 ? 1u : 0u);
+      mma_commit(&b_empty[s]);
+      mma_commit(&acc_full[s]);
+      last_mma = (int)it;
+    }
+    if (last_mma >= 0) mbar_wait(&acc_full[last_mma & 1], (last_mma >> 1) & 1);
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kLbEpiWarps + kLbProdWarps) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
   }
 }
 
 LC_D int16_t lb_center(uint32_t r, uint32_t q) { return r > (q - 1) / 2 ? (int16_t)((int32_t)r - (int32_t)q) : (int16_t)r; }
 
 struct LbFinishParams {
-  const uint32_t* partial;
+  uint32_t* sums;     // [limbs][r][648], read and zeroed for the next call
   const LbLimb* limbs;
   uint32_t* raw;      // [limbs][r][648]
   int16_t* matrix;    // [4][r][limbs][162]
-  uint32_t splits, r, nlimbs;
+  uint32_t r, nlimbs;
 };
 
 __global__ void __launch_bounds__(256) lb_finish_kernel(const __grid_constant__ LbFinishParams p) {
@@ -406,11 +734,10 @@ __global__ void __launch_bounds__(256) lb_finish_kernel(const __grid_constant__ 
   const uint32_t c = blockIdx.x, k = blockIdx.y;
   const LbLimb& L = p.limbs[k];
   const uint32_t q = L.q;
-  const uint32_t* part = p.partial + ((size_t)k * p.r + c) * p.splits * kLbN;
+  uint32_t* sums = p.sums + ((size_t)k * p.r + c) * kLbN;
   for (int u = threadIdx.x; u < kLbN; u += blockDim.x) {
-    uint64_t s = 0;
-    for (uint32_t sp = 0; sp < p.splits; ++sp) s += part[(size_t)sp * kLbN + u];
-    y[u] = (uint32_t)(s % q);
+    y[u] = sums[u] % q;
+    sums[u] = 0;
     p.raw[((size_t)k * p.r + c) * kLbN + u] = y[u];
   }
   __syncthreads();
@@ -457,7 +784,7 @@ __global__ void __launch_bounds__(kLbWarps * 32)
   for (size_t i = (size_t)blockIdx.x * kLbWarps + warp; i < count; i += (size_t)gridDim.x * kLbWarps) {
     for (int x = lane; x < kLbN; x += 32) v[x] = in[i * kLbN + x] % L.q;
     __syncwarp();
-    lb_transform<false>(v, s_tw, L, lane);
+    lb_transform(v, s_tw, L, lane);
     for (int x = lane; x < kLbN; x += 32) out[i * kLbN + x] = v[x];
     __syncwarp();
   }
@@ -485,25 +812,30 @@ struct LbRng {
   uint32_t below(uint32_t n) { return (uint32_t)(((next() >> 32) * n) >> 32); }
 };
 
-static int lb_key_finish(lc_lb_key* key) {
-  // canonical rows on the device
-  std::vector<uint16_t> canon(key->a_host.size());
+static int lb_key_finish(lc_lb_key* key, const std::vector<LbLimb>& tabs) {
+  // canonical rows on the device, one word per leaf
+  std::vector<uint32_t> canon((size_t)key->limbs * key->nr * kLbLeaves);
   for (uint32_t k = 0; k < key->limbs; ++k) {
     const int32_t q = key->primes[k];
-    for (size_t e = 0; e < key->nr * kLbN; ++e) {
-      const size_t idx = (size_t)k * key->nr * kLbN + e;
-      int32_t x = key->a_host[idx] % q;
-      canon[idx] = (uint16_t)(x < 0 ? x + q : x);
+    const uint32_t* ps = tabs[k].pair_slot;
+    for (size_t i = 0; i < key->nr; ++i) {
+      const int16_t* row = key->a_host.data() + ((size_t)k * key->nr + i) * kLbN;
+      uint32_t* out = canon.data() + ((size_t)k * key->nr + i) * kLbLeaves;
+      for (int j = 0; j < kLbLeaves; ++j) {
+        const int32_t x = row[ps[j] & 0xFFFF] % q, y = row[ps[j] >> 16] % q;
+        out[j] = (uint32_t)(x < 0 ? x + q : x) | (uint32_t)(y < 0 ? y + q : y) << 16;
+      }
     }
   }
-  if (cudaMalloc(&key->d_a, canon.size() * 2) != cudaSuccess) {
+  if (cudaMalloc(&key->d_a, canon.size() * 4) != cudaSuccess) {
     cudaGetLastError();
     return LC_ERR_OUT_OF_MEMORY;
   }
-  return map_cuda(cudaMemcpy(key->d_a, canon.data(), canon.size() * 2, cudaMemcpyHostToDevice));
+  return map_cuda(cudaMemcpy(key->d_a, canon.data(), canon.size() * 4, cudaMemcpyHostToDevice));
 }
 
-static int lb_key_alloc(size_t len_f162, const uint16_t* primes, uint32_t limbs, lc_lb_key** out) {
+static int lb_key_alloc(size_t len_f162, const uint16_t* primes, uint32_t limbs, std::vector<LbLimb>& tabs,
+                        lc_lb_key** out) {
   if (!out || !primes || limbs == 0 || limbs > 7) return LC_ERR_INVALID_ARGUMENT;
   *out = nullptr;
   // key.rs:96-100: len_f162 > 0 and a multiple of 4; no limb listed twice (:102-106)
@@ -522,14 +854,27 @@ static int lb_key_alloc(size_t len_f162, const uint16_t* primes, uint32_t limbs,
   key->nr = len_f162 / 4;
   key->limbs = limbs;
   key->primes.assign(primes, primes + limbs);
-  std::vector<LbLimb> tabs(limbs);
-  for (uint32_t k = 0; k < limbs; ++k) build_limb(primes[k], tabs[k]);
-  if (cudaMalloc(&key->d_limb, sizeof(LbLimb) * limbs) != cudaSuccess) {
+  tabs.resize(limbs);
+  // transform matrices, then the error word (zero)
+  const size_t per = (size_t)kLbTiles * 2 * kLbImg;
+  for (uint32_t k = 0; k < limbs; ++k) {
+    build_limb(primes[k], tabs[k]);
+    build_pairs(primes[k], tabs[k]);
+  }
+  if (cudaMalloc(&key->d_limb, sizeof(LbLimb) * limbs) != cudaSuccess ||
+      cudaMalloc(&key->d_img, limbs * per + 16) != cudaSuccess) {
     cudaGetLastError();
-    delete key;
+    lc_lb_key_destroy(key);
     return LC_ERR_OUT_OF_MEMORY;
   }
+  key->d_err = reinterpret_cast<uint32_t*>(key->d_img + limbs * per);
   rc = map_cuda(cudaMemcpy(key->d_limb, tabs.data(), sizeof(LbLimb) * limbs, cudaMemcpyHostToDevice));
+  if (!rc) {
+    lb_image_kernel<<<dim3(kLbImg / 256, kLbTiles, limbs), 256>>>(key->d_limb, key->d_img);
+    rc = map_cuda(cudaGetLastError());
+  }
+  if (!rc) rc = map_cuda(cudaMemset(key->d_err, 0, 4));  // after the kernel, on the same stream
+  if (!rc) rc = map_cuda(cudaStreamSynchronize(nullptr));
   if (rc) {
     lc_lb_key_destroy(key);
     return rc;
@@ -560,10 +905,11 @@ LC_API int lc_lb_key_create(size_t len_f162, const uint16_t* primes, uint32_t li
   using namespace lc;
   if (!a) return LC_ERR_INVALID_ARGUMENT;
   lc_lb_key* key = nullptr;
-  int rc = lb_key_alloc(len_f162, primes, limbs, &key);
+  std::vector<LbLimb> tabs;
+  int rc = lb_key_alloc(len_f162, primes, limbs, tabs, &key);
   if (rc) return rc;
   key->a_host.assign(a, a + (size_t)limbs * key->nr * kLbN);
-  rc = lb_key_finish(key);
+  rc = lb_key_finish(key, tabs);
   if (rc) {
     lc_lb_key_destroy(key);
     return rc;
@@ -579,7 +925,8 @@ LC_API int lc_lb_key_random(size_t len_f162, uint64_t seed, const uint16_t* prim
                             lc_lb_key** out) {
   using namespace lc;
   lc_lb_key* key = nullptr;
-  int rc = lb_key_alloc(len_f162, primes, limbs, &key);
+  std::vector<LbLimb> tabs;
+  int rc = lb_key_alloc(len_f162, primes, limbs, tabs, &key);
   if (rc) return rc;
   const size_t per = key->nr * kLbN;
   std::vector<uint32_t> coeffs(per), t(per);
@@ -602,7 +949,7 @@ LC_API int lc_lb_key_random(size_t len_f162, uint64_t seed, const uint16_t* prim
       key->a_host[(size_t)k * per + e] = (int16_t)((int32_t)t[e] > half ? (int32_t)t[e] - (int32_t)q : (int32_t)t[e]);
   }
   cudaFree(d_buf);
-  if (!rc) rc = lb_key_finish(key);
+  if (!rc) rc = lb_key_finish(key, tabs);
   if (rc) {
     lc_lb_key_destroy(key);
     return rc;
@@ -615,7 +962,8 @@ LC_API void lc_lb_key_destroy(lc_lb_key* key) {
   if (!key) return;
   cudaFree(key->d_a);
   cudaFree(key->d_limb);
-  cudaFree(key->d_partial);
+  cudaFree(key->d_img);
+  cudaFree(key->d_sums);
   cudaFree(key->d_in);
   cudaFree(key->d_out);
   delete key;
@@ -643,26 +991,55 @@ LC_API int lc_lb_commit(lc_lb_key* key, const uint64_t* witness, uint32_t r, uin
   if (!key || !witness || !raw || !matrix) return LC_ERR_INVALID_ARGUMENT;
   if (r < 2 || (r & (r - 1)) || r > (1u << 15)) return LC_ERR_INVALID_ARGUMENT;  // key.rs:388-391
   const uint32_t nr = (uint32_t)key->nr;
-  const int sms = std::max(1, device_sm_count());
-  // at least 16 CTAs per SM when the problem allows, about 8 ring elements per
-  // warp (64 per CTA), so the last wave is a small fraction of the launch
-  uint32_t splits = (uint32_t)std::max<size_t>(1, (size_t)16 * sms / ((size_t)r * key->limbs));
-  splits = std::max<uint32_t>(splits, nr / (8 * kLbWarps));
-  splits = std::min<uint32_t>(splits, std::max<uint32_t>(1, nr / kLbWarps));
-  // at most about 64 CTAs per SM in all: bounds the partial sums [limb][column][split][648]
-  splits = std::min<uint32_t>(splits, (uint32_t)std::max<size_t>(1, (size_t)64 * sms / ((size_t)r * key->limbs)));
-  const uint32_t per = (nr + splits - 1) / splits;
-  splits = (nr + per - 1) / per;
-  int rc = grow((void**)&key->d_partial, &key->partial_bytes, (size_t)key->limbs * r * splits * kLbN * 4);
-  if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  LbCommitParams p{witness, key->d_a, key->d_limb, key->d_partial, batches, nr, splits, per, r, key->len_f162};
-  lb_commit_kernel<<<dim3(splits, r, key->limbs), kLbWarps * 32, 0, st>>>(p);
-  rc = map_cuda(cudaGetLastError());
+  const size_t sums = (size_t)key->limbs * r * kLbN * 4;
+  if (sums > key->sums_bytes) {
+    int rc = grow((void**)&key->d_sums, &key->sums_bytes, sums);
+    if (!rc) rc = map_cuda(cudaMemsetAsync(key->d_sums, 0, sums, st));
+    if (rc) return rc;
+  }
+  static std::atomic<uint64_t> attr_done{0};
+  cudaError_t e = smem_attr_once(attr_done, lb_commit_kernel, kLbSmem);
+  if (e != cudaSuccess) return map_cuda(e);
+  LbCommitParams p{};
+  p.witness = witness;
+  p.a = key->d_a;
+  p.limbs = key->d_limb;
+  p.img = key->d_img;
+  p.sums = key->d_sums;
+  p.batches = batches;
+  p.err = key->d_err;
+  p.nr = nr;
+  p.r = r;
+  p.total = r * nr;  // at most 2^31
+  p.tiles = (p.total + kLbElems - 1) / kLbElems;
+  // One CTA per SM.  A tile of limb 0 counts kLbStoreWeight / 4 tiles of another
+  // limb when its transform is kept (reduced and stored per element).
+  const uint32_t w0 = batches ? kLbStoreWeight : 4, sms = (uint32_t)std::max(1, device_sm_count());
+  const uint32_t slots = std::max<uint32_t>(1, sms / kLbTiles), weight = w0 + 4 * (key->limbs - 1);
+  const auto cut = [&](uint32_t want, uint32_t* runs, uint32_t* per) {
+    *per = (p.tiles + std::max(1u, want) - 1) / std::max(1u, want);
+    *runs = (p.tiles + *per - 1) / *per;
+  };
+  cut((slots * w0 + weight / 2) / weight, &p.runs0, &p.per0);
+  cut(key->limbs > 1 ? (slots - std::min(slots, p.runs0)) / (key->limbs - 1) : 1, &p.runs, &p.per);
+  lb_commit_kernel<<<dim3(p.runs0 + p.runs * (key->limbs - 1), kLbTiles), kLbTcThreads, kLbSmem, st>>>(p);
+  int rc = map_cuda(cudaGetLastError());
   if (rc) return rc;
-  LbFinishParams f{key->d_partial, key->d_limb, raw, matrix, splits, r, key->limbs};
+  LbFinishParams f{key->d_sums, key->d_limb, raw, matrix, r, key->limbs};
   lb_finish_kernel<<<dim3(r, key->limbs), 256, 0, st>>>(f);
   return map_cuda(cudaGetLastError());
+}
+
+LC_API int lc_lb_key_check(lc_lb_key* key, lc_stream stream) {
+  using namespace lc;
+  if (!key) return LC_ERR_INVALID_ARGUMENT;
+  cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
+  uint32_t flag = 0;
+  if (e == cudaSuccess) e = cudaMemcpy(&flag, key->d_err, 4, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess && flag) e = cudaMemset(key->d_err, 0, 4);
+  if (e != cudaSuccess) return map_cuda(e);
+  return flag ? LC_ERR_TIMEOUT : LC_OK;
 }
 
 // Host buffers: witness [r * len_f162][3] u64 in, raw / matrix / batches out
@@ -686,7 +1063,7 @@ LC_API int lc_lb_commit_host(lc_lb_key* key, const uint64_t* witness, uint32_t r
   if (!rc) rc = map_cuda(cudaMemcpy(raw, o, raw_b, cudaMemcpyDeviceToHost));
   if (!rc) rc = map_cuda(cudaMemcpy(matrix, o + raw_b, mat_b, cudaMemcpyDeviceToHost));
   if (!rc && batches) rc = map_cuda(cudaMemcpy(batches, o + raw_b + mat_b, bat_b, cudaMemcpyDeviceToHost));
-  return rc;
+  return rc ? rc : lc_lb_key_check(key, nullptr);
 }
 
 // random_elems (binfield.rs:186-189): n uniform F162 elements as [n][3] u64 (host)

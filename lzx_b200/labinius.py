@@ -160,6 +160,12 @@ class CommitmentKey:
         check(_lib.lib().lc_lb_key_info(self._h, None, None, None, out.ctypes.data_as(C.c_void_p)), "lc_lb_key_info")
         return out
 
+    def check(self):
+        """``lc_lb_key_check``: wait for the current stream, report a device-side error."""
+        import torch
+        check(_lib.lib().lc_lb_key_check(self._h, C.c_void_p(torch.cuda.current_stream().cuda_stream)),
+              "lc_lb_key_check")
+
     def commit(self, witness, r: int, batches: bool = True):
         """``CommitmentKey::commit`` (key.rs:223-231): (CommitmentMatrix, AuxData)."""
         limbs, nr = self.limbs(), self.len_ring()

@@ -76,6 +76,26 @@ def test_commit_matches_oracle(limbs, len_f162, r):
     assert np.array_equal(dcm.value.cpu().numpy(), mat)
 
 
+@pytest.mark.parametrize("limbs", [[Modulus.Q3889_FS_S], [Modulus.Q4861_Q_S], list(Modulus)],
+                         ids=["split", "quadratic", "all"])
+@pytest.mark.parametrize("nr,r", [(1, 64), (15, 16), (16, 8), (63, 2), (64, 2), (65, 4), (100, 64)])
+def test_commit_tile_edges(limbs, nr, r):
+    """Columns that end inside a 16-element group, a 64-element tile or a run of
+    tiles; the second call on the key (other column count) starts from its
+    cleared sums."""
+    primes = [m.prime() for m in limbs]
+    key = CommitmentKey.random(4 * nr, 3 + nr, limbs[0], limbs[1:])
+    for cols in (r, 2):
+        w = random_witness(cols * 4 * nr, 17 + cols)
+        w[:, 2] |= np.uint64(0xF) << np.uint64(34)  # bits past the 162 of an element are not read
+        raw, mat, bat = lb.commit(key.a, primes, 4 * nr, w & np.array([2**64 - 1, 2**64 - 1, 2**34 - 1], np.uint64), cols)
+        cm, aux = key.commit(torch.from_numpy(w.view(np.int64)).cuda(), cols)
+        key.check()
+        assert np.array_equal(aux.raw.cpu().numpy().view(np.uint32), raw)
+        assert np.array_equal(cm.value.cpu().numpy(), mat)
+        assert np.array_equal(aux.batches.cpu().numpy().view(np.uint32), bat)
+
+
 def test_commit_suite_shape_sizexs():
     """suite sizexs (scheme.rs:91-99): 2^14 F162 in 16 columns, moduli 3889 + 2917."""
     limbs = [Modulus.Q3889_FS_S, Modulus.Q2917_Q_S]
