@@ -8,18 +8,28 @@
 // (lo = (lo'+hi')/2, hi = (lo'-hi')/(2w)), and a ring product is the slotwise
 // Karatsuba (u0 + u1 X)(v0 + v1 X) mod (X^2 - gamma) between two transforms.
 //
-// GPU layout: polynomials are contiguous [count][n] u64 residues.  A warp
-// owns 32/G polynomials (G = min(32, n/2) lanes per polynomial) staged in
-// shared memory; every level is one butterfly (or one slot) per lane per
-// n/(2G), separated by __syncwarp.
+// GPU layout: polynomials are contiguous [count][n] u64 residues.  T = n/V
+// lanes own one polynomial, V = min(16, n) values each, in registers.  Phase 0
+// holds elements t + T r: the levels whose pairs are at least T apart.  The
+// values change hands once, through a padded copy in the warp's shared memory,
+// and phase 1 holds V consecutive elements: the remaining levels and the
+// quadratic slots.  The inverse runs the same way back.
 //
-// Arithmetic: residues below q < 2^50 are exact doubles, so a modular
-// product runs on the FP64 pipe -- h = RN(ab), the exact remainder
-// l = fma(a, b, -h), a quotient c = the integer nearest h*(1/q) (one fma
-// into the 1.5*2^52 rounding constant), and r = fma(-c, q, h) + l, which is
-// exact and lies in (-q, q): |c - ab/q| <= 1/2 + 1/8 + 1/8 because
-// |l| <= 2^46 and q > 2^49.  One conditional add of q makes it canonical, so
-// every output equals the reference's u64 arithmetic bit for bit.
+// Arithmetic: values are doubles that hold integers, lazily in (-8q, 8q),
+// 8q < 2^53, so sums and differences are exact.  A product with a constant w,
+// kept centered (|w| <= q/2) with wq = RN(w/q), is
+//   h = RN(aw), l = fma(a, w, -h) (so h + l = aw exactly),
+//   c = fma(a, wq, M) - M (M = 1.5 * 2^52: the integer nearest a wq),
+//   r = fma(-c, q, h) + l = aw - cq exactly,
+// with |r| <= q/2 + |a|/16 for |a| <= 4q (|a wq| <= 2^51).  Larger |a| take
+// M = 1.5 * 2^53, which rounds to even integers: |r| <= q + |a|/16.  A forward
+// butterfly (lo + r, lo - r) raises the bound on its values by |r|, and the at
+// most six levels need no reduction: inputs below q reach 4.2 q after five and
+// stay below 5.5 q.  In the inverse every second level, and the one before the
+// last, reduces its sums: c = fma(x, 1/q, M) - M,
+// fma(-c, q, x), at most q/2.  The factors 1/2 of all levels are one factor in
+// the last level's constants.  Outputs become canonical as integers, so every
+// output equals the reference's u64 arithmetic bit for bit.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,18 +41,24 @@
 
 namespace lc {
 
-// Table layout (entries): forward twiddles of level d (2^d blocks) at
-// 2^d - 1, then the inverse constants inv2 * w^-1 at kQ50Inv + 2^d - 1, the
-// leaf gammas at kQ50Gamma, and inv2 at kQ50Inv2.
-constexpr int kQ50Inv = 64, kQ50Gamma = 128, kQ50Inv2 = 192, kQ50Tab = 193;
+struct Q50Const {
+  double w, wq;  // centered constant, RN(w / q)
+};
+
+// Table on the device (entries; copied into shared memory): phase-1 constants
+// of the forward levels, of the inverse levels, then the leaf gammas.
+constexpr int kQ50P1 = 48, kQ50Tab = 2 * kQ50P1 + 64;
 
 }  // namespace lc
 
 struct lc_quad50_plan {
   uint64_t q = 0, zeta = 0, generator = 0;
   uint32_t two_adicity = 0, log_n = 0;
-  uint64_t tab[lc::kQ50Tab] = {};
-  double* d_tab = nullptr;
+  uint64_t gamma[64] = {};
+  // phase-0 constants: level d's block i at 2^d - 1 + i; the inverse's entry 0
+  // and ninv carry the factor 2^-(levels)
+  lc::Q50Const fwd0[15] = {}, inv0[15] = {}, ninv = {};
+  lc::Q50Const* d_tab = nullptr;
   lc::HostPipeline staging;
 };
 
@@ -58,208 +74,269 @@ struct Q50Params {
   uint64_t* out;
   size_t count;
   double q, qinv;  // qinv = RN(1/q)
-  const double* tab;
+  uint64_t qi;
+  const Q50Const* tab;
+  Q50Const fwd0[15], inv0[15], ninv;  // uniform constants, read from the parameter bank
 };
 
-constexpr double kRound52 = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds [0, 2^51) to integers
+constexpr double kRound52 = 6755399441055744.0;   // 1.5 * 2^52
+constexpr double kRound53 = 13510798882111488.0;  // 1.5 * 2^53
 
-LC_D double q50_add(double a, double b, double q) {
-  const double s = __dadd_rn(a, b);
-  return s >= q ? __dadd_rn(s, -q) : s;
+LC_D double q50_load(uint64_t x) {  // exact for x < 2^52
+  return __dadd_rn(__longlong_as_double((long long)(x | 0x4330000000000000ull)), -4503599627370496.0);
 }
 
-LC_D double q50_sub(double a, double b, double q) {
-  const double d = __dadd_rn(a, -b);
-  return d < 0.0 ? __dadd_rn(d, q) : d;
+// the canonical residue of an integer in [-q, q)
+LC_D uint64_t q50_store(double r, uint64_t qi) {
+  const int64_t v = __double_as_longlong(__dadd_rn(r, kRound52)) - 0x4338000000000000ll;
+  return (uint64_t)(v + ((v >> 63) & (int64_t)qi));
 }
 
-// a * b mod q for residues a, b < q, 2^49 < q < 2^50
+template <bool BIG = false>  // |a| up to 8q
+LC_D double q50_mulw(double a, Q50Const w, double q) {
+  constexpr double M = BIG ? kRound53 : kRound52;
+  const double h = __dmul_rn(a, w.w);
+  const double l = __fma_rn(a, w.w, -h);
+  const double c = __dadd_rn(__fma_rn(a, w.wq, M), -M);
+  return __dadd_rn(__fma_rn(-c, q, h), l);
+}
+
+// a * b for |a|, |b| <= q: |r| <= 3q/4 (the quotient of h = RN(ab) is off by at most 1/4 before rounding)
 LC_D double q50_mul(double a, double b, double q, double qinv) {
   const double h = __dmul_rn(a, b);
   const double l = __fma_rn(a, b, -h);
   const double c = __dadd_rn(__fma_rn(h, qinv, kRound52), -kRound52);
-  const double r = __dadd_rn(__fma_rn(-c, q, h), l);
-  return r < 0.0 ? __dadd_rn(r, q) : r;
+  return __dadd_rn(__fma_rn(-c, q, h), l);
+}
+
+LC_D double q50_red(double x, double q, double qinv) {  // |x| < 2^53 to [-q/2, q/2]
+  const double c = __dadd_rn(__fma_rn(x, qinv, kRound52), -kRound52);
+  return __fma_rn(-c, q, x);
 }
 
 template <int LOG_N>
 struct Q50Geo {
   static constexpr int N = 1 << LOG_N;
-  static constexpr int HALF = N / 2;                // butterflies per level = quadratic slots
-  static constexpr int G = HALF < 32 ? HALF : 32;   // lanes per polynomial
-  static constexpr int PW = 32 / G;                 // polynomials per warp
-  static constexpr int BPT = HALF / G;              // butterflies (slots) per lane
-  static constexpr int WE = PW * N;                 // elements per warp
+  static constexpr int LOG_V = LOG_N < 4 ? LOG_N : 4, V = 1 << LOG_V;
+  static constexpr int LOG_T = LOG_N - LOG_V, T = 1 << LOG_T;  // lanes per polynomial
+  static constexpr int PW = 32 / T;                            // polynomials per warp
+  static constexpr int WE = PW * N;                            // elements per warp (32 V)
+  static constexpr int LEVELS = LOG_N - 1;
+  static constexpr int LOW0 = LOG_T > 1 ? LOG_T : 1;  // phase 0: pair bits LOG_N - 1 .. LOW0
+  // phase-1 constants of pair bit b: entry [j][t], j < V >> (b + 1)
+  LC_HD static constexpr int p1_off(int b) {
+    int off = 0;
+    for (int bb = LOG_T - 1; bb > b; --bb) off += (V >> (bb + 1)) * T;
+    return off;
+  }
+  // one pad word per 16: both sides of the exchange are free of bank conflicts
+  LC_HD static constexpr int pad(int e) { return e + (e >> 4); }
+  static constexpr int SLOT = WE + WE / 16 + 1;
 };
 
-// Register levels: lane l holds elements l + 32 r (r < E) of its warp's
-// region.  For n >= 64 the DIF levels whose half span is at least 32 pair
-// elements of one lane, with a twiddle that depends on r only.
+// phase 0 of the forward transform: v[r] = element t + T r
 template <int LOG_N>
-struct Q50Reg {
-  static constexpr int E = Q50Geo<LOG_N>::WE / 32;         // elements per lane
-  static constexpr int LEVELS = LOG_N >= 6 ? LOG_N - 5 : 0;  // forward d < LEVELS, inverse likewise
+LC_D void q50_forward0(double (&v)[Q50Geo<LOG_N>::V], const Q50Params& p) {
+  using Q = Q50Geo<LOG_N>;
+#pragma unroll
+  for (int b = LOG_N - 1; b >= Q::LOW0; --b) {
+    const int d = LOG_N - 1 - b, hr = 1 << (b - Q::LOG_T);
+#pragma unroll
+    for (int r = 0; r < Q::V; ++r) {
+      if (r & hr) continue;
+      const double t = q50_mulw(v[r + hr], p.fwd0[(1 << d) - 1 + (r >> (b + 1 - Q::LOG_T))], p.q);
+      v[r + hr] = __dadd_rn(v[r], -t);
+      v[r] = __dadd_rn(v[r], t);
+    }
+  }
+}
+
+// phase 1: v[r] = element V t + r
+template <int LOG_N, int B>
+LC_D void q50_forward1(double (&v)[Q50Geo<LOG_N>::V], const Q50Const* tab, uint32_t t, double q) {
+  using Q = Q50Geo<LOG_N>;
+  if constexpr (B >= 1) {
+    constexpr int hr = 1 << B;
+#pragma unroll
+    for (int r = 0; r < Q::V; ++r) {
+      if (r & hr) continue;
+      const double x = q50_mulw<LOG_N - 1 - B == 5>(v[r + hr], tab[Q::p1_off(B) + (r >> (B + 1)) * Q::T + t], q);
+      v[r + hr] = __dadd_rn(v[r], -x);
+      v[r] = __dadd_rn(v[r], x);
+    }
+    q50_forward1<LOG_N, B - 1>(v, tab, t, q);
+  }
+}
+
+// Inverse butterflies of pair bit B (level number B: 1 is the first).  Inputs are
+// below 2q; bounds in q of (sums, products) after the levels of n = 128: 4, 0.75;
+// 0.5 (from 8), 1.5; 3, 0.7; 0.5 (from 6), 1.4; 0.5 (from 2.8), 0.7; 0.6, 0.6.
+template <int LOG_N, int B>
+struct Q50Inv {
+  static constexpr bool kLast = B == LOG_N - 1;
+  static constexpr bool kReduce = !kLast && (B % 2 == 0 || B == LOG_N - 2);
+  static constexpr bool kBig = !kLast && B % 2 == 0;
 };
 
-template <int LOG_N>
-LC_D void q50_forward_regs(double (&v)[Q50Reg<LOG_N>::E], const double* tab, double q, double qinv) {
-  constexpr int E = Q50Reg<LOG_N>::E;
+template <int LOG_N, int B>
+LC_D void q50_inv_pair(double& lo, double& hi, Q50Const w, const Q50Params& p) {
+  const double s = __dadd_rn(lo, hi), d = __dadd_rn(lo, -hi);
+  hi = q50_mulw<Q50Inv<LOG_N, B>::kBig>(d, w, p.q);
+  if constexpr (Q50Inv<LOG_N, B>::kLast)
+    lo = q50_mulw(s, p.ninv, p.q);
+  else
+    lo = Q50Inv<LOG_N, B>::kReduce ? q50_red(s, p.q, p.qinv) : s;
+}
+
+template <int LOG_N, int B>
+LC_D void q50_inverse1(double (&v)[Q50Geo<LOG_N>::V], const Q50Const* tab, uint32_t t, const Q50Params& p) {
+  using Q = Q50Geo<LOG_N>;
+  if constexpr (B < Q::LOW0) {
 #pragma unroll
-  for (int d = 0; d < Q50Reg<LOG_N>::LEVELS; ++d) {
-    const int hr = (1 << (LOG_N - 1 - d)) / 32;  // register distance of the pair
+    for (int r = 0; r < Q::V; ++r) {
+      if (r & (1 << B)) continue;
+      q50_inv_pair<LOG_N, B>(v[r], v[r + (1 << B)], tab[kQ50P1 + Q::p1_off(B) + (r >> (B + 1)) * Q::T + t], p);
+    }
+    q50_inverse1<LOG_N, B + 1>(v, tab, t, p);
+  }
+}
+
+template <int LOG_N, int B>
+LC_D void q50_inverse0(double (&v)[Q50Geo<LOG_N>::V], const Q50Params& p) {
+  using Q = Q50Geo<LOG_N>;
+  if constexpr (B < LOG_N) {
+    constexpr int d = LOG_N - 1 - B, hr = 1 << (B - Q::LOG_T);
 #pragma unroll
-    for (int r = 0; r < E; ++r) {
+    for (int r = 0; r < Q::V; ++r) {
       if (r & hr) continue;
-      const double t = q50_mul(v[r + hr], tab[(1 << d) - 1 + r / (2 * hr)], q, qinv);
-      const double L = v[r];
-      v[r] = q50_add(L, t, q);
-      v[r + hr] = q50_sub(L, t, q);
+      q50_inv_pair<LOG_N, B>(v[r], v[r + hr], p.inv0[(1 << d) - 1 + (r >> (B + 1 - Q::LOG_T))], p);
     }
+    q50_inverse0<LOG_N, B + 1>(v, p);
   }
 }
 
+// u <- u (*) v slotwise, (u0 + u1 X)(v0 + v1 X) mod (X^2 - gamma_p): at most 2q
 template <int LOG_N>
-LC_D void q50_inverse_regs(double (&v)[Q50Reg<LOG_N>::E], const double* tab, double q, double qinv) {
-  constexpr int E = Q50Reg<LOG_N>::E;
-  const double inv2 = tab[kQ50Inv2];
-#pragma unroll
-  for (int d = Q50Reg<LOG_N>::LEVELS - 1; d >= 0; --d) {
-    const int hr = (1 << (LOG_N - 1 - d)) / 32;
-#pragma unroll
-    for (int r = 0; r < E; ++r) {
-      if (r & hr) continue;
-      const double L = v[r], H = v[r + hr];
-      v[r] = q50_mul(q50_add(L, H, q), inv2, q, qinv);
-      v[r + hr] = q50_mul(q50_sub(L, H, q), tab[kQ50Inv + (1 << d) - 1 + r / (2 * hr)], q, qinv);
-    }
-  }
-}
-
-// Shared-memory levels d in [Q50Reg::LEVELS, LOG_N - 1) of NX polynomials
-// (one per operand) of this lane's group, interleaved for independent work.
-template <int LOG_N, int NX>
-LC_D void q50_forward_smem(double* const (&x)[NX], const double* tab, uint32_t g, double q, double qinv) {
+LC_D void q50_slotwise(double (&u)[Q50Geo<LOG_N>::V], double (&v)[Q50Geo<LOG_N>::V], const Q50Const* tab, uint32_t t,
+                       const Q50Params& p) {
   using Q = Q50Geo<LOG_N>;
 #pragma unroll
-  for (int d = Q50Reg<LOG_N>::LEVELS; d + 1 < LOG_N; ++d) {
-    const int hb = LOG_N - 1 - d;  // log2 of the half span
-#pragma unroll
-    for (int r = 0; r < Q::BPT; ++r) {
-      const uint32_t u = g + Q::G * r;
-      const uint32_t i = u >> hb, j = u & ((1u << hb) - 1);
-      const uint32_t lo = (i << (hb + 1)) + j, hi = lo + (1u << hb);
-      const double w = tab[(1u << d) - 1 + i];
-#pragma unroll
-      for (int k = 0; k < NX; ++k) {
-        const double L = x[k][lo];
-        const double t = q50_mul(x[k][hi], w, q, qinv);
-        x[k][lo] = q50_add(L, t, q);
-        x[k][hi] = q50_sub(L, t, q);
-      }
-    }
-    __syncwarp();
+  for (int s = 0; s < Q::V / 2; ++s) {
+    const double u0 = q50_red(u[2 * s], p.q, p.qinv), u1 = q50_red(u[2 * s + 1], p.q, p.qinv);
+    const double v0 = q50_red(v[2 * s], p.q, p.qinv), v1 = q50_red(v[2 * s + 1], p.q, p.qinv);
+    const double p0 = q50_mul(u0, v0, p.q, p.qinv);
+    const double p1 = q50_mul(u1, v1, p.q, p.qinv);
+    const double cross = q50_mul(__dadd_rn(u0, u1), __dadd_rn(v0, v1), p.q, p.qinv);
+    u[2 * s] = __dadd_rn(p0, q50_mulw(p1, tab[2 * kQ50P1 + s * Q::T + t], p.q));
+    u[2 * s + 1] = __dadd_rn(cross, -__dadd_rn(p0, p1));
   }
 }
 
-template <int LOG_N>
-LC_D void q50_inverse_smem(double* x, const double* tab, uint32_t g, double q, double qinv) {
-  using Q = Q50Geo<LOG_N>;
-  const double inv2 = tab[kQ50Inv2];
-#pragma unroll
-  for (int d = LOG_N - 2; d >= Q50Reg<LOG_N>::LEVELS; --d) {
-    const int hb = LOG_N - 1 - d;
-#pragma unroll
-    for (int r = 0; r < Q::BPT; ++r) {
-      const uint32_t u = g + Q::G * r;
-      const uint32_t i = u >> hb, j = u & ((1u << hb) - 1);
-      const uint32_t lo = (i << (hb + 1)) + j, hi = lo + (1u << hb);
-      const double L = x[lo], H = x[hi];
-      x[lo] = q50_mul(q50_add(L, H, q), inv2, q, qinv);
-      x[hi] = q50_mul(q50_sub(L, H, q), tab[kQ50Inv + (1u << d) - 1 + i], q, qinv);
-    }
-    __syncwarp();
-  }
-}
+// Bound: FP64 issue.  A product at n = 128 is about 13 k FP64 operations (22 k
+// with a conditional correction after every sum and product and two constants
+// per inverse butterfly); 2^20 of them take 1.09 ms (1.97 ms before), 0.70 of the
+// pipe.  16 values per lane need 128 registers, so 16 warps per SM; fetching the
+// next task into registers instead of L2 spills (1.23 ms), no prefetch: 1.17 ms.
+constexpr int kQ50Warps = 4, kQ50Ctas = 4;
 
-// x <- x (*) y slotwise: (u0 + u1 X)(v0 + v1 X) mod (X^2 - gamma_p)
-template <int LOG_N>
-LC_D void q50_slotwise(double* x, const double* y, const double* tab, uint32_t g, double q, double qinv) {
-  using Q = Q50Geo<LOG_N>;
-#pragma unroll
-  for (int r = 0; r < Q::BPT; ++r) {
-    const uint32_t p = g + Q::G * r;
-    const double u0 = x[2 * p], u1 = x[2 * p + 1], v0 = y[2 * p], v1 = y[2 * p + 1];
-    const double p0 = q50_mul(u0, v0, q, qinv);
-    const double p1 = q50_mul(u1, v1, q, qinv);
-    const double cross = q50_mul(q50_add(u0, u1, q), q50_add(v0, v1, q), q, qinv);
-    x[2 * p] = q50_add(p0, q50_mul(p1, tab[kQ50Gamma + p], q, qinv), q);
-    x[2 * p + 1] = q50_sub(cross, q50_add(p0, p1, q), q);
-  }
-  __syncwarp();
-}
-
-constexpr int kQ50Warps = 8;
-
-// five CTAs per SM (48 registers, no spills): the kernel is latency-bound at four
 template <int LOG_N, int OP>
-__global__ void __launch_bounds__(kQ50Warps * 32, 5) quad50_kernel(const __grid_constant__ Q50Params p) {
+__global__ void __launch_bounds__(kQ50Warps * 32, kQ50Ctas) quad50_kernel(const __grid_constant__ Q50Params p) {
   using Q = Q50Geo<LOG_N>;
-  constexpr int E = Q50Reg<LOG_N>::E;
+  constexpr int V = Q::V, T = Q::T;
   constexpr bool TWO = OP == kQ50Slot || OP == kQ50Mul;
-  __shared__ double s_tab[kQ50Tab];
-  __shared__ __align__(16) double s_a[kQ50Warps][Q::WE];
-  __shared__ __align__(16) double s_b[kQ50Warps][TWO ? Q::WE : 1];
+  // which layout the operands arrive and the results leave in: 0 = t + T r, 1 = V t + r
+  constexpr bool IN0 = OP == kQ50Fwd || OP == kQ50Mul, OUT0 = OP == kQ50Inv_ || OP == kQ50Mul;
+  __shared__ Q50Const s_tab[kQ50Tab];
+  __shared__ double s_x[kQ50Warps][Q::SLOT];
   for (int e = threadIdx.x; e < kQ50Tab; e += blockDim.x) s_tab[e] = p.tab[e];
   __syncthreads();
   const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const uint32_t g = lane % Q::G, poly = lane / Q::G;
+  const uint32_t t = lane % T, poly = lane / T;
   const size_t total = p.count * Q::N;
   const size_t tasks = (p.count + Q::PW - 1) / Q::PW;
-  double* xa = s_a[warp];
-  double* xb = s_b[warp];
-  const double q = p.q, qinv = p.qinv;
+  double* x = s_x[warp];
+  const uint32_t e0 = poly * Q::N + t, e1 = poly * Q::N + t * V;  // this lane's first element in either layout
+  auto put = [&](const double (&v)[V], bool layout0) {
+#pragma unroll
+    for (int r = 0; r < V; ++r) x[Q::pad(layout0 ? e0 + T * r : e1 + r)] = v[r];
+    __syncwarp();
+  };
+  auto get = [&](double (&v)[V], bool layout0) {
+#pragma unroll
+    for (int r = 0; r < V; ++r) v[r] = x[Q::pad(layout0 ? e0 + T * r : e1 + r)];
+    __syncwarp();
+  };
   for (size_t task = (size_t)blockIdx.x * kQ50Warps + warp; task < tasks; task += (size_t)gridDim.x * kQ50Warps) {
     const size_t base = task * Q::WE;
     const uint32_t valid = total - base < (size_t)Q::WE ? (uint32_t)(total - base) : (uint32_t)Q::WE;
-    double va[E], vb[E];
+    // Global accesses are coalesced: with eight lanes to a polynomial layout 0
+    // is read and written in 64-byte runs as it is; the others pass through
+    // the warp's copy.  Plain loads (out may alias a or b).
+    auto load = [&](const uint64_t* src, double (&v)[V]) {
+      if constexpr (IN0 && T == 8) {
 #pragma unroll
-    for (int r = 0; r < E; ++r) {
-      // plain loads (out may alias a or b); residues < 2^50 convert exactly
-      const uint32_t e = lane + 32 * r;
-      va[r] = e < valid ? __ull2double_rn(p.a[base + e]) : 0.0;
-      if (TWO) vb[r] = e < valid ? __ull2double_rn(p.b[base + e]) : 0.0;
-    }
-    if (OP == kQ50Fwd || OP == kQ50Mul) q50_forward_regs<LOG_N>(va, s_tab, q, qinv);
-    if (OP == kQ50Mul) q50_forward_regs<LOG_N>(vb, s_tab, q, qinv);
+        for (int r = 0; r < V; ++r) v[r] = e0 + T * r < valid ? q50_load(src[base + e0 + T * r]) : 0.0;
+      } else {
 #pragma unroll
-    for (int r = 0; r < E; ++r) {
-      xa[lane + 32 * r] = va[r];
-      if (TWO) xb[lane + 32 * r] = vb[r];
+        for (int r = 0; r < V; ++r) {
+          const uint32_t e = lane + 32 * r;
+          x[Q::pad(e)] = e < valid ? q50_load(src[base + e]) : 0.0;
+        }
+        __syncwarp();
+        get(v, IN0);
+      }
+    };
+    // the next task's operands come into L2 meanwhile (one line per lane)
+    const size_t next = base + (size_t)gridDim.x * kQ50Warps * Q::WE + 16 * lane;
+    if (16 * lane < Q::WE && next < total) {
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(p.a + next));
+      if (TWO) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.b + next));
     }
-    __syncwarp();
-    double* x = xa + poly * Q::N;
-    double* y = xb + poly * Q::N;
-    if (OP == kQ50Fwd) {
-      double* const xs[1] = {x};
-      q50_forward_smem<LOG_N, 1>(xs, s_tab, g, q, qinv);
+    double u[V], v[V];
+    load(p.a, u);
+    if (TWO) load(p.b, v);
+    if (OP == kQ50Fwd || OP == kQ50Mul) {
+      q50_forward0<LOG_N>(u, p);
+      if (T > 1) {
+        put(u, true);
+        get(u, false);
+      }
+      q50_forward1<LOG_N, Q::LOW0 - 1>(u, s_tab, t, p.q);
     }
-    if (OP == kQ50Inv_) q50_inverse_smem<LOG_N>(x, s_tab, g, q, qinv);
-    if (OP == kQ50Slot) q50_slotwise<LOG_N>(x, y, s_tab, g, q, qinv);
     if (OP == kQ50Mul) {
-      double* const xs[2] = {x, y};
-      q50_forward_smem<LOG_N, 2>(xs, s_tab, g, q, qinv);
-      q50_slotwise<LOG_N>(x, y, s_tab, g, q, qinv);
-      q50_inverse_smem<LOG_N>(x, s_tab, g, q, qinv);
+      q50_forward0<LOG_N>(v, p);
+      if (T > 1) {
+        put(v, true);
+        get(v, false);
+      }
+      q50_forward1<LOG_N, Q::LOW0 - 1>(v, s_tab, t, p.q);
     }
-#pragma unroll
-    for (int r = 0; r < E; ++r) va[r] = xa[lane + 32 * r];
-    if (OP == kQ50Inv_ || OP == kQ50Mul) q50_inverse_regs<LOG_N>(va, s_tab, q, qinv);
-#pragma unroll
-    for (int r = 0; r < E; ++r) {
-      const uint32_t e = lane + 32 * r;
-      if (e < valid) p.out[base + e] = __double2ull_rn(va[r]);
+    if (TWO) q50_slotwise<LOG_N>(u, v, s_tab, t, p);
+    if (OP == kQ50Inv_ || OP == kQ50Mul) {
+      q50_inverse1<LOG_N, 1>(u, s_tab, t, p);
+      if (T > 1) {
+        put(u, false);
+        get(u, true);
+      }
+      q50_inverse0<LOG_N, Q::LOW0>(u, p);
     }
-    __syncwarp();
+    if (OP == kQ50Fwd || OP == kQ50Slot || LOG_N == 1) {  // the last inverse level leaves 0.6q by itself
+#pragma unroll
+      for (int r = 0; r < V; ++r) u[r] = q50_red(u[r], p.q, p.qinv);
+    }
+    if constexpr (OUT0 && T == 8) {
+#pragma unroll
+      for (int r = 0; r < V; ++r)
+        if (e0 + T * r < valid) p.out[base + e0 + T * r] = q50_store(u[r], p.qi);
+    } else {
+      put(u, OUT0);
+#pragma unroll
+      for (int r = 0; r < V; ++r) {
+        const uint32_t e = lane + 32 * r;
+        if (e < valid) p.out[base + e] = q50_store(x[Q::pad(e)], p.qi);
+      }
+      __syncwarp();
+    }
   }
 }
 
@@ -267,10 +344,12 @@ template <int LOG_N, int OP>
 static int q50_launch(const lc_quad50_plan* plan, const uint64_t* a, const uint64_t* b, uint64_t* out,
                       size_t count, cudaStream_t st) {
   using Q = Q50Geo<LOG_N>;
-  Q50Params p{a, b, out, count, (double)plan->q, 1.0 / (double)plan->q, plan->d_tab};
+  Q50Params p{a, b, out, count, (double)plan->q, 1.0 / (double)plan->q, plan->q, plan->d_tab, {}, {}, plan->ninv};
+  std::copy(plan->fwd0, plan->fwd0 + 15, p.fwd0);
+  std::copy(plan->inv0, plan->inv0 + 15, p.inv0);
   const size_t tasks = (count + Q::PW - 1) / Q::PW;
   const size_t want = (tasks + kQ50Warps - 1) / kQ50Warps;
-  const size_t cap = (size_t)std::max(1, device_sm_count()) * 8;
+  const size_t cap = (size_t)std::max(1, device_sm_count()) * kQ50Ctas;
   quad50_kernel<LOG_N, OP><<<(unsigned)std::min(want, cap), kQ50Warps * 32, 0, st>>>(p);
   return map_cuda(cudaGetLastError());
 }
@@ -345,32 +424,46 @@ LC_API int lc_quad50_plan_create(uint64_t q, uint32_t two_adicity, uint64_t gene
   p->generator = generator;
   p->two_adicity = two_adicity;
   p->log_n = log_n;
-  const uint64_t inv2 = hpow(2, q - 2, q);
+  auto constant = [q](uint64_t w) {  // centered, below 2^49: exact
+    const double c = w > q / 2 ? -(double)(q - w) : (double)w;
+    return Q50Const{c, c / (double)q};
+  };
+  const uint64_t ninv = hpow(hpow(2, log_n - 1, q), q - 2, q);  // the levels' factors 1/2
+  const int log_v = std::min(4, (int)log_n), log_t = (int)log_n - log_v, v = 1 << log_v, t = 1 << log_t;
+  Q50Const tab[kQ50Tab] = {};
+  p->ninv = constant(ninv);
+  int p1 = 0;
   for (uint32_t d = 0; d + 1 < log_n; ++d) {  // :272-289
+    const int b = (int)log_n - 1 - (int)d;    // pair bit
     for (uint32_t i = 0; i < (1u << d); ++i) {
       const uint64_t e = ((2 * (uint64_t)rev_bits(i, d) + 1) << (5 - d)) % 128;
-      const uint64_t w = hpow(zeta, e, q);
-      p->tab[(1u << d) - 1 + i] = w;
-      p->tab[kQ50Inv + (1u << d) - 1 + i] = hmul(inv2, hpow(w, q - 2, q), q);
+      const uint64_t w = hpow(zeta, e, q), wi = hpow(w, q - 2, q);
+      if (b >= std::max(1, log_t)) {
+        p->fwd0[(1u << d) - 1 + i] = constant(w);
+        p->inv0[(1u << d) - 1 + i] = constant(d == 0 ? hmul(wi, ninv, q) : wi);
+      } else {  // block i = lane t's j-th, stored [j][t]
+        const int per = v >> (b + 1), at = p1 + (int)(i % per) * t + (int)(i / per);
+        tab[at] = constant(w);
+        tab[kQ50P1 + at] = constant(wi);
+      }
     }
+    if (b < std::max(1, log_t)) p1 += (v >> (b + 1)) * t;
   }
   for (uint32_t s = 0; s < (1u << (log_n - 1)); ++s) {  // :291-296
     const uint64_t e = ((2 * (uint64_t)rev_bits(s, log_n - 1) + 1) << (7 - log_n)) % 128;
-    p->tab[kQ50Gamma + s] = hpow(zeta, e, q);
+    p->gamma[s] = hpow(zeta, e, q);
+    tab[2 * kQ50P1 + (int)(s % (v / 2)) * t + (int)(s / (v / 2))] = constant(p->gamma[s]);
   }
-  p->tab[kQ50Inv2] = inv2;
-  double dtab[kQ50Tab];
-  for (int i = 0; i < kQ50Tab; ++i) dtab[i] = (double)p->tab[i];  // < 2^50: exact
   if (device_sm_count() <= 0) {
     delete p;
     return LC_ERR_NO_DEVICE;
   }
-  if (cudaMalloc(&p->d_tab, sizeof(p->tab)) != cudaSuccess) {
+  if (cudaMalloc(&p->d_tab, sizeof(tab)) != cudaSuccess) {
     cudaGetLastError();
     delete p;
     return LC_ERR_OUT_OF_MEMORY;
   }
-  cudaError_t e = cudaMemcpy(p->d_tab, dtab, sizeof(dtab), cudaMemcpyHostToDevice);
+  cudaError_t e = cudaMemcpy(p->d_tab, tab, sizeof(tab), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(p->d_tab);
     delete p;
@@ -391,7 +484,7 @@ LC_API int lc_quad50_plan_info(const lc_quad50_plan* plan, uint64_t* zeta, uint6
   if (!plan) return LC_ERR_INVALID_ARGUMENT;
   if (zeta) *zeta = plan->zeta;
   if (slot_constants)
-    for (uint32_t s = 0; s < (1u << (plan->log_n - 1)); ++s) slot_constants[s] = plan->tab[lc::kQ50Gamma + s];
+    for (uint32_t s = 0; s < (1u << (plan->log_n - 1)); ++s) slot_constants[s] = plan->gamma[s];
   return LC_OK;
 }
 

@@ -61,6 +61,33 @@ def test_transforms_and_products_match_oracle(mod, log_n):
         assert np.array_equal(t.mul(a, b), want)  # host-buffer entry point
 
 
+@pytest.mark.parametrize("log_n", [1, 2, 3, 4, 5, 6, 7])
+def test_extreme_residues(log_n):
+    """Operands that drive the lazy values to their bounds: all q - 1, q - 1 and 0
+    alternating in blocks of every span, and values next to q/2; counts around
+    a warp's polynomials."""
+    mod = oracle.Q_50
+    q, n = mod[0], 1 << log_n
+    ot = oracle.QuadSlotTables50(oracle.Modulus50(*mod), log_n)
+    t = QuadSlotTables(Modulus50(*mod), log_n)
+    idx = np.arange(n, dtype=np.uint64)
+    rows = [np.full(n, q - 1, np.uint64), np.full(n, q // 2, np.uint64), np.full(n, q // 2 + 1, np.uint64)]
+    for b in range(log_n):
+        rows += [np.where(idx >> np.uint64(b) & np.uint64(1), q - 1, 0).astype(np.uint64),
+                 np.where(idx >> np.uint64(b) & np.uint64(1), q // 2, q // 2 + 1).astype(np.uint64)]
+    rows = np.array(rows)
+    per_warp = max(32 * min(16, n) // n, 1)
+    for count in (per_warp - 1, per_warp, per_warp + 1):
+        if count == 0:
+            continue
+        a, b = rows[np.arange(count) % len(rows)], rows[(np.arange(count) * 3 + 1) % len(rows)]
+        fa = per_poly(ot.forward, a)
+        assert np.array_equal(host(t.forward(dev(a))), fa)
+        assert np.array_equal(host(t.inverse(dev(a))), per_poly(ot.inverse, a))
+        assert np.array_equal(host(t.slotwise_mul(dev(a), dev(b))), per_poly(ot.slotwise_mul, a, b))
+        assert np.array_equal(host(t.mul(dev(a), dev(b))), per_poly(ot.mul, a, b))
+
+
 def test_large_batch_and_in_place():
     log_n, count = 7, 1 << 15
     mod = oracle.Q_50
