@@ -85,7 +85,7 @@ LC_D uint32_t to_residue<uint32_t, uint8_t>(uint8_t x, uint32_t) {
 }
 
 // Witness NTT, frequency-major output.  CTA (j, b-block of BB witnesses):
-// loads the BB polynomials w[b][j][*] (16-byte vector loads when aligned),
+// loads the BB polynomials w[b][j][*] (consecutive lanes, consecutive words),
 // transforms them in shared memory and writes What_T[t][j][b0 + b] -- for
 // each NTT slot t one contiguous run of BB values -- with zeros for
 // b >= batch so the padded columns of the product tiles are exact zeros.
@@ -128,23 +128,21 @@ __global__ void __launch_bounds__(NT)
   const uint32_t j0 = blockIdx.x * JB;
   const uint32_t b0 = blockIdx.y * BB;
   for (int i = threadIdx.x; i < G::fwd_entries(); i += NT) tw[i] = twg[i];
-  constexpr int EPC = 16 / sizeof(S);  // elements per 16-byte chunk
-  constexpr int CH = N / EPC;          // chunks per polynomial
-  const bool vec = (N * sizeof(S)) % 16 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
-  if (vec) {
-    for (int e = threadIdx.x; e < PP * CH; e += NT) {
-      const int pp = e / CH, k = e % CH;
+  if (sizeof(S) == 1 && (reinterpret_cast<uintptr_t>(w) & 3) == 0) {
+    // four digits per load; lane l stores digit (u + l / 8) mod 4 in step u, so
+    // that a warp's 32 stores (stride 4) fall on 32 banks
+    const uint32_t rot = threadIdx.x >> 3;
+    for (int e = threadIdx.x; e < PP * (N / 4); e += NT) {
+      const int pp = e / (N / 4), k = e % (N / 4);
       const int jj = pp / BB, b = pp % BB;
-      T* dst = slots + pp * SS + k * EPC;
-      if (b0 + b < batch && j0 + jj < m) {
-        const uint4 v =
-            *reinterpret_cast<const uint4*>(w + ((size_t)(b0 + b) * m + j0 + jj) * N + (size_t)k * EPC);
-        const S* x = reinterpret_cast<const S*>(&v);
+      uint32_t v = 0;
+      if (b0 + b < batch && j0 + jj < m)
+        v = *reinterpret_cast<const uint32_t*>(w + ((size_t)(b0 + b) * m + j0 + jj) * N + (size_t)k * 4);
+      T* dst = slots + pp * SS + 4 * k;
 #pragma unroll
-        for (int u = 0; u < EPC; ++u) dst[u] = to_residue<T, S>(x[u], q);
-      } else {
-#pragma unroll
-        for (int u = 0; u < EPC; ++u) dst[u] = 0;
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t x = (u + rot) & 3;
+        dst[x] = to_residue<T, S>((S)(v >> (8 * x)), q);
       }
     }
   } else {
@@ -161,8 +159,12 @@ __global__ void __launch_bounds__(NT)
   const int grp = threadIdx.x / G::T;
   const uint32_t t = threadIdx.x % G::T;
 #pragma unroll 1
-  for (int it = 0; it < IT; ++it)
+  for (int it = 0; it < IT; ++it) {
+    // a warp whose first polynomial is padding holds only padding (zeros)
+    const int first = it * GROUPS + (int)(threadIdx.x & ~31u) / G::T;
+    if (b0 + first % BB >= batch || j0 + first / BB >= m) continue;
     transform_slot<A, LOG_N, LOG_V, false>(slots + (it * GROUPS + grp) * SS, tw, ar, t);
+  }
   __syncthreads();
   // for each slot tt the tile's (jj, b) values are one contiguous run when BB == b_pad
   for (int e = threadIdx.x; e < PP * N; e += NT) {
@@ -835,35 +837,35 @@ static int launch_witness_cfg(const lc_ajtai_key* key, const S* w, size_t batch,
   return map_cuda(cudaGetLastError());
 }
 
-// Polynomials per CTA of the small-batch tiles: as many slots as fit in
-// 96 KB, a multiple of the 128-thread CTA's polynomial groups, at most 128.
+// Polynomials per 128-thread CTA of a witness tile: 64, 32 or 16, the most
+// whose slots fit in 40 KB, so that five or more CTAs share an SM and one's
+// loads and stores overlap another's transforms (tiles of 96 KB, two CTAs per
+// SM, took 99 us for 60 020 Goldilocks polynomials of degree 128, these 71).
 template <class A, int LOG_N, int LOG_V>
-struct SmallWitnessTile {
+struct WitnessTile {
   static constexpr int groups = 128 / Geo<LOG_N, LOG_V>::T;
-  static constexpr int fit = (96 * 1024) / (WitnessSlotStride<A, LOG_N>::value * (int)sizeof(typename A::T));
-  static constexpr int polys = (fit > 128 ? 128 : fit) / groups * groups;
+  static constexpr int fit = (40 * 1024) / (WitnessSlotStride<A, LOG_N>::value * (int)sizeof(typename A::T));
+  static constexpr int polys = fit >= 64 ? 64 : fit >= 32 ? 32 : 16;
+  static_assert(polys % groups == 0 && fit >= 16, "tile");
 };
 
-// 128 witnesses per CTA when the batch is tiled and 128 slots fit in 160 KB of
-// shared memory (64 otherwise); small batches: 8, 4 or 1 witnesses by as many
-// ring elements as fill SmallWitnessTile, 32 witnesses when b_pad is neither.
+// A tile is BB witnesses by PP / BB ring elements, BB the largest of 32, 16, 8,
+// 4 that divides b_pad (at most PP): for each NTT slot it writes runs of BB
+// values, contiguous over its ring elements when BB == b_pad.
 template <class A, int LOG_N, int LOG_V, class S>
 static int launch_witness_to(const lc_ajtai_key* key, const S* w, size_t batch, uint32_t b_pad,
                              typename A::T* dst, cudaStream_t st) {
-  constexpr bool fits128 =
-      (size_t)128 * WitnessSlotStride<A, LOG_N>::value * sizeof(typename A::T) <= 160 * 1024;
-  if (b_pad % 128 == 0) {
-    if constexpr (fits128)
-      return launch_witness_cfg<A, LOG_N, LOG_V, S, 256, 128>(key, w, batch, b_pad, dst, st);
-    else
-      return launch_witness_cfg<A, LOG_N, LOG_V, S, 256, 64>(key, w, batch, b_pad, dst, st);
-  }
-  constexpr int PP = SmallWitnessTile<A, LOG_N, LOG_V>::polys;
-  constexpr int G = SmallWitnessTile<A, LOG_N, LOG_V>::groups;
-  static_assert(PP >= 8 && PP % 8 == 0 && G % 8 == 0, "small tile");
+  constexpr int PP = WitnessTile<A, LOG_N, LOG_V>::polys;
+  constexpr int G = WitnessTile<A, LOG_N, LOG_V>::groups;
+  static_assert(G % 8 == 0, "small tile");
   // tiny problems (fewer polynomials than full tiles for every SM): one
   // polynomial per thread group, so the grid still spreads over the SMs
   const bool tiny = (size_t)key->m * b_pad < (size_t)std::max(1, device_sm_count()) * PP;
+  if (!tiny && PP >= 32 && b_pad % 32 == 0)
+    return launch_witness_cfg<A, LOG_N, LOG_V, S, 128, PP < 32 ? PP : 32, PP < 32 ? 1 : PP / 32>(key, w, batch, b_pad,
+                                                                                             dst, st);
+  if (!tiny && b_pad % 16 == 0)
+    return launch_witness_cfg<A, LOG_N, LOG_V, S, 128, 16, PP / 16>(key, w, batch, b_pad, dst, st);
   if (b_pad % 8 == 0)
     return tiny ? launch_witness_cfg<A, LOG_N, LOG_V, S, 128, 8, G / 8>(key, w, batch, b_pad, dst, st)
                 : launch_witness_cfg<A, LOG_N, LOG_V, S, 128, 8, PP / 8>(key, w, batch, b_pad, dst, st);
@@ -873,7 +875,7 @@ static int launch_witness_to(const lc_ajtai_key* key, const S* w, size_t batch, 
   if (b_pad < 4)
     return tiny ? launch_witness_cfg<A, LOG_N, LOG_V, S, 128, 1, G>(key, w, batch, b_pad, dst, st)
                 : launch_witness_cfg<A, LOG_N, LOG_V, S, 128, 1, PP>(key, w, batch, b_pad, dst, st);
-  return launch_witness_cfg<A, LOG_N, LOG_V, S, 128, 32>(key, w, batch, b_pad, dst, st);
+  return launch_witness_cfg<A, LOG_N, LOG_V, S, 128, 16, PP / 16>(key, w, batch, b_pad, dst, st);
 }
 
 template <class A, int LOG_N, int LOG_V, class S>
@@ -1253,12 +1255,22 @@ static int commit_any(lc_ajtai_key* key, const S* w, size_t batch, void* out, cu
     key->last_fused = rc == LC_OK;
     if (rc != LC_ERR_UNSUPPORTED) return rc;
   }
-  // tiles of 128 witnesses from 64 on; from 4 on a multiple of 4 (zero
-  // columns) for the quad product
-  const uint32_t b_pad = batch >= 64 ? (uint32_t)((batch + kBTile - 1) / kBTile * kBTile)
-                                     : batch >= 4 ? (uint32_t)((batch + 3) / 4 * 4) : (uint32_t)batch;
   const size_t eb = key->wide ? 8 : 4;
-  int rc = grow(&key->d_what_t, &key->what_bytes, (size_t)key->n * key->m * b_pad * eb);
+  // Tiles of 128 witnesses from 64 on.  From 4 on, for the tensor-core products,
+  // the power of two whose row is at least 32 bytes, zero columns included: at
+  // 20 witnesses (kappa = 6, m = 3001, d = 128) the integer form's products and
+  // sums on 20 columns took 76 us, the tensor form's on 32 columns 42 us.  For
+  // the integer form, and when that scratch cannot be had, a multiple of 4.
+  uint32_t b_pad = batch >= 64 ? (uint32_t)((batch + kBTile - 1) / kBTile * kBTile)
+                               : batch >= 4 ? (uint32_t)((batch + 3) / 4 * 4) : (uint32_t)batch;
+  int rc = LC_ERR_OUT_OF_MEMORY;
+  if (batch >= 4 && batch < 64 && key->slot_products == LC_PRODUCTS_TENSOR) {
+    uint32_t pow2 = (uint32_t)(32 / eb);
+    while (pow2 < batch) pow2 *= 2;
+    rc = grow(&key->d_what_t, &key->what_bytes, (size_t)key->n * key->m * pow2 * eb);
+    if (rc == LC_OK) b_pad = pow2;
+  }
+  if (rc) rc = grow(&key->d_what_t, &key->what_bytes, (size_t)key->n * key->m * b_pad * eb);
   if (rc) return rc;
   rc = witness_ntt<S>(key, w, batch, b_pad, st);
   if (rc) return rc;

@@ -809,7 +809,7 @@ struct SpIdesc {
 
 struct SpParams {
   int32_t* partial;  // [split][t][ntile][NCTA][128]
-  uint32_t m, nslots, ntiles, splits;
+  uint32_t m, nslots, ntiles, splits, jper;  // jper ring elements per split, a multiple of kSpRows
   uint32_t* err;
 };
 
@@ -829,8 +829,8 @@ __global__ void __launch_bounds__(kSpThreads, 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * kSpStages + 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t t = blockIdx.x, nt = blockIdx.y, split = blockIdx.z;
-  const uint32_t j0 = split * kSpKSplit;
-  const uint32_t j1 = min(p.m, j0 + kSpKSplit);
+  const uint32_t j0 = split * p.jper;
+  const uint32_t j1 = min(p.m, j0 + p.jper);
   const int nst = (int)((j1 - j0 + kSpRows - 1) / kSpRows);
 
   if (tid == 0) {
@@ -946,54 +946,83 @@ __global__ void __launch_bounds__(kSpThreads, 1)
 }
 
 // Chat[b][i][t] = sum_{la,lw} 2^(8 (la + lw)) sum_split D[split][t][nt][(bl, lw)][(i, la)]  mod q.
-// Pair sums over the splits fit 64 bits (< 2^31 * splits); the 2L - 1 sums of
-// equal la + lw = k are folded with 2^(8k) mod q (128 bits for Goldilocks,
-// 64-bit remainders for u32 q).
+// A warp forms the 16 rows i of one (t, b): the L columns (bl, lw) of a split
+// are contiguous, and a lane reads four consecutive la of one i with each
+// 16-byte load (L = 8: lane pairs share an i; L = 4: rows 64 .. 127 are the zero
+// atom, so the half-warps take alternate columns).  Its sums by lw + la stay
+// below 2^47 (at most 2^14 splits).  WPS warps share the splits of a (t, b)
+// and add their residues through shared memory: one thread per output ran 32
+// CTAs over the 64 MB of a folding step's 32 splits in 103 us, this 20.
+constexpr uint32_t kSpMaxSplits = 1u << 14;
+
 template <class E>
-__global__ void slot_products_reduce_kernel(const int32_t* __restrict__ part, E* __restrict__ chat, uint32_t n,
-                                            uint32_t kappa, uint32_t batch, uint32_t ncta, uint32_t ntiles,
-                                            uint32_t splits, uint32_t q) {
+__global__ void __launch_bounds__(256)
+    slot_products_reduce_kernel(const int32_t* __restrict__ part, E* __restrict__ chat, uint32_t n, uint32_t kappa,
+                                uint32_t batch, uint32_t ncta, uint32_t ntiles, uint32_t splits, uint32_t wps,
+                                uint32_t q) {
   constexpr int L = sizeof(E);
-  const size_t total = (size_t)n * batch * kappa;
-  const uint32_t wpt = ncta / L;  // witnesses per N tile
-  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t i = idx % kappa;
-    const uint32_t b = (uint32_t)((idx / kappa) % batch);
-    const uint32_t t = (uint32_t)(idx / ((size_t)kappa * batch));
+  constexpr int COLS = L == 8 ? 8 : 2;   // columns per lane
+  constexpr int KS = L == 8 ? 11 : 6;    // sums per lane
+  __shared__ E s_r[8][16];
+  const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const size_t total = (size_t)n * batch;  // (t, b) groups, 8 / wps per CTA
+  for (size_t g0 = (size_t)blockIdx.x * (8 / wps); g0 < total; g0 += (size_t)gridDim.x * (8 / wps)) {
+    const size_t group = g0 + warp / wps;
+    const bool in = group < total;
+    const uint32_t t = (uint32_t)(group / batch), b = (uint32_t)(group % batch), wpt = ncta / L;
     const uint32_t nt = b / wpt, bl = b % wpt;
-    uint64_t tk[2 * L - 1];
+    uint64_t tk[KS];
 #pragma unroll
-    for (int k = 0; k < 2 * L - 1; ++k) tk[k] = 0;
-    for (uint32_t sp = 0; sp < splits; ++sp) {
-      const int32_t* d = part + (((size_t)sp * n + t) * ntiles + nt) * (size_t)ncta * 128;
+    for (int k = 0; k < KS; ++k) tk[k] = 0;
+    if (in) {
+      const size_t step = (size_t)n * ntiles * ncta * 128;
+      const int32_t* d = part + ((size_t)t * ntiles + nt) * ncta * 128 + (size_t)bl * L * 128 +
+                         (L == 8 ? 4 * lane : 4 * (lane % 16) + 128 * (lane / 16));
+#pragma unroll 2
+      for (uint32_t sp = warp % wps; sp < splits; sp += wps) {
 #pragma unroll
-      for (int lw = 0; lw < L; ++lw) {
-        const int32_t* col = d + (size_t)(bl * L + lw) * 128 + i * L;
-#pragma unroll
-        for (int la = 0; la < L; ++la) tk[la + lw] += (uint64_t)(uint32_t)col[la];
+        for (int c = 0; c < COLS; ++c) {
+          const uint4 v = *reinterpret_cast<const uint4*>(d + sp * step + (L == 8 ? 128 : 256) * c);
+          const int k = L == 8 ? c : 2 * c;
+          tk[k] += v.x;
+          tk[k + 1] += v.y;
+          tk[k + 2] += v.z;
+          tk[k + 3] += v.w;
+        }
       }
     }
-    E res;
-    if constexpr (L == 8) {
+    E r;
+    uint32_t i;
+    bool mine;
+    if constexpr (L == 8) {  // odd lanes hold la = 4 .. 7: 2^32 more
       unsigned __int128 v = 0;
-      uint64_t c = 1;  // 2^(8k) mod p
 #pragma unroll
-      for (int k = 0; k < 2 * L - 1; ++k) {
-        v += (unsigned __int128)tk[k] * c;
-        c = gl_mul(c, 256);
-      }
-      res = gl_canon(gl_reduce128_lazy((uint64_t)(v >> 64), (uint64_t)v));
-    } else {
-      uint64_t v = 0, c = 1 % q;  // 2^(8k) mod q
+      for (int k = 0; k < KS; ++k) v += (unsigned __int128)tk[k] << (8 * k);
+      r = gl_canon(gl_reduce128_lazy((uint64_t)(v >> 64), (uint64_t)v));
+      if (lane & 1) r = gl_mul(r, 1ull << 32);
+      r = gl_add(r, __shfl_xor_sync(0xffffffffu, r, 1));
+      i = lane / 2;
+      mine = !(lane & 1);
+    } else {  // the upper half-warp holds odd lw: 2^8 more
+      uint64_t v = 0;
 #pragma unroll
-      for (int k = 0; k < 2 * L - 1; ++k) {
-        v = (v + (tk[k] % q) * c % q) % q;  // each term < q < 2^32 before the sum
-        c = (c << 8) % q;
-      }
-      res = (E)v;
+      for (int k = KS - 1; k >= 0; --k) v = ((v << 8) + tk[k]) % q;
+      if (lane >= 16) v = (v << 8) % q;
+      r = (E)((v + __shfl_xor_sync(0xffffffffu, (uint32_t)v, 16)) % q);
+      i = lane % 16;
+      mine = lane < 16;
     }
-    chat[((size_t)b * kappa + i) * n + t] = res;
+    if (mine) s_r[warp][i] = r;
+    __syncthreads();
+    if (mine && in && warp % wps == 0 && i < kappa) {
+      uint64_t sum = r;
+      for (uint32_t w = 1; w < wps; ++w) {
+        if constexpr (L == 8) sum = gl_add(sum, s_r[warp + w][i]);
+        else sum += s_r[warp + w][i];
+      }
+      chat[((size_t)b * kappa + i) * n + t] = L == 8 ? (E)sum : (E)(sum % q);
+    }
+    __syncthreads();  // s_r is read out
   }
 }
 
@@ -1037,8 +1066,18 @@ int tc_slot_products(const void* ahat_t, uint32_t a_m, const void* what_t, uint3
   else
     return LC_ERR_UNSUPPORTED;
   const uint64_t ntiles = row / ncta;
-  const uint32_t splits = (m + kSpKSplit - 1) / kSpKSplit;
-  if (ntiles > 65535 || splits > 65535) return LC_ERR_UNSUPPORTED;  // grid y, z
+  // K splits: at least one per kSpKSplit ring elements, and enough for every SM
+  // to hold one CTA of 512-byte tiles or two narrower ones (m = 7998, 64 slots,
+  // 64-byte rows: 64 CTAs without, 40 us; 256 with, 18 us), each of at least
+  // four ring stages
+  const uint64_t sms = (uint64_t)std::max(1, device_sm_count());
+  const uint64_t resident = ncta == 512 ? sms : 2 * sms;
+  const uint64_t want = std::max<uint64_t>((m + kSpKSplit - 1) / kSpKSplit, resident / (n * ntiles));
+  uint32_t jper = (uint32_t)((m + want - 1) / std::max<uint64_t>(want, 1));
+  jper = std::max<uint32_t>((jper + kSpRows - 1) / kSpRows * kSpRows, kSpStages * kSpRows);
+  jper = std::min(jper, kSpKSplit);
+  const uint32_t splits = (m + jper - 1) / jper;
+  if (ntiles > 65535 || splits > kSpMaxSplits) return LC_ERR_UNSUPPORTED;  // grid y; the reduction's sums
   const size_t need = (size_t)splits * n * ntiles * ncta * 128 * sizeof(int32_t);
   if (need > *part_bytes) {
     if (*part) cudaFree(*part);
@@ -1076,20 +1115,21 @@ int tc_slot_products(const void* ahat_t, uint32_t a_m, const void* what_t, uint3
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return LC_ERR_UNSUPPORTED;
   }
-  const SpParams prm{static_cast<int32_t*>(*part), m, n, (uint32_t)ntiles, splits, err};
+  const SpParams prm{static_cast<int32_t*>(*part), m, n, (uint32_t)ntiles, splits, jper, err};
   int rc = aw == 128 ? launch_slot_products_n<128>(ncta, amap, wmap, prm, st)
                      : launch_slot_products_n<64>(ncta, amap, wmap, prm, st);
   if (rc) return rc;
-  const size_t total = (size_t)n * batch * kappa;
-  const unsigned blocks = (unsigned)std::min<size_t>((total + 255) / 256, (size_t)device_sm_count() * 16);
+  uint32_t wps = 1;
+  while (wps < 8 && wps < splits) wps *= 2;
+  const size_t blocks = std::min<size_t>(((size_t)n * batch * wps + 7) / 8, 1u << 20);
   if (elem_bytes == 8)
-    slot_products_reduce_kernel<uint64_t><<<blocks, 256, 0, st>>>(
+    slot_products_reduce_kernel<uint64_t><<<(unsigned)blocks, 256, 0, st>>>(
         static_cast<const int32_t*>(*part), static_cast<uint64_t*>(chat), n, kappa, (uint32_t)batch, ncta,
-        (uint32_t)ntiles, splits, q);
+        (uint32_t)ntiles, splits, wps, q);
   else
-    slot_products_reduce_kernel<uint32_t><<<blocks, 256, 0, st>>>(
+    slot_products_reduce_kernel<uint32_t><<<(unsigned)blocks, 256, 0, st>>>(
         static_cast<const int32_t*>(*part), static_cast<uint32_t*>(chat), n, kappa, (uint32_t)batch, ncta,
-        (uint32_t)ntiles, splits, q);
+        (uint32_t)ntiles, splits, wps, q);
   return map_cuda(cudaGetLastError());
 }
 

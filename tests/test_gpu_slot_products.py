@@ -149,3 +149,32 @@ def test_switch_arguments():
     assert L.lc_ajtai_key_set_slot_products(key.handle, 2) == _lib.LC_ERR_INVALID_ARGUMENT
     assert L.lc_ajtai_key_set_slot_products(None, 0) == _lib.LC_ERR_INVALID_ARGUMENT
     assert L.lc_ajtai_key_get_slot_products(None) == -1
+
+
+@pytest.mark.parametrize("ring", ["gl64", "gl128", "gl256", "q32_64", "q32_256", "crt128"])
+@pytest.mark.parametrize("kappa,m,batch", [
+    (6, 700, 5), (2, 1281, 9), (16, 257, 20), (3, 300, 33), (5, 64, 63),
+    (1, 4097, 17),   # several K splits with a short last one
+    (16, 255, 12),   # one K split
+])
+def test_padded_batches_and_splits(ring, kappa, m, batch):
+    """Batches between the tensor form's tile widths (padded with zero columns)
+    and every number of K splits: equal to the integer form's results."""
+    from lzx_b200.batch import U32AjtaiKey
+    d = int(ring.removeprefix("gl").removeprefix("q32_").removeprefix("crt"))
+    log_d = d.bit_length() - 1
+    rng = np.random.default_rng(m + batch)
+    if ring.startswith("gl"):
+        key = GoldilocksAjtaiKey(log_d, kappa, m, synth.synth_gl(m, 0, kappa * m * d).reshape(kappa, m, d))
+        dev, W = key._dev, synth.synth_gl(m, 1, batch * m * d).reshape(batch, m, d)
+    else:
+        mod = Modulus32.Q_32 if ring.startswith("q32") else CRT_SET_30BIT[1]
+        key = U32AjtaiKey(mod, log_d, kappa, m, synth.synth_mod32(m, 0, mod.q, kappa * m * d).reshape(kappa, m, d))
+        dev, W = key._dev, synth.synth_mod32(m, 1, mod.q, batch * m * d).reshape(batch, m, d)
+    W[-1] = 0
+    W8 = rng.integers(-128, 128, (batch, m, d)).astype(np.int8)
+    for w in (W, W8, W8.view(np.uint8)):
+        dev.slot_products = _lib.LC_PRODUCTS_TENSOR
+        tensor = dev.commit_array(w)
+        dev.slot_products = _lib.LC_PRODUCTS_INT64
+        assert np.array_equal(tensor, dev.commit_array(w))
