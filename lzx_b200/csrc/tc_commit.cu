@@ -353,21 +353,23 @@ __global__ void tc_reduce_kernel(const int64_t* __restrict__ partial, uint64_t* 
 // (the natural-order negacyclic NTT, out[t] = w(psi^(2t+1))).  With the
 // residues V split into 8 byte limbs, D_l[r][t] = sum_c W[r][c] V_l[t][c] is
 // exact in int32 (64 * 128 * 255 < 2^21, u8 digits 64 * 255 * 255 < 2^22) and
-// What = sum_l 2^(8l) D_l (mod p).  An M = 128 tile holds R consecutive ring
+// What = sum_l 2^(8l) D_l (mod p) (gl_fold_limbs).  An M = 128 tile holds R consecutive ring
 // elements x BB witnesses (R * BB = 128; rows ordered witness fastest, one
 // 64-byte ring element each, read by a 3-D TMA view of w[b][j][64] -- x the
-// digit, y the witness, z the ring element -- with the 64-byte swizzle); a
-// tile is four MMAs (two limb groups N = 256, K = 64 as two K-steps) into all
-// 512 TMEM columns.  Sixteen epilogue warps read the limbs back, fold them
-// mod p and write What_T[t][j][b]: a warp's 32 rows are 32 consecutive
-// entries of one slot.
+// digit, y the witness, z the ring element -- with the 64-byte swizzle).  A
+// tile runs as two halves of 32 slots (N = 256 columns (limb, slot), K = 64 as
+// two K-steps) into two TMEM accumulators, so the MMAs of one half run while
+// the sixteen epilogue warps read, fold and store the other: a warp's 32 rows
+// are 32 consecutive What_T[t][j][b] entries of one slot.  With one 512-column
+// accumulator per tile the folds waited for the MMAs: 965 us per 2^29 outputs,
+// now 855 (4.8 GB, 5.6 TB/s: the stores bound it).
 constexpr int kTnSlots = 4;
 constexpr int kTnATile = 128 * 64;  // 128 rows (ring element, witness) x 64 digit bytes
 constexpr int kTnVTile = 256 * 128;
 constexpr int kTnOffV = kTnSlots * kTnATile;
 constexpr int kTnOffBar = kTnOffV + 2 * kTnVTile;
 constexpr size_t kTnSmem = 1024 + kTnOffBar + 256;
-constexpr int kTnEpiWarps = 16;  // 4 per TMEM lane quarter, 16 slots each
+constexpr int kTnEpiWarps = 16;  // 4 per TMEM lane quarter, 8 slots of each half
 constexpr int kTnThreads = (kTnEpiWarps + 2) * 32;
 static_assert(kTnSmem <= 227 * 1024, "shared memory");
 
@@ -379,33 +381,6 @@ struct TnParams {
   uint32_t* err;
 };
 
-// sum_l 2^(8l) D_l mod p for one output (|D_l| < 2^22), as a 64-bit value
-// congruent mod p but not necessarily canonical (it may lie in [p, 2^64)):
-// every reader of the witness transforms -- the byte-limb slot products and
-// the 160-bit integer products -- takes any 64-bit representative.  A = D0 +
-// 2^8 D1 + 2^16 D2 + 2^24 D3 and B (limbs 4..7) are exact in int64 (|A|,
-// |B| < 2^47); the value is A + 2^32 B == S + 2^32 lo(B) with
-// S = A + hi(B) (2^32 - 1) (2^64 == 2^32 - 1 mod p), |S| < 2^48.  With
-// U = S + 2^32 lo(B) in (-2^48, 2^64 + 2^48), R = U mod 2^64 and
-// U = R + k 2^64, k = carry - [S < 0] in {-1, 0, 1}: the value is
-// R + k (2^32 - 1), which stays inside [0, 2^64) in each case (k = 1 only
-// when R < 2^48, k = -1 only when R > 2^64 - 2^48).
-LC_D uint64_t tn_fold(const uint32_t (&d)[8][8], int u) {
-  // limb pairs in 32 bits: |D| < 2^21 (s8 digits) or 0 <= D < 2^22 (u8), so
-  // D_l + 2^8 D_(l+1) stays inside int32
-  const int32_t p01 = (int32_t)d[0][u] + (int32_t)d[1][u] * 256;
-  const int32_t p23 = (int32_t)d[2][u] + (int32_t)d[3][u] * 256;
-  const int32_t p45 = (int32_t)d[4][u] + (int32_t)d[5][u] * 256;
-  const int32_t p67 = (int32_t)d[6][u] + (int32_t)d[7][u] * 256;
-  const int64_t A = (int64_t)p01 + (int64_t)p23 * 65536;
-  const int64_t B = (int64_t)p45 + (int64_t)p67 * 65536;
-  const int64_t S = A + (B >> 32) * (int64_t)kGlEps;
-  const uint64_t lo = (uint64_t)(uint32_t)B << 32;
-  const uint64_t R = (uint64_t)S + lo;
-  const int k = (int)(R < lo) - (int)(S < 0);
-  return R + (uint64_t)(int64_t)k * kGlEps;
-}
-
 template <bool S8>
 __global__ void __launch_bounds__(kTnThreads, 1)
     tc_ntt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ TnParams p) {
@@ -415,11 +390,11 @@ __global__ void __launch_bounds__(kTnThreads, 1)
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + kTnOffBar);
   uint64_t* loaded = bars;        // [4] A tile of a slot landed (tx bytes)
   uint64_t* freed = bars + 4;     // [4] the MMAs that read a slot finished
-  uint64_t* acc_full = bars + 8;  // MMAs of a ring element finished
-  uint64_t* acc_empty = bars + 9; // the epilogue warps read TMEM
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 11);
-  uint64_t* all_done = bars + 12;  // final commit: every MMA issued has finished
+  uint64_t* acc_full = bars + 8;    // [2] MMAs of a half finished
+  uint64_t* acc_empty = bars + 10;  // [2] the epilogue warps read that half
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 13);
+  uint64_t* all_done = bars + 14;  // final commit: every MMA issued has finished
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
@@ -427,8 +402,10 @@ __global__ void __launch_bounds__(kTnThreads, 1)
       mbar_init(&loaded[s], 1);
       mbar_init(&freed[s], 1);
     }
-    mbar_init(acc_full, 1);
-    mbar_init(acc_empty, kTnEpiWarps);
+    for (int h = 0; h < 2; ++h) {
+      mbar_init(&acc_full[h], 1);
+      mbar_init(&acc_empty[h], kTnEpiWarps);
+    }
     mbar_init(all_done, 1);
     *abort_flag = 0;
     fence_mbar_init();
@@ -479,69 +456,68 @@ __global__ void __launch_bounds__(kTnThreads, 1)
           fail();
           break;
         }
-        if (i >= 1 && !mbar_wait(acc_empty, (uint32_t)((i - 1) & 1))) {  // the epilogue read the last item
+        tc_fence_after();
+        const uint32_t aa = smem_u32(a_slot(i));
+        bool ok = true;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          ok = ok && (i == 0 || mbar_wait(&acc_empty[h], (uint32_t)((i - 1) & 1)));  // the last item's half is read
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t va = smem_u32(base + kTnOffV + h * kTnVTile);
+#pragma unroll
+          for (int ks = 0; ks < 2; ++ks)
+            mma_i8(tmem + h * 256, umma_desc_sw64(aa + 32 * ks), umma_desc_sw128(va + 32 * ks), TcIdesc<S8>::value,
+                   ks > 0 ? 1u : 0u);
+          mma_commit(&acc_full[h]);
+        }
+        if (!ok) {
           fail();
           break;
         }
-        tc_fence_after();
-        const uint32_t aa = smem_u32(a_slot(i));
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          const uint32_t va = smem_u32(base + kTnOffV + g * kTnVTile);
-#pragma unroll
-          for (int ks = 0; ks < 2; ++ks)
-            mma_i8(tmem + g * 256, umma_desc_sw64(aa + 32 * ks), umma_desc_sw128(va + 32 * ks),
-                   TcIdesc<S8>::value, ks > 0 ? 1u : 0u);
-        }
-        mma_commit(acc_full);
         mma_commit(&freed[i % kTnSlots]);
       }
       mma_commit(all_done);
       if (!mbar_wait(all_done, 0)) fail();
     }
   } else {
-    // ---------------- epilogue: warp w reads TMEM lanes 32 (w % 4).., slots 16 (w / 4)..
+    // ---------------- epilogue: warp w reads TMEM lanes 32 (w % 4).., slots 8 (w / 4).. of each half
     // row = (ring element jl, witness bb), witness fastest: a warp's 32 rows
     // are 32 consecutive What_T entries of one slot
     const uint32_t q = warp & 3, part = warp >> 2;
     const uint32_t row = 32 * q + lane;
     const uint32_t jl = row / p.BB, bb = row % p.BB;
-    for (uint64_t i = 0; i < n_my; ++i) {
+    const size_t stride = (size_t)p.m * p.b_pad;  // one slot t
+    bool ok = true;
+    for (uint64_t i = 0; i < n_my && ok; ++i) {
       const uint64_t item = blockIdx.x + i * gridDim.x;
       const uint32_t jb = (uint32_t)(item % p.nblk), bt = (uint32_t)(item / p.nblk);
-      const uint32_t b = bt * p.BB + bb;
-      {
+      const uint32_t b = bt * p.BB + bb, j = jb * p.R + jl;
+      const bool valid = b < p.b_pad && j < p.m;
+#pragma unroll 1
+      for (uint32_t h = 0; h < 2; ++h) {
         // warp-uniform decision: the TMEM loads below are .sync.aligned
-        const bool ok = !*abort_flag && mbar_wait(acc_full, (uint32_t)(i & 1));
-        if (!__all_sync(0xffffffffu, ok)) {
+        ok = !*abort_flag && mbar_wait(&acc_full[h], (uint32_t)(i & 1));
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
           fail();
           break;
         }
         tc_fence_after();
-        const uint32_t j = jb * p.R + jl;
-        const bool valid = b < p.b_pad && j < p.m;
-        const size_t stride = (size_t)p.m * p.b_pad;  // one slot t
-        uint64_t* dst = p.what_t + (size_t)(16 * part) * stride + (size_t)j * p.b_pad + b;
-#pragma unroll 1
-        for (int tb = 0; tb < 2; ++tb) {
-          const uint32_t t0 = 16 * part + 8 * tb;
-          uint32_t d[8][8];
+        uint32_t d[8][8];
 #pragma unroll
-          for (int l = 0; l < 8; ++l) tmem_ld8(tmem + ((32 * q) << 16) + (l >> 2) * 256 + (l & 3) * 64 + t0, d[l]);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (tb == 1) {
-            // this warp's accumulator columns are all in registers: the next
-            // item's MMAs may overwrite them while the fold runs
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty);
-          }
+        for (int l = 0; l < 8; ++l) tmem_ld8(tmem + ((32 * q) << 16) + h * 256 + l * 32 + 8 * part, d[l]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        // the columns are in registers: the next item's MMAs may overwrite them
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[h]);
+        uint64_t v[8];
+        gl_fold_limbs8(d, v);
+        uint64_t* dst = p.what_t + (size_t)(32 * h + 8 * part) * stride + (size_t)j * p.b_pad + b;
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            if (valid) *dst = tn_fold(d, u);
-            dst += stride;
-          }
-        }
+        for (int u = 0; u < 8; ++u)
+          if (valid) dst[u * stride] = v[u];
       }
     }
   }
@@ -655,7 +631,7 @@ int tc_commit(lc_tc_tables* t, const void* w, bool s8, size_t batch, uint64_t* o
 }
 
 
-// The limb tiles of V in their shared-memory image: tile g, row n = 64 (l - 4g) + t,
+// The limb tiles of V in their shared-memory image: tile h, row n = 32 l + t - 32 h,
 // 16-byte chunk c16 of the 128-byte row at n*128 + ((c16 ^ (n & 7)) << 4);
 // bytes 0..63 hold limb l of V[t][c], bytes 64..127 are zero.
 static void tn_build_image(std::vector<uint8_t>& img) {
@@ -673,7 +649,7 @@ static void tn_build_image(std::vector<uint8_t>& img) {
   const uint64_t psi = powp(7, (kGlP - 1) >> 7);  // primitive 128th root (generator 7)
   for (int g = 0; g < 2; ++g)
     for (int n = 0; n < 256; ++n) {
-      const int l = 4 * g + n / 64, t = n % 64;
+      const int l = n / 32, t = 32 * g + n % 32;
       for (int c = 0; c < 64; ++c) {
         const uint64_t v = powp(psi, (uint64_t)((2 * t + 1) * c) % 128);
         const int c16 = c / 16;

@@ -121,6 +121,47 @@ LC_D void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// Eight outputs sum_l 2^(8l) D_l mod p (p = 2^64 - 2^32 + 1, |D_l| <= 256 * 128 *
+// 255, so D_l + 2^8 D_(l+1) fits int32), each as a 64-bit value congruent mod p
+// but not necessarily canonical: every reader of the witness transforms -- the
+// byte-limb slot products and the 160-bit integer products -- takes any 64-bit
+// representative.  A = D0 + 2^8 D1 + 2^16 D2 + 2^24 D3 and B (limbs 4..7) are
+// exact in int64 (below 2^47.1).  With hB:lB = B (hB signed) and X = A - hB,
+//   A + 2^32 B == X + 2^32 (hB + lB)   (2^64 == 2^32 - 1),
+// so the low word is X's and the high word s + lB with s = hi(X) + hB, |s| < 2^17.
+// That sum leaves [0, 2^32) by k = 1 or -1 only when its low word lies within
+// 2^18 of the ends (2^-13 of the outputs); then k (2^32 - 1) is added, which
+// stays inside [0, 2^64).
+LC_D void gl_fold_limbs8(const uint32_t (&d)[8][8], uint64_t (&out)[8]) {
+  uint32_t hi[8], lo[8];
+  int32_t s[8];
+  bool edge = false;
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const int32_t p01 = (int32_t)d[0][u] + (int32_t)d[1][u] * 256;
+    const int32_t p23 = (int32_t)d[2][u] + (int32_t)d[3][u] * 256;
+    const int32_t p45 = (int32_t)d[4][u] + (int32_t)d[5][u] * 256;
+    const int32_t p67 = (int32_t)d[6][u] + (int32_t)d[7][u] * 256;
+    const int64_t A = (int64_t)p23 * 65536 + p01;
+    const int64_t B = (int64_t)p67 * 65536 + p45;
+    const int32_t hB = (int32_t)(B >> 32);
+    const int64_t X = A - hB;
+    s[u] = (int32_t)(X >> 32) + hB;
+    lo[u] = (uint32_t)X;
+    hi[u] = (uint32_t)B + (uint32_t)s[u];
+    edge |= hi[u] + 0x40000u < 0x80000u;
+  }
+#pragma unroll
+  for (int u = 0; u < 8; ++u) out[u] = (uint64_t)hi[u] << 32 | lo[u];
+  if (edge) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int k = s[u] >= 0 ? (int)(hi[u] < (uint32_t)s[u]) : -(int)(hi[u] >= (uint32_t)s[u]);
+      out[u] += (uint64_t)(int64_t)k * 0xFFFFFFFFull;
+    }
+  }
+}
+
 // ------------------------------------------------------------------ host side
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

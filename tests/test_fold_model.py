@@ -93,3 +93,38 @@ def test_crt_lane_fold_matches_modulo():
                 assert y <= m32 and y < 2 * q  # the 32-bit sum does not wrap
                 got = min(y, (y - q) & m32)
                 assert got == (x[0] + 256 * x[1] + 65536 * x[2] + 16777216 * x[3]) % q
+
+
+def fold_words(d):
+    """``gl_fold_limbs8`` (lzx_b200/csrc/tcgen05.cuh): the same value by 32-bit words, the rare wrap on its own path."""
+    def s32(x):
+        assert -(1 << 31) <= x < (1 << 31)
+        return x
+    p = [s32(d[2 * i] + 256 * d[2 * i + 1]) for i in range(4)]
+    a, b = 65536 * p[1] + p[0], 65536 * p[3] + p[2]
+    hb, lb = b >> 32, b & 0xFFFFFFFF
+    x = a - hb
+    s = (x >> 32) + hb
+    hi = (lb + s) & 0xFFFFFFFF
+    out = hi << 32 | (x & 0xFFFFFFFF)
+    k = (1 if hi < s else 0) if s >= 0 else (-1 if hi >= (s & 0xFFFFFFFF) else 0)
+    if not (hi + 0x40000) & 0xFFFFFFFF < 0x80000:
+        assert k == 0, "a wrap leaves the high word within 2^18 of its ends"
+    assert 0 <= out + k * EPS <= M64
+    return out + k * EPS
+
+
+def test_word_fold_is_congruent_and_in_range():
+    rng = np.random.default_rng(13)
+    lim = 256 * 128 * 255
+    cases = [[0] * 8, [lim] * 8, [-lim] * 8, [lim, -lim] * 4, [-lim, lim] * 4,
+             [0, 0, 0, 0, -lim, -lim, -lim, -lim], [lim, lim, lim, lim, -lim, 0, 0, 0]]
+    cases += rng.integers(-lim, lim + 1, size=(20000, 8)).tolist()
+    cases += rng.choice([-lim, -1, 0, 1, lim], size=(5000, 8)).tolist()
+    # high words next to the wrap: limbs 4..7 that cancel to a few units
+    small = rng.integers(-3, 4, size=(5000, 8))
+    small[:, :4] = rng.integers(-lim, lim + 1, size=(5000, 4))
+    cases += small.tolist()
+    for d in cases:
+        d = [int(x) for x in d]
+        assert fold_words(d) % P == sum(x << (8 * l) for l, x in enumerate(d)) % P, d
