@@ -141,7 +141,9 @@ typedef struct lc_ajtai_key lc_ajtai_key;
 
 /* `matrix`: the k*m entries A[i][j] in coefficient form, row-major
  * (entry (i,j) at (i*m + j)*n), residues of the plan's element type; host
- * memory, or device memory when matrix_on_device != 0.  Replaces the
+ * memory, or device memory when matrix_on_device != 0 (ready in the order of
+ * the legacy default stream; only read during the call, which is synchronous).
+ * Replaces the
  * cached-NTT part of AjtaiPublicKey::from_seed (ajtai.rs:91-96); the seed
  * expansion (uniform_from_seed, ring.rs:102-180) runs on the device in
  * lc_ajtai_key_from_seed, or on the host before this call. */

@@ -60,8 +60,13 @@ class _DeviceKey:
     def __init__(self, plan, k: int, m: int, matrix, flags: int = 0):
         h = C.c_void_p()
         if _is_torch_cuda(matrix):
+            import torch
             matrix = matrix.contiguous()
             ptr, on_dev = C.c_void_p(matrix.data_ptr()), 1
+            # the key is built on the legacy default stream, which does not wait for torch's other streams
+            stream = torch.cuda.current_stream()
+            if stream.cuda_stream:
+                stream.synchronize()
         else:
             matrix = np.ascontiguousarray(matrix)
             ptr, on_dev = matrix.ctypes.data_as(C.c_void_p), 0

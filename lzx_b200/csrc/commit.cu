@@ -1179,15 +1179,6 @@ template <class A, class S, int LOG_N, int LOG_V>
 static int launch_commit_fused(lc_ajtai_key* key, const S* w, size_t batch, void* out, cudaStream_t st) {
   using C = FusedCommitCfg<A, LOG_N, LOG_V>;
   constexpr uint32_t N = 1u << LOG_N;
-  // accumulators for the largest batch of this key, zeroed once; every call
-  // leaves them zero again
-  if (!key->d_fused) {
-    const size_t bytes = 16 + kFusedMaxBatch * key->k * N * 16;
-    int rc = grow(&key->d_fused, &key->fused_bytes, bytes);
-    if (rc) return rc;
-    rc = map_cuda(cudaMemsetAsync(key->d_fused, 0, bytes, st));
-    if (rc) return rc;
-  }
   auto kern = commit_fused_kernel<A, S, LOG_N, LOG_V>;
   static std::atomic<uint64_t> attr_done{0};
   {
@@ -1408,77 +1399,94 @@ int key_create_check(const lc_ntt_plan* plan, uint32_t k, uint32_t m, uint32_t f
   return LC_OK;
 }
 
-// A key from the coefficient-form matrix in `tmp` (device memory holding
-// k*m*n residues, row-major (i, j)), which the call takes over: it is
-// transformed in place, transposed into the key's Ahat_T and freed, on every
-// return path.  One device synchronisation reports the kernels' errors.
-int key_create_from(const lc_ntt_plan* plan, uint32_t k, uint32_t m, void* tmp, uint32_t flags,
+// The key's block: `ahat` bytes of NTT(A) (0 for a view), the accumulators of
+// the single-launch commit for the largest batch it takes (log_n 6..8; every
+// call leaves them zero) and the two error words.  Queues the zeroing.
+static int key_block(lc_ajtai_key* key, const lc_ntt_plan* plan, size_t ahat) {
+  const size_t fused =
+      key->log_n >= 6 && key->log_n <= 8 ? 16 + kFusedMaxBatch * (size_t)key->k * key->n * 16 : 0;
+  ahat = (ahat + 255) / 256 * 256;
+  if (cudaGetDevice(&key->device) != cudaSuccess) return map_cuda(cudaGetLastError());
+  key->block_bytes = ahat + fused + 16;
+  int rc = block_alloc(&key->d_block, key->block_bytes);
+  if (rc) return rc;
+  char* p = static_cast<char*>(key->d_block);
+  if (ahat) key->d_ahat_t = p;
+  if (fused) key->d_fused = p + ahat;
+  key->d_err = reinterpret_cast<uint32_t*>(p + ahat + fused);
+  rc = map_cuda(cudaMemsetAsync(p + ahat, 0, fused + 16, nullptr));
+  return rc ? rc : plan_share(plan, key->d_err + 1, &key->plan);
+}
+
+template <class A, class E>
+static int key_transform(const lc_ajtai_key* key, const E* matrix) {
+  E* dst = static_cast<E*>(key->d_ahat_t);
+  switch (key->log_n) {
+    case 6: return launch_witness_to<A, 6, 3, E>(key, matrix, key->k, kIPad, dst, nullptr);
+    case 7: return launch_witness_to<A, 7, 4, E>(key, matrix, key->k, kIPad, dst, nullptr);
+    case 8: return launch_witness_to<A, 8, 4, E>(key, matrix, key->k, kIPad, dst, nullptr);
+    default: return LC_ERR_UNSUPPORTED;
+  }
+}
+
+// A key from the coefficient-form matrix `matrix` (memory of the current
+// device, k*m*n residues, row-major (i, j), 16-byte aligned).  NTT(A) in the
+// layout Ahat_T[t][j][16] is the witness transform of A's rows as a batch of 16
+// (log_n 6..8, one launch); other degrees transform a copy and transpose it.
+// One synchronisation reports the kernels' errors.
+int key_create_from(const lc_ntt_plan* plan, uint32_t k, uint32_t m, const void* matrix, uint32_t flags,
                     lc_ajtai_key** out) {
   lc_ajtai_key* key = new (std::nothrow) lc_ajtai_key();
-  if (!key) {
-    cudaFree(tmp);
-    return LC_ERR_OUT_OF_MEMORY;
-  }
+  if (!key) return LC_ERR_OUT_OF_MEMORY;
+  block_users(1);
   key->k = k;
   key->m = m;
   key->a_m = m;
   key->log_n = plan->log_n;
   key->n = 1u << plan->log_n;
   key->wide = plan->kind == PlanKind::Goldilocks;
-  int rc;
-  if (key->wide)
-    rc = lc_ntt_plan_create_goldilocks(plan->log_n, &key->plan);
-  else
-    rc = lc_ntt_plan_create_u32(plan->log_n, plan->q, plan->two_adicity, plan->generator, 1, &key->plan);
-  if (rc) {
-    cudaFree(tmp);
-    delete key;
-    return rc;
-  }
-  const size_t eb = key->wide ? 8 : 4;
-  if (cudaMalloc(&key->d_ahat_t, (size_t)key->n * m * kIPad * eb) != cudaSuccess ||
-      cudaMalloc(&key->d_err, 4) != cudaSuccess) {
-    cudaGetLastError();
-    cudaFree(tmp);
-    lc_ajtai_key_destroy(key);
-    return LC_ERR_OUT_OF_MEMORY;
-  }
-  cudaMemsetAsync(key->d_err, 0, 4, nullptr);
+  const size_t eb = key->wide ? 8 : 4, bytes = (size_t)k * m * key->n * eb;
+  int rc = key_block(key, plan, (size_t)key->n * m * kIPad * eb);
+  void* tmp = nullptr;
   // the tensor-core witness transform's matrix image (once per device; a
   // failure only leaves the CUDA-core transform in use)
-  if (plan->kind == PlanKind::Goldilocks && plan->log_n == 6) tc_ntt_prepare();
-  // rotation-limb tables from the coefficient form (before it is transformed in place)
-  if (flags & LC_KEY_TENSOR_I8) {
-    rc = tc_tables_create(static_cast<const uint64_t*>(tmp), k, m, &key->tc);
-    if (rc) {
-      cudaFree(tmp);
-      lc_ajtai_key_destroy(key);
-      return rc;
-    }
-    key->engine = LC_ENGINE_TENSOR_I8;
+  if (!rc && plan->kind == PlanKind::Goldilocks && plan->log_n == 6) tc_ntt_prepare();
+  // rotation-limb tables from the coefficient form
+  if (!rc && (flags & LC_KEY_TENSOR_I8)) {
+    rc = tc_tables_create(static_cast<const uint64_t*>(matrix), k, m, &key->tc);
+    if (!rc) key->engine = LC_ENGINE_TENSOR_I8;
   }
   // cached NTT of every entry (AjtaiPublicKey::from_seed, ajtai.rs:91-96)
-  rc = run_ntt(key->plan, tmp, tmp, (size_t)k * m, false, nullptr);
   if (!rc) {
-    const size_t smem = (size_t)kIPad * key->n * eb;
-    if (smem > 48 * 1024) {
-      cudaFuncSetAttribute(key_transpose_kernel<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem);
-      cudaFuncSetAttribute(key_transpose_kernel<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem);
+    rc = plan->kind == PlanKind::Goldilocks
+             ? key_transform<Goldilocks>(key, static_cast<const uint64_t*>(matrix))
+             : plan->kind == PlanKind::U32Lazy ? key_transform<ShoupLazy>(key, static_cast<const uint32_t*>(matrix))
+                                               : key_transform<MontCanon>(key, static_cast<const uint32_t*>(matrix));
+    if (rc == LC_ERR_UNSUPPORTED) {
+      rc = block_alloc(&tmp, bytes);
+      if (!rc) rc = run_ntt(key->plan, matrix, tmp, (size_t)k * m, false, nullptr);
+      if (!rc) {
+        const size_t smem = (size_t)kIPad * key->n * eb;
+        if (smem > 48 * 1024) {
+          cudaFuncSetAttribute(key_transpose_kernel<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)smem);
+          cudaFuncSetAttribute(key_transpose_kernel<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)smem);
+        }
+        if (key->wide)
+          key_transpose_kernel<uint64_t><<<m, 256, smem>>>((const uint64_t*)tmp, (uint64_t*)key->d_ahat_t,
+                                                            k, m, key->n);
+        else
+          key_transpose_kernel<uint32_t><<<m, 256, smem>>>((const uint32_t*)tmp, (uint32_t*)key->d_ahat_t,
+                                                            k, m, key->n);
+        rc = map_cuda(cudaGetLastError());
+      }
     }
-    if (key->wide)
-      key_transpose_kernel<uint64_t><<<m, 256, smem>>>((const uint64_t*)tmp, (uint64_t*)key->d_ahat_t,
-                                                        k, m, key->n);
-    else
-      key_transpose_kernel<uint32_t><<<m, 256, smem>>>((const uint32_t*)tmp, (uint32_t*)key->d_ahat_t,
-                                                        k, m, key->n);
-    rc = map_cuda(cudaGetLastError());
   }
-  // one synchronisation: the kernels' errors, and nothing reads tmp any more
-  const cudaError_t e = cudaDeviceSynchronize();
+  // one synchronisation: the kernels' errors, and nothing reads the matrix any more
+  const cudaError_t e = cudaStreamSynchronize(nullptr);
   if (!rc) rc = map_cuda(e);
-  cudaFree(tmp);
+  block_free(tmp, bytes, key->device);
   if (rc) {
     lc_ajtai_key_destroy(key);
     return rc;
@@ -1504,26 +1512,44 @@ LC_API int lc_ajtai_key_create_ex(const lc_ntt_plan* plan, uint32_t k, uint32_t 
   if (rc) return rc;
   const size_t eb = plan->kind == PlanKind::Goldilocks ? 8 : 4;
   const size_t bytes = (size_t)k * m * ((size_t)1 << plan->log_n) * eb;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return lc::map_cuda(cudaGetLastError());
+  // aligned memory of this device is read in place; a host matrix, another
+  // device's or an unaligned one is copied first
+  if (matrix_on_device && ((uintptr_t)matrix & 15) == 0) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, matrix) != cudaSuccess)
+      cudaGetLastError();
+    else if (a.type == cudaMemoryTypeDevice && a.device == dev)
+      return lc::key_create_from(plan, k, m, matrix, flags, out);
+  }
   void* tmp = nullptr;
-  if (cudaMalloc(&tmp, bytes) != cudaSuccess) {
-    cudaGetLastError();
-    return LC_ERR_OUT_OF_MEMORY;
-  }
-  const cudaError_t e =
-      cudaMemcpy(tmp, matrix, bytes, matrix_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) {
-    cudaFree(tmp);
-    return map_cuda(e);
-  }
-  return lc::key_create_from(plan, k, m, tmp, flags, out);
+  rc = lc::block_alloc(&tmp, bytes);
+  if (rc) return rc;
+  rc = lc::map_cuda(
+      cudaMemcpy(tmp, matrix, bytes, matrix_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
+  if (!rc) rc = lc::key_create_from(plan, k, m, tmp, flags, out);
+  lc::block_free(tmp, bytes, dev);  // synchronous above: nothing queued reads it
+  return rc;
 }
 
 LC_API void lc_ajtai_key_destroy(lc_ajtai_key* key) {
   if (!key) return;
-  if (key->owns_ahat && key->d_ahat_t) cudaFree(key->d_ahat_t);
-  for (void* p : {key->d_what_t, key->d_partial, key->d_chat, key->d_wtmp, key->d_fused, (void*)key->d_grid, key->d_in,
-                  key->d_out, (void*)key->d_err})
+  for (void* p : {key->d_what_t, key->d_partial, key->d_chat, key->d_wtmp, (void*)key->d_grid, key->d_in, key->d_out})
     if (p) cudaFree(p);
+  if (key->d_block) {
+    // commits of this key may still run on any stream of its device
+    int cur = key->device;
+    cudaGetDevice(&cur);
+    if (cur != key->device) cudaSetDevice(key->device);
+    if (cudaDeviceSynchronize() == cudaSuccess)
+      block_free(key->d_block, key->block_bytes, key->device);
+    else {
+      cudaGetLastError();
+      cudaFree(key->d_block);
+    }
+    if (cur != key->device) cudaSetDevice(cur);
+  }
   if (key->host_stream) cudaStreamDestroy(key->host_stream);
   if (key->h_flags) cudaFreeHost(key->h_flags);
   if (key->h_stage_in) cudaFreeHost(key->h_stage_in);
@@ -1531,6 +1557,7 @@ LC_API void lc_ajtai_key_destroy(lc_ajtai_key* key) {
   if (key->plan) lc_ntt_plan_destroy(key->plan);
   tc_tables_destroy(key->tc);
   delete key;
+  block_users(-1);
 }
 
 LC_API int lc_ajtai_key_view(const lc_ajtai_key* parent, uint32_t k, uint32_t m, lc_ajtai_key** out) {
@@ -1538,6 +1565,7 @@ LC_API int lc_ajtai_key_view(const lc_ajtai_key* parent, uint32_t k, uint32_t m,
   *out = nullptr;
   lc_ajtai_key* key = new (std::nothrow) lc_ajtai_key();
   if (!key) return LC_ERR_OUT_OF_MEMORY;
+  block_users(1);
   key->k = k;
   key->m = m;
   key->a_m = parent->a_m;
@@ -1545,15 +1573,8 @@ LC_API int lc_ajtai_key_view(const lc_ajtai_key* parent, uint32_t k, uint32_t m,
   key->n = parent->n;
   key->wide = parent->wide;
   key->d_ahat_t = parent->d_ahat_t;
-  key->owns_ahat = false;
-  const lc_ntt_plan* pp = parent->plan;
-  int rc = key->wide ? lc_ntt_plan_create_goldilocks(pp->log_n, &key->plan)
-                     : lc_ntt_plan_create_u32(pp->log_n, pp->q, pp->two_adicity, pp->generator, 1, &key->plan);
-  if (!rc && cudaMalloc(&key->d_err, 4) != cudaSuccess) {
-    cudaGetLastError();
-    rc = LC_ERR_OUT_OF_MEMORY;
-  }
-  if (!rc) rc = map_cuda(cudaMemset(key->d_err, 0, 4));
+  int rc = key_block(key, parent->plan, 0);
+  if (!rc) rc = map_cuda(cudaStreamSynchronize(nullptr));  // the zeroing is done before any stream uses the view
   if (rc) {
     lc_ajtai_key_destroy(key);
     return rc;

@@ -68,6 +68,14 @@ struct HostPipeline {
   }
 };
 
+// Twiddle tables of a plan on one device, shared by the ring's plan and the
+// plans of the keys made from it.
+struct PlanTables {
+  void* block = nullptr;
+  int device = 0;
+  std::atomic<int> refs{1};
+};
+
 }  // namespace lc
 
 struct lc_ntt_plan {
@@ -79,7 +87,8 @@ struct lc_ntt_plan {
   uint32_t two_adicity[8] = {};
   uint32_t generator[8] = {};
   // one device block: the forward table, the inverse table, the error word
-  void* d_block = nullptr;
+  // (a key's plan shares the tables and has its error word in the key's block)
+  lc::PlanTables* tables = nullptr;
   void* d_tw_fwd = nullptr;
   void* d_tw_inv = nullptr;
   uint32_t tw_fwd_entries = 0;
@@ -99,9 +108,13 @@ struct lc_ajtai_key {
   lc_ntt_plan* plan = nullptr;  // owned copy of the ring's plan
   uint32_t k = 0, m = 0, n = 0, log_n = 0;
   bool wide = false;           // Goldilocks (u64) or u32
-  void* d_ahat_t = nullptr;    // [n][a_m][16]
+  // one device block: the cached NTT(A) (not in a view's), the single-launch
+  // commit's accumulators (log_n 6..8) and the error words of key and plan
+  void* d_block = nullptr;
+  size_t block_bytes = 0;
+  int device = 0;
+  void* d_ahat_t = nullptr;    // [n][a_m][16], in d_block or the parent's (lc_ajtai_key_view)
   uint32_t a_m = 0;            // ring elements per NTT slot of d_ahat_t (m, or the parent's m for a view)
-  bool owns_ahat = true;       // false for a view (lc_ajtai_key_view)
   // scratch, grown on demand
   void* d_what_t = nullptr;
   size_t what_bytes = 0;
@@ -111,8 +124,7 @@ struct lc_ajtai_key {
   size_t chat_bytes = 0;
   void* d_wtmp = nullptr;  // generic witness path: converted + transformed witnesses
   size_t wtmp_bytes = 0;
-  void* d_fused = nullptr;  // single-launch commit: ticket (16 B), then 128-bit accumulators
-  size_t fused_bytes = 0;
+  void* d_fused = nullptr;  // single-launch commit: ticket (16 B), then 128-bit accumulators; in d_block
   unsigned int* d_grid = nullptr;  // grid-barrier counter of the one-launch products + inverse NTT
   int fused = 1;            // one-launch forms: 0 never, 1 where faster, 2 every form (lc_ajtai_key_set_fused)
   bool last_fused = false;  // the last commit on this key ran as one launch
@@ -148,11 +160,20 @@ inline cudaError_t smem_attr_once(std::atomic<uint64_t>& done, K kern, size_t by
 }
 
 int device_sm_count();
-// Ajtai key creation (commit.cu): the argument check, and the creation from a
-// device buffer of the coefficient-form matrix that the call takes over.
+// Ajtai key creation (commit.cu): the argument check, and the creation from
+// the coefficient-form matrix in memory of the current device, 16-byte aligned
+// (read only; the call is synchronous).
 int key_create_check(const lc_ntt_plan* plan, uint32_t k, uint32_t m, uint32_t flags);
-int key_create_from(const lc_ntt_plan* plan, uint32_t k, uint32_t m, void* tmp, uint32_t flags,
+int key_create_from(const lc_ntt_plan* plan, uint32_t k, uint32_t m, const void* matrix_dev, uint32_t flags,
                     lc_ajtai_key** out);
+// A plan for the current device with `plan`'s moduli: its tables are shared when
+// they live on that device.  `d_err` (device, zeroed) is its error word then.
+int plan_share(const lc_ntt_plan* plan, uint32_t* d_err, lc_ntt_plan** out);
+// Device blocks of keys (lattice_cuda.cu): a few freed ones are kept for the
+// next key.  block_free wants a block that no queued work uses any more.
+int block_alloc(void** p, size_t bytes);
+void block_free(void* p, size_t bytes, int device);
+void block_users(int delta);  // live plans and keys: the last one frees what is kept
 int map_cuda(cudaError_t e);
 int run_ntt(const lc_ntt_plan* plan, const void* in, void* out, size_t count, bool inverse,
             cudaStream_t s);

@@ -241,19 +241,17 @@ LC_API int lc_ajtai_key_from_seed(const lc_ntt_plan* plan, uint32_t k, uint32_t 
   int rc = key_create_check(plan, k, m, 0);
   if (rc) return rc;
   const size_t count = (size_t)k * m, n = (size_t)1 << plan->log_n;
-  uint32_t* mat = nullptr;
-  if (cudaMalloc(&mat, count * n * 4) != cudaSuccess) {
-    cudaGetLastError();
-    return LC_ERR_OUT_OF_MEMORY;
-  }
-  // the expansion is written straight into the buffer the key is built from
+  void* mat = nullptr;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return map_cuda(cudaGetLastError());
+  rc = block_alloc(&mat, count * n * 4);
+  if (rc) return rc;
   static const uint8_t dom[7] = {'a', 'j', 't', 'a', 'i', '-', 'A'};
-  rc = uniform_from_seed(plan, dom, 7, seed, 32, 0, count, mat, nullptr);
-  if (rc) {
-    cudaFree(mat);
-    return rc;
-  }
-  return key_create_from(plan, k, m, mat, 0, out);  // takes over mat
+  rc = uniform_from_seed(plan, dom, 7, seed, 32, 0, count, static_cast<uint32_t*>(mat), nullptr);
+  if (!rc) rc = key_create_from(plan, k, m, mat, 0, out);  // synchronous
+  else cudaStreamSynchronize(nullptr);
+  block_free(mat, count * n * 4, dev);
+  return rc;
 }
 
 }  // extern "C"

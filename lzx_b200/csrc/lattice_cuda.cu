@@ -123,6 +123,79 @@ int device_sm_count() {
   return g_num_sms;
 }
 
+// ---------------------------------------------------------------- key blocks
+//
+// Making a key costs a cudaMalloc and destroying it a cudaFree, each a driver
+// call of 100 us and more that also serialises with the device's other work; a
+// verifier that derives its key from the seed on every call paid both several
+// times per call (from_seed + one commit, k = 2, m = 2000: 940 us).
+// Freed blocks of up to 32 MiB are kept for the next key, at most 64 MiB per
+// device; they go back to the driver when an allocation fails and when the last
+// plan and key of the process is destroyed.  A block enters the list only when
+// the device is idle (lc_ajtai_key_destroy), so its next user may use any stream.
+constexpr size_t kBlockKeepMax = (size_t)32 << 20, kBlockKeepTotal = (size_t)64 << 20;
+
+struct KeptBlock {
+  void* p;
+  size_t bytes;
+  int device;
+};
+static std::mutex g_block_mu;
+static std::vector<KeptBlock> g_blocks;
+static long g_block_users = 0;
+
+static size_t block_size(size_t bytes) {  // what may be kept has at most 1/8 unused
+  if (bytes > kBlockKeepMax) return bytes;
+  size_t step = 512;
+  while (step * 16 < bytes) step *= 2;
+  return (bytes + step - 1) / step * step;
+}
+
+// frees the kept blocks (of every device); g_block_mu held
+static void block_drain() {
+  for (const KeptBlock& b : g_blocks) cudaFree(b.p);
+  g_blocks.clear();
+}
+
+int block_alloc(void** p, size_t bytes) {
+  const size_t size = block_size(bytes);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return map_cuda(cudaGetLastError());
+  std::lock_guard<std::mutex> lk(g_block_mu);
+  for (size_t i = 0; i < g_blocks.size(); ++i)
+    if (g_blocks[i].bytes == size && g_blocks[i].device == dev) {
+      *p = g_blocks[i].p;
+      g_blocks.erase(g_blocks.begin() + (long)i);
+      return LC_OK;
+    }
+  if (cudaMalloc(p, size) == cudaSuccess) return LC_OK;
+  cudaGetLastError();
+  block_drain();
+  if (cudaMalloc(p, size) == cudaSuccess) return LC_OK;
+  cudaGetLastError();
+  *p = nullptr;
+  return LC_ERR_OUT_OF_MEMORY;
+}
+
+void block_free(void* p, size_t bytes, int device) {
+  if (!p) return;
+  const size_t size = block_size(bytes);
+  std::lock_guard<std::mutex> lk(g_block_mu);
+  size_t kept = size;
+  for (const KeptBlock& b : g_blocks)
+    if (b.device == device) kept += b.bytes;
+  if (size <= kBlockKeepMax && kept <= kBlockKeepTotal)
+    g_blocks.push_back({p, size, device});
+  else
+    cudaFree(p);
+}
+
+void block_users(int delta) {
+  std::lock_guard<std::mutex> lk(g_block_mu);
+  g_block_users += delta;
+  if (g_block_users == 0) block_drain();
+}
+
 int map_cuda(cudaError_t e) {
   if (e == cudaSuccess) return LC_OK;
   cudaGetLastError();
@@ -287,6 +360,37 @@ int run_ntt(const lc_ntt_plan* plan, const void* in, void* out, size_t count, bo
 
 }  // namespace lc
 
+namespace lc {
+int plan_share(const lc_ntt_plan* plan, uint32_t* d_err, lc_ntt_plan** out) {
+  *out = nullptr;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return map_cuda(cudaGetLastError());
+  if (dev != plan->tables->device)
+    return plan->kind == PlanKind::Goldilocks
+               ? lc_ntt_plan_create_goldilocks(plan->log_n, out)
+               : lc_ntt_plan_create_u32(plan->log_n, plan->q, plan->two_adicity, plan->generator, plan->num_moduli, out);
+  lc_ntt_plan* p = new (std::nothrow) lc_ntt_plan();
+  if (!p) return LC_ERR_OUT_OF_MEMORY;
+  p->kind = plan->kind;
+  p->log_n = plan->log_n;
+  p->num_moduli = plan->num_moduli;
+  std::copy(plan->q, plan->q + 8, p->q);
+  std::copy(plan->qinv, plan->qinv + 8, p->qinv);
+  std::copy(plan->two_adicity, plan->two_adicity + 8, p->two_adicity);
+  std::copy(plan->generator, plan->generator + 8, p->generator);
+  p->tables = plan->tables;
+  p->tables->refs.fetch_add(1, std::memory_order_relaxed);
+  p->d_tw_fwd = plan->d_tw_fwd;
+  p->d_tw_inv = plan->d_tw_inv;
+  p->tw_fwd_entries = plan->tw_fwd_entries;
+  p->tw_inv_entries = plan->tw_inv_entries;
+  p->tw_bytes = plan->tw_bytes;
+  p->d_err = d_err;
+  *out = p;
+  return LC_OK;
+}
+}  // namespace lc
+
 // ====================================================================== C ABI
 
 extern "C" {
@@ -343,16 +447,21 @@ static int finish_plan(lc_ntt_plan* plan, const std::vector<uint64_t>& fwd_raw_a
       for (uint32_t k = 0; k < ei; ++k) i[m * ei + k] = conv(inv_raw_all[m * ei + k]);
     }
   }
-  if (cudaMalloc(&plan->d_block, img.size() * 8) != cudaSuccess) {
+  plan->tables = new (std::nothrow) PlanTables();
+  if (!plan->tables) return LC_ERR_OUT_OF_MEMORY;
+  block_users(1);
+  uint64_t* block = nullptr;
+  if (cudaGetDevice(&plan->tables->device) != cudaSuccess || cudaMalloc(&block, img.size() * 8) != cudaSuccess) {
     cudaGetLastError();
-    plan->d_block = nullptr;
     return LC_ERR_OUT_OF_MEMORY;
   }
-  plan->d_tw_fwd = plan->d_block;
-  plan->d_tw_inv = static_cast<uint64_t*>(plan->d_block) + nf;
-  plan->d_err = reinterpret_cast<uint32_t*>(static_cast<uint64_t*>(plan->d_block) + nf + ni);
-  return map_cuda(cudaMemcpy(plan->d_block, img.data(), img.size() * 8, cudaMemcpyHostToDevice));
+  plan->tables->block = block;
+  plan->d_tw_fwd = block;
+  plan->d_tw_inv = block + nf;
+  plan->d_err = reinterpret_cast<uint32_t*>(block + nf + ni);
+  return map_cuda(cudaMemcpy(block, img.data(), img.size() * 8, cudaMemcpyHostToDevice));
 }
+
 
 LC_API int lc_ntt_plan_create_u32(uint32_t log_n, const uint32_t* q, const uint32_t* two_adicity,
                                   const uint32_t* generator, uint32_t num_moduli,
@@ -438,7 +547,12 @@ LC_API int lc_ntt_plan_create_goldilocks(uint32_t log_n, lc_ntt_plan** out) {
 
 LC_API void lc_ntt_plan_destroy(lc_ntt_plan* plan) {
   if (!plan) return;
-  if (plan->d_block) cudaFree(plan->d_block);  // both tables and the error word
+  PlanTables* t = plan->tables;
+  if (t && t->refs.fetch_sub(1, std::memory_order_acq_rel) == 1) {
+    if (t->block) cudaFree(t->block);  // both tables and the error word
+    delete t;
+    block_users(-1);
+  }
   if (plan->d_pow) cudaFree(plan->d_pow);
   plan->staging.release();
   delete plan;

@@ -121,3 +121,41 @@ def test_c_abi_key_from_seed():
         assert np.array_equal(out, host._dev.commit_array(w[None])[0])
     finally:
         L.lc_ajtai_key_destroy(h)
+
+
+@pytest.mark.parametrize("threads", [1, 4])
+def test_keys_made_and_destroyed_in_turn(threads):
+    """Keys made one after another (blocks of freed ones are reused), each
+    destroyed right after its commitment was queued on a stream of its own:
+    every commitment equals that of a key that stays, in one and in several
+    host threads, for degrees with and without the one-launch key transform."""
+    import threading
+    shapes = [(6, 2, 300), (6, 16, 40), (8, 2, 16), (5, 3, 33), (6, 2, 300)]
+    ring = {ld: RingConfig(Modulus32.Q_32, ld) for ld, _, _ in shapes}
+    rng = np.random.default_rng(3)
+    want, wit = {}, {}
+    for i, (ld, k, m) in enumerate(shapes):
+        wit[i] = torch.from_numpy(rng.integers(0, 3221225473, (2, m, 1 << ld), dtype=np.uint32).view(np.int32)).cuda()
+        stays = AjtaiPublicKey.from_seed(AjtaiParams(ring[ld], k, m, 1 << 20), bytes([i]) * 32)
+        want[i] = stays.commit_batch(wit[i]).cpu()
+        t = oracle.NttTables32(omod(Modulus32.Q_32), ld)
+        assert np.array_equal(stays._matrix, oracle.ajtai32_from_seed(t, k, m, bytes([i]) * 32)[0].reshape(-1, 1 << ld))
+    bad = []
+
+    def work():
+        stream = torch.cuda.Stream()
+        for rep in range(6):
+            for i, (ld, k, m) in enumerate(shapes):
+                with torch.cuda.stream(stream):
+                    key = AjtaiPublicKey.from_seed(AjtaiParams(ring[ld], k, m, 1 << 20), bytes([i]) * 32)
+                    got = key.commit_batch(wit[i])
+                    del key
+                    if not torch.equal(got.cpu(), want[i]):
+                        bad.append((rep, i))
+
+    pool = [threading.Thread(target=work) for _ in range(threads)]
+    for t in pool:
+        t.start()
+    for t in pool:
+        t.join()
+    assert not bad
