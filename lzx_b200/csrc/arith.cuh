@@ -204,6 +204,42 @@ LC_D uint64_t gl_mul(uint64_t a, uint64_t b) {
   return ((uint64_t)r1 << 32) | r0;
 }
 
+// a * b mod p in [0, 2^64), not necessarily canonical.
+LC_D uint64_t gl_mul_lazy(uint64_t a, uint64_t b) {
+  uint32_t r0, r1;
+  asm("{\n\t"
+      ".reg .u32 a0, a1, b0, b1, p0, p1, p2, p3, m, u0, u1, c, e;\n\t"
+      "mov.b64 {a0, a1}, %2;\n\t"
+      "mov.b64 {b0, b1}, %3;\n\t"
+      "mov.u32 e, 0xFFFFFFFF;\n\t"
+      "mul.lo.u32 p0, a0, b0;\n\t"
+      "mul.hi.u32 p1, a0, b0;\n\t"
+      "mul.lo.u32 p2, a1, b1;\n\t"
+      "mul.hi.u32 p3, a1, b1;\n\t"
+      "mad.lo.cc.u32 p1, a0, b1, p1;\n\t"
+      "madc.hi.cc.u32 p2, a0, b1, p2;\n\t"
+      "addc.u32 p3, p3, 0;\n\t"
+      "mad.lo.cc.u32 p1, a1, b0, p1;\n\t"
+      "madc.hi.cc.u32 p2, a1, b0, p2;\n\t"
+      "addc.u32 p3, p3, 0;\n\t"
+      "sub.cc.u32 p0, p0, p3;\n\t"
+      "subc.cc.u32 p1, p1, 0;\n\t"
+      "subc.u32 m, 0, 0;\n\t"
+      "sub.cc.u32 p0, p0, m;\n\t"
+      "subc.u32 p1, p1, 0;\n\t"
+      "sub.cc.u32 u0, 0, p2;\n\t"
+      "subc.u32 u1, p2, 0;\n\t"
+      "add.cc.u32 p0, p0, u0;\n\t"
+      "addc.cc.u32 p1, p1, u1;\n\t"
+      "addc.u32 c, 0, 0;\n\t"
+      "mad.lo.cc.u32 %0, c, e, p0;\n\t"
+      "addc.u32 %1, p1, 0;\n\t"
+      "}"
+      : "=r"(r0), "=r"(r1)
+      : "l"(a), "l"(b));
+  return ((uint64_t)r1 << 32) | r0;
+}
+
 // Canonical inputs -> canonical output.
 LC_D uint64_t gl_add(uint64_t a, uint64_t b) {
   uint64_t s = a + b;

@@ -178,6 +178,17 @@ int map_cuda(cudaError_t e);
 int run_ntt(const lc_ntt_plan* plan, const void* in, void* out, size_t count, bool inverse,
             cudaStream_t s);
 
+// Goldilocks transforms on the INT8 tensor cores (gl_ntt.cu), degrees 64 ..
+// 1024; gl_ntt_prepare makes the tables (once per device and degree,
+// synchronous, outside stream capture).  kGnMinValues: batches of fewer values
+// are faster in registers (ntt_tile_kernel): forward / inverse at 2^20 values
+// n = 64 10.4 / 12.1 us against 13.3 / 12.5, n = 128 12.8 / 15.6 against 14.1 /
+// 14.2, n = 256 13.9 / 17.5 against 13.6 / 13.6 (at 2^18: 9.5 / 10.3 against
+// 10.1 / 10.3); from n = 512 on one polynomial already takes 32 us there, 12
+// here, and the register form is not built.
+constexpr size_t kGnMinValues[11] = {0, 0, 0, 0, 0, 0, (size_t)1 << 21, (size_t)1 << 20, (size_t)1 << 19, 0, 0};
+int gl_ntt_prepare(uint32_t log_n);
+int gl_ntt(uint32_t log_n, const void* in, void* out, size_t count, bool inverse, uint32_t* err, cudaStream_t st);
 // Goldilocks, d = 64: build the rotation-limb tables from the coefficient
 // matrix [k][m][64] on the device (default stream); commit byte-digit
 // witnesses [batch][m][64] -> residues [batch][k][64] on `st`.

@@ -312,8 +312,12 @@ static int dispatch(int log_n, const NttParams& p, int variant, cudaStream_t s) 
     case 6: return launch_tile<A, 6, 3, INV>(p, variant, s);
     case 7: return launch_tile<A, 7, 4, INV>(p, variant, s);
     case 8: return launch_tile<A, 8, 4, INV>(p, variant, s);
-    case 9: return launch_tile<A, 9, 5, INV>(p, variant, s);
-    case 10: return launch_tile<A, 10, 5, INV>(p, variant, s);
+    case 9:
+      if constexpr (wide) return LC_ERR_UNSUPPORTED;  // gl_ntt
+      else return launch_tile<A, 9, 5, INV>(p, variant, s);
+    case 10:
+      if constexpr (wide) return LC_ERR_UNSUPPORTED;
+      else return launch_tile<A, 10, 5, INV>(p, variant, s);
     case 11:
       if constexpr (wide) return LC_ERR_UNSUPPORTED;
       else return launch_tile<A, 11, 6, INV>(p, variant, s);
@@ -348,6 +352,10 @@ static int run_ntt_moduli(const lc_ntt_plan* plan, uint32_t m0, uint32_t nm, con
     case PlanKind::U32Mont:
       return inverse ? dispatch<MontCanon, true>(ln, p, v, s) : dispatch<MontCanon, false>(ln, p, v, s);
     case PlanKind::Goldilocks:
+      if (v == 0 || ln >= 9) {
+        const int rc = gl_ntt(plan->log_n, in, out, count, inverse, plan->d_err, s);
+        if (rc != LC_ERR_UNSUPPORTED) return rc;
+      }
       return inverse ? dispatch<Goldilocks, true>(ln, p, v, s) : dispatch<Goldilocks, false>(ln, p, v, s);
   }
   return LC_ERR_INVALID_ARGUMENT;
@@ -537,6 +545,10 @@ LC_API int lc_ntt_plan_create_goldilocks(uint32_t log_n, lc_ntt_plan** out) {
   plan->tw_fwd_entries = (uint32_t)f.size();
   plan->tw_inv_entries = (uint32_t)i.size();
   int rc = finish_plan(plan, f, i);
+  if (rc == LC_OK && log_n >= 6) {
+    const int prep = gl_ntt_prepare(log_n);
+    if (log_n >= 9) rc = prep;  // below, the register transform does without
+  }
   if (rc != LC_OK) {
     lc_ntt_plan_destroy(plan);
     return rc;

@@ -335,3 +335,29 @@ def test_device_synth_matches_host_generator():
         got = t.cpu().numpy()
         want = host()
         assert np.array_equal(got.view(want.dtype), want), kind
+
+
+@pytest.mark.parametrize("log_n,count", [
+    (6, 1 << 15), (6, (1 << 15) + 63), (7, 1 << 13), (7, (1 << 13) + 1), (8, 1 << 11), (8, (1 << 11) + 15),
+    (9, 3), (9, 8), (9, 1185), (10, 3), (10, 4), (10, 5), (10, 599),
+])
+def test_goldilocks_tensor_core_batches(log_n, count):
+    """Batches that the tensor-core transform takes, a whole number of its
+    4096-value tiles and not, random and extreme residues, out of place and in
+    place, against the oracle."""
+    n = 1 << log_n
+    a = synth.synth_gl(31 + log_n, count, count * n).reshape(count, n)
+    p = (1 << 64) - (1 << 32) + 1
+    a[0], a[1], a[-1] = p - 1, 0, np.arange(n) % 2 * np.uint64(p - 1)
+    a[1, n - 1] = p - 1
+    ot, t = oracle.NttTablesGl(log_n), GoldilocksNttTables(log_n)
+    want = ot.forward_batch(a)
+    dev = torch.from_numpy(a.view(np.int64)).cuda()
+    out = torch.empty_like(dev)
+    t.forward_fast(dev, out)
+    assert np.array_equal(out.cpu().numpy().view(np.uint64), want)
+    t.inverse_fast(out)  # in place
+    assert np.array_equal(out.cpu().numpy().view(np.uint64), a)
+    t.inverse_fast(dev, out)
+    assert np.array_equal(out.cpu().numpy().view(np.uint64), ot.inverse_batch(a))
+    _lib.check(_lib.lib().lc_ntt_plan_check(t.handle, None), "lc_ntt_plan_check")
