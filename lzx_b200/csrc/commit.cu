@@ -146,12 +146,27 @@ __global__ void __launch_bounds__(NT)
       }
     }
   } else {
-    for (int e = threadIdx.x; e < PP * N; e += NT) {
-      const int pp = e / N, c = e % N;
-      const int jj = pp / BB, b = pp % BB;
-      T v = 0;
-      if (b0 + b < batch && j0 + jj < m) v = to_residue<T, S>(w[((size_t)(b0 + b) * m + j0 + jj) * N + c], q);
-      slots[pp * SS + c] = v;
+    // coefficient c of polynomials first, first + step, ..: compile-time tile
+    // positions, eight loads in flight
+    constexpr int STEP = NT >= N ? NT / N : 1, CSTEP = NT >= N ? N : NT;
+    for (int c = threadIdx.x % CSTEP; c < N; c += CSTEP) {
+      const uint32_t first = threadIdx.x / CSTEP;
+#pragma unroll
+      for (int g = 0; g < PP; g += 8 * STEP) {
+        T v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const uint32_t pp = g + u * STEP + first, jj = pp / BB, b = pp % BB;
+          v[u] = 0;
+          if (pp < PP && b0 + b < batch && j0 + jj < m)
+            v[u] = to_residue<T, S>(w[((size_t)(b0 + b) * m + j0 + jj) * N + c], q);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const uint32_t pp = g + u * STEP + first;
+          if (pp < PP) slots[pp * SS + c] = v[u];
+        }
+      }
     }
   }
   __syncthreads();
@@ -167,12 +182,15 @@ __global__ void __launch_bounds__(NT)
   }
   __syncthreads();
   // for each slot tt the tile's (jj, b) values are one contiguous run when BB == b_pad
-  for (int e = threadIdx.x; e < PP * N; e += NT) {
-    const int tt = e / PP, pp = e % PP;
-    const int jj = pp / BB, b = pp % BB;
-    if (b0 + b < b_pad && j0 + jj < m)
-      what_t[((size_t)tt * m + j0 + jj) * b_pad + b0 + b] = slots[pp * SS + tt];
-  }
+  static_assert(NT % PP == 0, "a thread keeps its polynomial");
+  const uint32_t pp = threadIdx.x % PP, jj = pp / BB, b = pp % BB;
+  if (b0 + b >= b_pad || j0 + jj >= m) return;
+  constexpr int TSTEP = NT / PP;
+  const T* src = slots + pp * SS + threadIdx.x / PP;
+  T* dst = what_t + ((size_t)(threadIdx.x / PP) * m + j0 + jj) * b_pad + b0 + b;
+  const size_t stride = (size_t)TSTEP * m * b_pad;
+#pragma unroll 8
+  for (int tt = 0; tt < N; tt += TSTEP, dst += stride) *dst = src[tt];
 }
 
 // Generic witness path (ring degrees without a fused kernel): element
@@ -786,6 +804,94 @@ __global__ void __launch_bounds__(256) sum_intt_kernel(const __grid_constant__ S
   }
 }
 
+// ------------------------------------------------------------------ limb sums + inverse NTT in one launch
+//
+// After the tensor-core products with few K splits: CTA (b, four rows i) forms
+// sum_{la,lw} 2^(8 (la + lw)) sum_split D[split][t][nt][(bl, lw)][(i, la)] mod q for
+// every slot t (a warp per slot and step; the four rows are 16 L consecutive
+// bytes of each column), straight into shared-memory slots, inverse-transforms
+// the four rows there and writes out[b][i][..].  The reduction and the inverse
+// transform as two launches took 9.6 + 9.2 us for 20 witnesses x 6 Goldilocks
+// rows of d = 128 and 8.8 + 4.4 for 16 x 2 Q_32 rows of d = 64, this 15.3 and 8.6
+// with 1024 threads (23 and 13 with 256: a warp's rounds of memory latency).
+// More splits go through slot_products_reduce_kernel, which spreads them over
+// warps.
+struct SlotFinishParams {
+  const int32_t* part;  // [splits][n][ntiles][ncta][128]
+  void* out;            // [batch][kappa][n]
+  const void* twi;
+  uint32_t kappa, batch, ncta, ntiles, splits, q, qinv;
+};
+constexpr uint32_t kSlotFinishSplits = 8;
+
+template <class A, int LOG_N, int LOG_V>
+__global__ void __launch_bounds__(1024) slot_finish_kernel(const __grid_constant__ SlotFinishParams p) {
+  using E = typename A::T;
+  using Tw = typename A::Tw;
+  using G = Geo<LOG_N, LOG_V>;
+  constexpr int N = G::N, SS = WitnessSlotStride<A, LOG_N>::value, L = sizeof(E);
+  __shared__ Tw twi[G::inv_entries()];
+  __shared__ __align__(16) E slots[4 * SS];
+  const uint32_t tid = threadIdx.x, threads = blockDim.x, warp = tid / 32, warps = threads / 32, lane = tid % 32;
+  for (uint32_t e = tid; e < (uint32_t)G::inv_entries(); e += threads) twi[e] = static_cast<const Tw*>(p.twi)[e];
+  const uint32_t quads = (p.kappa + 3) / 4, b = blockIdx.x / quads, iq = blockIdx.x % quads;
+  const uint32_t wpt = p.ncta / L, nt = b / wpt, bl = b % wpt;
+  const size_t tile = (size_t)p.ncta * 128, step = (size_t)N * p.ntiles * tile;  // one split
+  if constexpr (L == 8) {
+    // lane: la half and row in the low three bits, columns c and c + 4 above
+    const uint32_t seg = lane & 7, c = lane >> 3, shift = 8 * c + 32 * (seg & 1);
+    const int32_t* d = p.part + (size_t)nt * tile + (bl * 8 + c) * 128 + iq * 32 + seg * 4;
+    for (uint32_t t = warp; t < (uint32_t)N; t += warps) {
+      const int32_t* dt = d + (size_t)t * p.ntiles * tile;
+      uint64_t tk[8] = {};
+#pragma unroll 2
+      for (uint32_t sp = 0; sp < p.splits; ++sp) {
+        const uint4 x = *reinterpret_cast<const uint4*>(dt + sp * step);
+        const uint4 y = *reinterpret_cast<const uint4*>(dt + sp * step + 4 * 128);
+        tk[0] += x.x, tk[1] += x.y, tk[2] += x.z, tk[3] += x.w;
+        tk[4] += y.x, tk[5] += y.y, tk[6] += y.z, tk[7] += y.w;
+      }
+      unsigned __int128 v = 0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v += (unsigned __int128)tk[k] << (8 * k);
+      v = (unsigned __int128)gl_reduce128_lazy((uint64_t)(v >> 64), (uint64_t)v) << shift;
+      uint64_t r = gl_canon(gl_reduce128_lazy((uint64_t)(v >> 64), (uint64_t)v));
+#pragma unroll
+      for (int x : {1, 8, 16}) r = gl_add(r, __shfl_xor_sync(0xffffffffu, r, x));
+      if (c == 0 && !(seg & 1)) slots[(seg >> 1) * SS + t] = r;
+    }
+  } else {
+    // lane: row in the low two bits, column lw, then one of two slots
+    const uint32_t i = lane & 3, lw = (lane >> 2) & 3;
+    const int32_t* d = p.part + (size_t)nt * tile + (bl * 4 + lw) * 128 + iq * 16 + i * 4;
+    for (uint32_t t = 2 * warp + (lane >> 4); t < (uint32_t)N; t += 2 * warps) {
+      const int32_t* dt = d + (size_t)t * p.ntiles * tile;
+      uint64_t tk[4] = {};
+#pragma unroll 4
+      for (uint32_t sp = 0; sp < p.splits; ++sp) {
+        const uint4 x = *reinterpret_cast<const uint4*>(dt + sp * step);
+        tk[0] += x.x, tk[1] += x.y, tk[2] += x.z, tk[3] += x.w;
+      }
+      uint64_t v = 0;
+#pragma unroll
+      for (int k = 3; k >= 0; --k) v = ((v << 8) + tk[k]) % p.q;
+      v = (v << (8 * lw)) % p.q;
+      v += __shfl_xor_sync(0xffffffffu, v, 4);
+      v += __shfl_xor_sync(0xffffffffu, v, 8);
+      if (lw == 0) slots[i * SS + t] = (E)(v % p.q);
+    }
+  }
+  __syncthreads();
+  if (tid < 4 * G::T) {  // whole warps
+    const A ar = make_arith_q<A>(p.q, p.qinv);
+    transform_slot<A, LOG_N, LOG_V, true>(slots + (tid / G::T) * SS, twi, ar, tid % G::T);
+  }
+  __syncthreads();
+  E* out = static_cast<E*>(p.out) + ((size_t)b * p.kappa + 4 * iq) * N;
+  for (uint32_t e = tid; e < 4 * N; e += threads)
+    if (4 * iq + e / N < p.kappa) out[e] = slots[(e / N) * SS + e % N];
+}
+
 }  // namespace lc
 
 using namespace lc;
@@ -1084,17 +1190,55 @@ static int sum_intt(lc_ajtai_key* key, size_t batch, uint32_t b_pad, uint32_t sp
   return LC_ERR_UNSUPPORTED;
 }
 
+template <class A, int LOG_N, int LOG_V>
+static int launch_slot_finish(const lc_ajtai_key* key, size_t batch, const SlotPartials& sp, void* out,
+                              cudaStream_t st) {
+  SlotFinishParams prm{static_cast<const int32_t*>(key->d_partial), out, key->plan->d_tw_inv, key->k, (uint32_t)batch,
+                       sp.ncta, sp.ntiles, sp.splits, key->plan->q[0], key->plan->qinv[0]};
+  const size_t grid = batch * ((key->k + 3) / 4);
+  // few CTAs: each takes its slots in as few rounds of memory latency as it can
+  const unsigned threads = grid <= 2 * (size_t)std::max(1, device_sm_count()) ? 1024 : 256;
+  slot_finish_kernel<A, LOG_N, LOG_V><<<(unsigned)grid, threads, 0, st>>>(prm);
+  return map_cuda(cudaGetLastError());
+}
+
+template <class A>
+static int slot_finish_as(const lc_ajtai_key* key, size_t batch, const SlotPartials& sp, void* out, cudaStream_t st) {
+  switch (key->log_n) {
+    case 6: return launch_slot_finish<A, 6, 3>(key, batch, sp, out, st);
+    case 7: return launch_slot_finish<A, 7, 4>(key, batch, sp, out, st);
+    case 8: return launch_slot_finish<A, 8, 4>(key, batch, sp, out, st);
+    default: return LC_ERR_UNSUPPORTED;
+  }
+}
+
+// Limb sums and inverse transforms of the tensor-core products in one launch;
+// LC_ERR_UNSUPPORTED for many K splits and outside d = 64 .. 256.
+template <class E>
+static int slot_finish(const lc_ajtai_key* key, size_t batch, const SlotPartials& sp, void* out, cudaStream_t st) {
+  if (sp.splits > kSlotFinishSplits) return LC_ERR_UNSUPPORTED;
+  if constexpr (std::is_same<E, uint64_t>::value) return slot_finish_as<Goldilocks>(key, batch, sp, out, st);
+  else if (key->plan->kind == PlanKind::U32Lazy) return slot_finish_as<ShoupLazy>(key, batch, sp, out, st);
+  else return slot_finish_as<MontCanon>(key, batch, sp, out, st);
+}
+
 template <class E>
 static int commit_core(lc_ajtai_key* key, size_t batch, uint32_t b_pad, void* out, cudaStream_t st) {
   const uint32_t n = key->n, m = key->m, kappa = key->k;
   const uint32_t q = key->plan->q[0];
   // the per-slot products as byte-limb GEMMs on the tensor cores
   if (key->slot_products == LC_PRODUCTS_TENSOR) {
-    int rc = grow(&key->d_chat, &key->chat_bytes, (size_t)batch * kappa * n * sizeof(E));
-    if (rc) return rc;
-    rc = tc_slot_products(key->d_ahat_t, key->a_m, key->d_what_t, (uint32_t)sizeof(E), q, m, n, kappa, batch,
-                          b_pad, &key->d_partial, &key->partial_bytes, key->d_chat, key->d_err, st);
-    if (rc == LC_OK) return run_ntt(key->plan, key->d_chat, out, (size_t)batch * kappa, true, st);
+    SlotPartials sp{};
+    int rc = tc_slot_products(key->d_ahat_t, key->a_m, key->d_what_t, (uint32_t)sizeof(E), m, n, kappa, b_pad,
+                              &key->d_partial, &key->partial_bytes, &sp, key->d_err, st);
+    if (rc == LC_OK) {
+      rc = slot_finish<E>(key, batch, sp, out, st);
+      if (rc != LC_ERR_UNSUPPORTED) return rc;
+      rc = grow(&key->d_chat, &key->chat_bytes, (size_t)batch * kappa * n * sizeof(E));
+      if (!rc)
+        rc = tc_slot_reduce(key->d_partial, sp, (uint32_t)sizeof(E), q, n, kappa, batch, key->d_chat, st);
+      return rc ? rc : run_ntt(key->plan, key->d_chat, out, (size_t)batch * kappa, true, st);
+    }
     if (rc != LC_ERR_UNSUPPORTED) return rc;
   }
   const bool tiled = b_pad % kBTile == 0;

@@ -72,9 +72,10 @@ __global__ void gadget_kernel(const uint64_t* __restrict__ z, size_t count, uint
 // raw & (2^22-1), (raw >> 22) & (2^22-1), raw >> 44 at coefficients 3e..3e+2
 // of the flattened [elems][n] output; the rest zero.
 __global__ void pack_kernel(const uint64_t* __restrict__ v, size_t count, uint32_t* __restrict__ out,
-                            size_t total) {
+                            size_t first, size_t total) {
   constexpr uint64_t mask = (1ull << 22) - 1;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+  for (size_t i = first + blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
+       i += (size_t)gridDim.x * blockDim.x) {
     const size_t e = i / 3;
     uint32_t c = 0;
     if (e < count) {
@@ -83,6 +84,37 @@ __global__ void pack_kernel(const uint64_t* __restrict__ v, size_t count, uint32
       c = (uint32_t)(part == 0 ? raw & mask : part == 1 ? (raw >> 22) & mask : raw >> 44);
     }
     out[i] = c;
+  }
+}
+
+// The same for whole groups of 128 values (v and out 16-byte aligned): a warp
+// loads its group as 16-byte pairs, four values a lane, and exchanges the 384
+// limbs through shared memory into 16-byte stores.  Bound: HBM, 20 bytes per
+// value; 2.7 M values took 22 us with one limb per thread (three loads of every
+// value, a division each).
+__global__ void __launch_bounds__(256) pack_group_kernel(const ulonglong2* __restrict__ v, size_t groups,
+                                                         uint4* __restrict__ out) {
+  constexpr uint32_t mask = (1u << 22) - 1;
+  __shared__ uint4 s_buf[8][96];
+  const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  uint32_t* mine = reinterpret_cast<uint32_t*>(s_buf[warp] + 3 * lane);
+  for (size_t g = blockIdx.x * (size_t)8 + warp; g < groups; g += (size_t)gridDim.x * 8) {
+    const ulonglong2 x = __ldg(v + g * 64 + 2 * lane), y = __ldg(v + g * 64 + 2 * lane + 1);
+    const uint64_t raw[4] = {gl_canon(x.x), gl_canon(x.y), gl_canon(y.x), gl_canon(y.y)};
+    uint32_t c[12];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      c[3 * e] = (uint32_t)raw[e] & mask;
+      c[3 * e + 1] = (uint32_t)(raw[e] >> 22) & mask;
+      c[3 * e + 2] = (uint32_t)(raw[e] >> 44);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      reinterpret_cast<uint4*>(mine)[k] = make_uint4(c[4 * k], c[4 * k + 1], c[4 * k + 2], c[4 * k + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) out[g * 96 + 32 * k + lane] = s_buf[warp][32 * k + lane];
+    __syncwarp();
   }
 }
 
@@ -126,7 +158,14 @@ LC_API int lc_pack_field_elements(const uint64_t* values, size_t count, uint32_t
   if (out_elems < need) return LC_ERR_DIMENSION_MISMATCH;
   if (device_sm_count() <= 0) return LC_ERR_NO_DEVICE;
   const size_t total = out_elems * n;
-  pack_kernel<<<grid_for(total), 256, 0, (cudaStream_t)stream>>>(values, count, out, total);
+  cudaStream_t st = (cudaStream_t)stream;
+  const size_t groups = (((uintptr_t)values | (uintptr_t)out) & 15) ? 0 : count / 128;
+  if (groups)
+    pack_group_kernel<<<(unsigned)std::min<size_t>((groups + 7) / 8, (size_t)device_sm_count() * 8), 256, 0, st>>>(
+        reinterpret_cast<const ulonglong2*>(values), groups, reinterpret_cast<uint4*>(out));
+  // what is left of the values, and the zeros
+  if (groups * 384 < total)
+    pack_kernel<<<grid_for(total - groups * 384), 256, 0, st>>>(values, count, out, groups * 384, total);
   return map_cuda(cudaGetLastError());
 }
 

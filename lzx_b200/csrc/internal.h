@@ -207,13 +207,19 @@ int tc_commit(lc_tc_tables* t, const void* w, bool s8, size_t batch, uint64_t* o
 int tc_ntt_prepare();
 int tc_witness_ntt(const void* w, bool s8, size_t batch, uint32_t m, uint32_t b_pad, uint64_t* what_t,
                    uint32_t* err, cudaStream_t st);
-// Per-slot products Chat[b][i][t] = sum_j Ahat_T[t][j][i] What_T[t][j][b]
-// (mod q; Goldilocks for elem_bytes 8, the u32 modulus q for elem_bytes 4) as
-// exact byte-limb GEMMs on the INT8 tensor cores (n slots, m ring elements,
-// a_m the key's row stride); scratch grown in *part.  LC_ERR_UNSUPPORTED
-// unless a witness row of What_T (elem_bytes * b_pad bytes) is 32, 64, 128,
-// 256 or a multiple of 512 bytes.
-int tc_slot_products(const void* ahat_t, uint32_t a_m, const void* what_t, uint32_t elem_bytes, uint32_t q,
-                     uint32_t m, uint32_t n, uint32_t kappa, size_t batch, uint32_t b_pad, void** part,
-                     size_t* part_bytes, void* chat, uint32_t* err, cudaStream_t st);
+// Per-slot products sum_j Ahat_T[t][j][i] What_T[t][j][b] (elem_bytes 8:
+// Goldilocks, 4: a u32 modulus) as exact byte-limb GEMMs on the INT8 tensor
+// cores (n slots, m ring elements, a_m the key's row stride): int32 limb sums
+// in *part (grown), laid out as *sp says.  LC_ERR_UNSUPPORTED unless a witness
+// row of What_T (elem_bytes * b_pad bytes) is 32, 64, 128, 256 or a multiple of
+// 512 bytes.  tc_slot_reduce adds the splits and folds the limbs mod q into
+// Chat[b][i][t].
+struct SlotPartials {
+  uint32_t ncta, ntiles, splits;  // [splits][n][ntiles][ncta][128]
+};
+int tc_slot_products(const void* ahat_t, uint32_t a_m, const void* what_t, uint32_t elem_bytes, uint32_t m,
+                     uint32_t n, uint32_t kappa, uint32_t b_pad, void** part, size_t* part_bytes, SlotPartials* sp,
+                     uint32_t* err, cudaStream_t st);
+int tc_slot_reduce(const void* part, const SlotPartials& sp, uint32_t elem_bytes, uint32_t q, uint32_t n,
+                   uint32_t kappa, size_t batch, void* chat, cudaStream_t st);
 }  // namespace lc

@@ -1026,10 +1026,9 @@ static int launch_slot_products_n(uint32_t ncta, const CUtensorMap& amap, const 
   }
 }
 
-int tc_slot_products(const void* ahat_t, uint32_t a_m, const void* what_t, uint32_t elem_bytes, uint32_t q,
-                     uint32_t m, uint32_t n, uint32_t kappa, size_t batch, uint32_t b_pad, void** part,
-                     size_t* part_bytes, void* chat, uint32_t* err, cudaStream_t st) {
-  if (batch == 0) return LC_OK;
+int tc_slot_products(const void* ahat_t, uint32_t a_m, const void* what_t, uint32_t elem_bytes, uint32_t m,
+                     uint32_t n, uint32_t kappa, uint32_t b_pad, void** part, size_t* part_bytes, SlotPartials* sp,
+                     uint32_t* err, cudaStream_t st) {
   EncodeTiledFn enc = encode_fn();
   if (!enc || kappa > 16 || m == 0 || (elem_bytes != 8 && elem_bytes != 4)) return LC_ERR_UNSUPPORTED;
   // N tile: 512 bytes, or the whole row when it is 32, 64, 128 or 256 bytes
@@ -1094,18 +1093,23 @@ int tc_slot_products(const void* ahat_t, uint32_t a_m, const void* what_t, uint3
   const SpParams prm{static_cast<int32_t*>(*part), m, n, (uint32_t)ntiles, splits, jper, err};
   int rc = aw == 128 ? launch_slot_products_n<128>(ncta, amap, wmap, prm, st)
                      : launch_slot_products_n<64>(ncta, amap, wmap, prm, st);
-  if (rc) return rc;
+  *sp = {ncta, (uint32_t)ntiles, splits};
+  return rc;
+}
+
+int tc_slot_reduce(const void* part, const SlotPartials& sp, uint32_t elem_bytes, uint32_t q, uint32_t n,
+                   uint32_t kappa, size_t batch, void* chat, cudaStream_t st) {
   uint32_t wps = 1;
-  while (wps < 8 && wps < splits) wps *= 2;
+  while (wps < 8 && wps < sp.splits) wps *= 2;
   const size_t blocks = std::min<size_t>(((size_t)n * batch * wps + 7) / 8, 1u << 20);
   if (elem_bytes == 8)
     slot_products_reduce_kernel<uint64_t><<<(unsigned)blocks, 256, 0, st>>>(
-        static_cast<const int32_t*>(*part), static_cast<uint64_t*>(chat), n, kappa, (uint32_t)batch, ncta,
-        (uint32_t)ntiles, splits, wps, q);
+        static_cast<const int32_t*>(part), static_cast<uint64_t*>(chat), n, kappa, (uint32_t)batch, sp.ncta,
+        sp.ntiles, sp.splits, wps, q);
   else
     slot_products_reduce_kernel<uint32_t><<<(unsigned)blocks, 256, 0, st>>>(
-        static_cast<const int32_t*>(*part), static_cast<uint32_t*>(chat), n, kappa, (uint32_t)batch, ncta,
-        (uint32_t)ntiles, splits, wps, q);
+        static_cast<const int32_t*>(part), static_cast<uint32_t*>(chat), n, kappa, (uint32_t)batch, sp.ncta,
+        sp.ntiles, sp.splits, wps, q);
   return map_cuda(cudaGetLastError());
 }
 
