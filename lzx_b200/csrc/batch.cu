@@ -441,8 +441,11 @@ LC_D void finish_item(const LaneDesc& L, const SubJob* __restrict__ subs, uint32
   const A ar = make_arith_q<A>(L.q, L.qinv);
   const int grp = tid / Geo<LOG_N, LOG_V>::T;
   const uint32_t lt = tid % Geo<LOG_N, LOG_V>::T;
+  // whole warps: the transform synchronises its warp, so a warp with any of the
+  // job's rows runs all of its slots (at most 16, all there; the others unused)
+  const uint32_t wfirst = (uint32_t)(tid & ~31) / Geo<LOG_N, LOG_V>::T;
   for (uint32_t p0 = 0; p0 < J.kappa; p0 += GROUPS)
-    if (p0 + grp < J.kappa) transform_slot<A, LOG_N, LOG_V, true>(slots + (p0 + grp) * SS, tw, ar, lt);
+    if (p0 + wfirst < J.kappa) transform_slot<A, LOG_N, LOG_V, true>(slots + (p0 + grp) * SS, tw, ar, lt);
   __syncthreads();
   T* out = reinterpret_cast<T*>(J.out);
   for (uint32_t e = tid; e < J.kappa * N; e += kBatchThreads) out[e] = slots[(e / N) * SS + e % N];

@@ -217,3 +217,22 @@ def test_batch_argument_checks(mixed_classes):
     empty.check()
     with pytest.raises(LatticeCudaError):  # no such product mode
         empty.products = 7
+
+
+@pytest.mark.parametrize("products", [CommitBatch.PRODUCTS_TENSOR, CommitBatch.PRODUCTS_INT64])
+@pytest.mark.parametrize("kappa", [1, 2, 3, 5, 7, 9, 15, 16])
+def test_batch_row_counts(mixed_classes, kappa, products):
+    """Row counts that fill no whole warp of the finish launch's transforms."""
+    jobs = []
+    for c in (0, 1, 2, 3, 4):
+        cl = mixed_classes[c]
+        n = 37 + c
+        w = torch.from_numpy(synth.synth_i8(kappa, c, n * cl["d"]).reshape(n, cl["d"])).cuda()
+        dt = torch.int64 if cl["moduli"][0] is None else torch.int32
+        jobs.append(CommitJob(c, kappa, n, w, torch.empty((len(cl["keys"]), kappa, cl["d"]), dtype=dt, device="cuda")))
+    batch = CommitBatch([c["keys"] for c in mixed_classes], jobs, graph=False)
+    batch.products = products
+    batch.run()
+    batch.check()
+    for j in jobs:
+        assert torch.equal(j.out, one_by_one(mixed_classes, j)), (j.cls, kappa)
