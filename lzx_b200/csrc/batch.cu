@@ -694,6 +694,7 @@ __global__ void __launch_bounds__(TwCfg<EW, PN>::THREADS, 1)
         const LaneDesc& L = lanes[it.lane];
         const uint32_t d = 1u << L.log_n, passes = tw_limbs(L) * d / PN, kb = d > 128 ? d / 128 : 1;
         const CUtensorMap* vm = vmaps + it.lane;
+        tensormap_acquire(vm);
         for (uint32_t k = 0; k < passes && !*abort_flag; ++k, ++g) {
           if (g >= NS && !mbar_wait(&b_empty[g % NS], (uint32_t)(((g - NS) / NS) & 1))) {
             fail();
@@ -903,24 +904,34 @@ __global__ void __launch_bounds__(TwCfg<EW, PN>::THREADS, 1)
 // M = 128 (the key row's 16 x L bytes (i, la); u32 keys fill half and the
 // second A atom is a zero tile), N = 32 L bytes (b, lw), K = the chunk.  The
 // key rows Ahat[t][j][16] arrive by TMA (a 3-D map per lane: row bytes,
-// j < a_m, slot); the witness rows come from the staircase, where row j of
-// the block is the 32 L contiguous bytes at what[t Sp + Rp[j] + 32 blk]
-// (16-byte aligned) of which only the first cnt(j) - 32 blk jobs are active:
-// four gather warps copy them in 16-byte chunks with zero-filling cp.async
-// straight into the 128-byte-swizzled MN-major layout the MMA descriptor
-// reads (chunk c of row r at c ^ (r & 7)),
-// so the shorter jobs of a block contribute zeros and nothing outside the
-// staircase is read.  The epilogue (the same four warps) writes D, one
+// j < a_m, slot), and so do the witness rows: the staircase is cut into segments
+// of ring elements with the same number of active jobs (and at multiples of the
+// chunk), in which row j starts at a constant stride (16-byte aligned), so a 3-D
+// map per segment -- bytes of the active jobs, rows, slots -- loads 64 rows by
+// 128 bytes with the 128-byte swizzle of the MN-major layout the MMA reads; what
+// lies past the active jobs or the segment's rows reads as zero.  Stages start at
+// segment starts: the key rows past a segment's end meet zero witness rows there
+// and come again with the next segment.  The epilogue warps write D, one
 // [32 L columns][128 rows] int32 tile per item; the finish launch folds the
 // limb pairs over the block's chunks.
+//
+// Bound: HBM.  Gathering the rows with 16-byte cp.async copies (a shuffle of row
+// offsets and counts per copy) kept the shared-memory pipe 69 % busy: products
+// of 128 jobs up to 2^16 ring elements 1.95 (Goldilocks) and 3.37 ms (CRT
+// lanes), with the segment maps 0.93 and 2.28; the CRT lanes' 64-byte key rows
+// and mostly empty witness rows take the same TMA row requests (about three
+// cycles each) as full ones.
 constexpr int kTpRows = 64;            // ring elements per stage
 constexpr int kTpStages = 4;
-constexpr int kTpLag = 2;              // gather stages in flight before a stage is handed to the MMA
-constexpr int kTpAhead = 2;            // stages the staircase offsets are loaded ahead of their copies
-constexpr int kTpThreads = 192;        // warp 0 TMA, 1 MMA + TMEM, 2..5 gather + epilogue
+constexpr int kTpThreads = 192;        // warp 0 TMA, 1 MMA + TMEM, 2..5 epilogue
 
 struct TpItem {
   uint32_t lane, t, blk, chunk;
+  uint32_t seg, nst;  // first segment of the chunk, stages over all of its segments
+};
+
+struct TpSeg {
+  uint32_t j0, len;  // ring elements j0 .. j0 + len - 1
 };
 
 template <int EB>
@@ -949,13 +960,14 @@ struct TpIdesc {
 template <int EB>
 __global__ void __launch_bounds__(kTpThreads, 1)
     lane_products_tc_kernel(const TpItem* __restrict__ items, const LaneDesc* __restrict__ lanes,
-                            const SubJob* __restrict__ subs, const CUtensorMap* __restrict__ amaps, uint32_t* err) {
+                            const TpSeg* __restrict__ segs, const CUtensorMap* __restrict__ amaps,
+                            const CUtensorMap* __restrict__ smaps, uint32_t* err) {
   using C = TpCfg<EB>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* base =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + kTpStages * C::STAGE);
-  uint64_t* full = bars;                  // [4] key rows landed (tx) and 128 gather threads arrived
+  uint64_t* full = bars;                  // [4] stage landed (tx bytes)
   uint64_t* empty = bars + kTpStages;     // [4] the stage's MMAs finished
   uint64_t* done = bars + 2 * kTpStages;  // every MMA finished
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kTpStages + 1);
@@ -964,14 +976,11 @@ __global__ void __launch_bounds__(kTpThreads, 1)
   const TpItem it = items[blockIdx.x];
   const LaneDesc& L = lanes[it.lane];
   const uint32_t d = 1u << L.log_n;
-  const uint32_t nblk = subs[L.sub0 + kTpJobs * it.blk].n;  // the block's longest job
-  const uint32_t j0 = it.chunk * kTpChunk;
-  const uint32_t j1 = min(nblk, j0 + kTpChunk);
-  const int nst = (int)((j1 - j0 + kTpRows - 1) / kTpRows);
+  const int nst = (int)it.nst;
 
   if (tid == 0) {
     for (int s = 0; s < kTpStages; ++s) {
-      mbar_init(&full[s], 1 + 128);
+      mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
     mbar_init(done, 1);
@@ -1003,17 +1012,32 @@ __global__ void __launch_bounds__(kTpThreads, 1)
   int last_loaded = -1, last_mma = -1;
 
   if (warp == 0) {
-    // ---------------- TMA: key rows (i, la) of slot t
+    // ---------------- TMA: key rows (i, la) of slot t, witness rows of the block
     if (lane == 0) {
       const CUtensorMap* amap = amaps + it.lane;
+      uint32_t sg = it.seg, off = 0;
+      TpSeg cur = segs[sg];
+      tensormap_acquire(amap);
+      tensormap_acquire(smaps + sg);
       for (int s = 0; s < nst && !*abort_flag; ++s) {
         if (s >= kTpStages && !mbar_wait(&empty[s % kTpStages], (uint32_t)(((s - kTpStages) / kTpStages) & 1))) {
           fail();
           break;
         }
-        mbar_arrive_expect_tx(&full[s % kTpStages], (uint32_t)C::A_LOAD);
-        tma_load_3d(stage(s), amap, 0, (int)(j0 + kTpRows * s), (int)it.t, &full[s % kTpStages]);
+        uint64_t* bar = &full[s % kTpStages];
+        mbar_arrive_expect_tx(bar, (uint32_t)(C::A_LOAD + C::ATOMS * C::B_ATOM));
+        tma_load_3d(stage(s), amap, 0, (int)(cur.j0 + off), (int)it.t, bar);
+#pragma unroll
+        for (int a = 0; a < C::ATOMS; ++a)
+          tma_load_3d(stage(s) + C::A_BYTES + a * C::B_ATOM, smaps + sg, (int)(it.blk * C::NB + a * 128), (int)off,
+                      (int)it.t, bar);
         last_loaded = s;
+        off += kTpRows;
+        if (off >= cur.len && s + 1 < nst) {
+          cur = segs[++sg];
+          tensormap_acquire(smaps + sg);
+          off = 0;
+        }
       }
     }
   } else if (warp == 1) {
@@ -1038,78 +1062,8 @@ __global__ void __launch_bounds__(kTpThreads, 1)
       if (last_mma >= 0) mma_commit(done);
     }
   } else {
-    // ---------------- gather: warp g = warp - 2 fills rows 16 g .. 16 g + 15 of
-    // every stage in 16-byte chunks.  Row j of the block starts at
-    // what[t Sp + Rp[j] + 32 blk], 16-byte aligned; chunk k holds jobs
-    // 32 blk + k J .. + J - 1 (J = 16 / EB), of which the first
-    // cnt(j) - 32 blk - k J are active and copied, the rest zero-filled.
-    constexpr int J = 16 / EB;           // jobs per chunk
-    constexpr int CPR = C::NB / 16;      // chunks per row (16 or 8)
-    constexpr int RPI = 32 / CPR;        // rows per warp instruction (2 or 4)
-    const int g = warp - 2;
-    using E = typename std::conditional<EB == 8, uint64_t, uint32_t>::type;
-    const E* W = reinterpret_cast<const E*>(L.what) + (size_t)it.t * L.Sp + (size_t)kTpJobs * it.blk;
-    const uint32_t k = (uint32_t)lane % CPR, rsub = (uint32_t)lane / CPR;
-    const uint32_t boff = (k >> 3) * C::B_ATOM;  // swizzle atom of the chunk
-    const uint32_t kc = k & 7;
-    const int first_job = kTpJobs * (int)it.blk + (int)(k * J);
-    // R[jb .. jb + 16] (job counts) and Rp[jb .. jb + 15] (row starts) of a
-    // stage, loaded kTpAhead stages ahead (a register queue) so their
-    // latency hides behind the copies and waits of the stages between
-    auto offsets = [&](int s, uint64_t& r, uint64_t& rp) {
-      const uint32_t jb = j0 + kTpRows * s + 16 * g;
-      const bool in_r = s < nst && lane <= 16 && jb + lane <= L.n_max;
-      r = in_r ? __ldg(L.R + jb + lane) : 0;
-      rp = in_r ? __ldg(L.Rp + jb + lane) : 0;
-    };
-    uint64_t rq[kTpAhead], rpq[kTpAhead];
-#pragma unroll
-    for (int a = 0; a < kTpAhead; ++a) offsets(a, rq[a], rpq[a]);
-    bool ok = true;
-    for (int s = 0; s < nst; ++s) {
-      if (*abort_flag) {
-        ok = false;
-        break;
-      }
-      if (s >= kTpStages && !mbar_wait(&empty[s % kTpStages], (uint32_t)(((s - kTpStages) / kTpStages) & 1))) {
-        fail();
-        ok = false;
-        break;
-      }
-      const uint32_t jb = j0 + kTpRows * s + 16 * g;
-      const uint64_t rl = rq[0], rpl = rpq[0];
-#pragma unroll
-      for (int a = 0; a + 1 < kTpAhead; ++a) {
-        rq[a] = rq[a + 1];
-        rpq[a] = rpq[a + 1];
-      }
-      offsets(s + kTpAhead, rq[kTpAhead - 1], rpq[kTpAhead - 1]);
-      const uint32_t sb = smem_u32(stage(s)) + C::A_BYTES + boff;
-#pragma unroll
-      for (int rr = 0; rr < 16; rr += RPI) {
-        const int r = rr + (int)rsub;
-        const uint64_t r0 = __shfl_sync(0xffffffffu, rl, r);
-        const uint64_t r1 = __shfl_sync(0xffffffffu, rl, r + 1);
-        const uint64_t rp = __shfl_sync(0xffffffffu, rpl, r);
-        const uint32_t j = jb + r, row = 16 * g + r;
-        const int act = (j < j1) ? (int)(r1 - r0) - first_job : 0;  // active jobs from this chunk's first
-        const uint32_t bytes = act <= 0 ? 0u : act >= J ? 16u : (uint32_t)act * EB;
-        const uint32_t dst = sb + row * 128 + ((kc ^ (row & 7)) << 4);
-        cp_async16_zfill(dst, bytes ? (const void*)(W + rp + k * J) : L.what, bytes);
-      }
-      cp_async_commit();
-      if (s >= kTpLag) {
-        cp_async_wait<kTpLag>();
-        fence_proxy_async_smem();
-        mbar_arrive(&full[(s - kTpLag) % kTpStages]);
-      }
-    }
-    cp_async_wait<0>();
-    fence_proxy_async_smem();
-    if (ok)
-      for (int s = max(0, nst - kTpLag); s < nst; ++s) mbar_arrive(&full[s % kTpStages]);
     // ---------------- epilogue: lane = row (i, la); column = (b, lw)
-    const bool fin = ok && nst > 0 && !*abort_flag && mbar_wait(done, 0);
+    const bool fin = nst > 0 && !*abort_flag && mbar_wait(done, 0);
     if (__all_sync(0xffffffffu, fin)) {
       tc_fence_after();
       const uint32_t lq = warp & 3, row = 32 * lq + lane;
@@ -1200,6 +1154,8 @@ struct lc_batch {
   int32_t* d_tpart = nullptr;
   uint32_t* d_tchunk0 = nullptr;
   CUtensorMap* d_amaps = nullptr;
+  CUtensorMap* d_smaps = nullptr;         // per segment of the staircases
+  lc::TpSeg* d_segs = nullptr;
   lc::TpItem* d_titems = nullptr;
   uint64_t titems[2] = {0, 0};           // Goldilocks items, then u32 items
   std::vector<int32_t*> lane_tpart;
@@ -1225,14 +1181,15 @@ static void batch_free(lc_batch* b) {
   for (void* p : {(void*)b->d_lanes, (void*)b->d_subs, (void*)b->d_R, (void*)b->d_itemj, (void*)b->d_what,
                   (void*)b->d_partial, (void*)b->d_counters, (void*)b->d_err, (void*)b->d_citem,
                   (void*)b->d_cblk, (void*)b->d_tpart, (void*)b->d_tchunk0, (void*)b->d_amaps,
-                  (void*)b->d_titems, (void*)b->d_vmaps, (void*)b->d_twitems})
+                  (void*)b->d_titems, (void*)b->d_vmaps, (void*)b->d_twitems, (void*)b->d_smaps,
+                  (void*)b->d_segs})
     if (p) cudaFree(p);
   for (auto& v : b->vimgs) cudaFree(v.second);
   delete b;
 }
 
-// Tensor-core products: per lane a TMA map of its key rows, per 32-job block
-// the K chunks, the items (longest first, Goldilocks lanes then u32 lanes)
+// Tensor-core products: per lane a TMA map of its key rows and of every segment
+// of its staircase, per 32-job block the K chunks, the items (longest first, Goldilocks lanes then u32 lanes)
 // and the partial tiles.  Leaves tensor_ok false when a lane cannot run
 // there (no tensor-map encoder, or an element width other than 8 / 4 bytes).
 static int batch_tensor_setup(lc_batch* b) {
@@ -1240,9 +1197,11 @@ static int batch_tensor_setup(lc_batch* b) {
   if (!enc || b->lanes.empty()) return LC_OK;
   const size_t nl = b->lanes.size();
   std::vector<CUtensorMap> maps(nl);
+  std::vector<CUtensorMap> smaps;
+  std::vector<TpSeg> segs;
   std::vector<uint32_t> tchunk0;
   std::vector<size_t> tc_off(nl), part_off(nl);
-  std::vector<std::pair<uint32_t, TpItem>> items[2];  // (rows, item)
+  std::vector<std::pair<uint32_t, TpItem>> items[2];  // (stages, item)
   size_t part_elems = 0;
   for (size_t l = 0; l < nl; ++l) {
     const LaneDesc& L = b->lanes[l];
@@ -1256,6 +1215,29 @@ static int batch_tensor_setup(lc_batch* b) {
             CU_TENSOR_MAP_INTERLEAVE_NONE, aw == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return LC_OK;
+    // segments: constant count of active jobs, cut at multiples of the chunk
+    const std::vector<uint64_t>& R = b->R[l];
+    std::vector<uint32_t> chunk_seg;  // first segment of every chunk
+    const uint32_t pad = 16 / eb;
+    uint64_t row0 = 0;  // where the segment's first row starts, in entries
+    for (uint32_t j = 0; j < L.n_max;) {
+      const uint64_t cnt = R[j + 1] - R[j], stride = (cnt + pad - 1) / pad * pad;
+      uint32_t e = j + 1;
+      while (e < L.n_max && e % kTpChunk && R[e + 1] - R[e] == cnt) ++e;
+      if (j % kTpChunk == 0) chunk_seg.push_back((uint32_t)segs.size());
+      const cuuint64_t sdims[3] = {cnt * eb, e - j, d};
+      const cuuint64_t sstr[2] = {stride * eb, L.Sp * eb};
+      const cuuint32_t sbox[3] = {128, (cuuint32_t)kTpRows, 1};
+      CUtensorMap map;
+      if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, static_cast<char*>(L.what) + row0 * eb, sdims, sstr, sbox, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return LC_OK;
+      smaps.push_back(map);
+      segs.push_back({j, e - j});
+      row0 += stride * (e - j);
+      j = e;
+    }
     tc_off[l] = tchunk0.size();
     part_off[l] = part_elems;
     const uint32_t nblk = (L.nb + kTpJobs - 1) / kTpJobs;
@@ -1265,8 +1247,11 @@ static int batch_tensor_setup(lc_batch* b) {
       const uint32_t chunks = (nfirst + kTpChunk - 1) / kTpChunk;
       tchunk0.push_back(acc);
       for (uint32_t c = 0; c < chunks; ++c) {
-        const uint32_t rows = std::min(nfirst, (c + 1) * kTpChunk) - c * kTpChunk;
-        for (uint32_t t = 0; t < d; ++t) items[eb == 8 ? 0 : 1].push_back({rows, TpItem{(uint32_t)l, t, blk, c}});
+        const uint32_t j1 = std::min(nfirst, (c + 1) * kTpChunk);
+        uint32_t nst = 0;  // nfirst and the chunk's end are segment ends
+        for (size_t g = chunk_seg[c]; g < segs.size() && segs[g].j0 < j1; ++g) nst += (segs[g].len + kTpRows - 1) / kTpRows;
+        for (uint32_t t = 0; t < d; ++t)
+          items[eb == 8 ? 0 : 1].push_back({nst, TpItem{(uint32_t)l, t, blk, c, chunk_seg[c], nst}});
       }
       acc += chunks;
     }
@@ -1279,6 +1264,8 @@ static int batch_tensor_setup(lc_batch* b) {
   for (auto& v : items)
     for (auto& x : v) flat.push_back(x.second);
   if (cudaMalloc(&b->d_amaps, nl * sizeof(CUtensorMap)) != cudaSuccess ||
+      cudaMalloc(&b->d_smaps, std::max<size_t>(1, smaps.size()) * sizeof(CUtensorMap)) != cudaSuccess ||
+      cudaMalloc(&b->d_segs, std::max<size_t>(1, segs.size()) * sizeof(TpSeg)) != cudaSuccess ||
       cudaMalloc(&b->d_tchunk0, tchunk0.size() * 4) != cudaSuccess ||
       cudaMalloc(&b->d_titems, std::max<size_t>(1, flat.size()) * sizeof(TpItem)) != cudaSuccess ||
       cudaMalloc(&b->d_tpart, std::max<size_t>(256, part_elems * 4)) != cudaSuccess) {
@@ -1286,6 +1273,8 @@ static int batch_tensor_setup(lc_batch* b) {
     return LC_ERR_OUT_OF_MEMORY;
   }
   cudaMemcpy(b->d_amaps, maps.data(), nl * sizeof(CUtensorMap), cudaMemcpyHostToDevice);
+  cudaMemcpy(b->d_smaps, smaps.data(), smaps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice);
+  cudaMemcpy(b->d_segs, segs.data(), segs.size() * sizeof(TpSeg), cudaMemcpyHostToDevice);
   cudaMemcpy(b->d_tchunk0, tchunk0.data(), tchunk0.size() * 4, cudaMemcpyHostToDevice);
   if (!flat.empty()) cudaMemcpy(b->d_titems, flat.data(), flat.size() * sizeof(TpItem), cudaMemcpyHostToDevice);
   b->titems[0] = items[0].size();
@@ -1508,10 +1497,10 @@ static int batch_launch(lc_batch* b, cudaStream_t st) {
     // one CTA per item; grids above 2^31 - 1 items are refused at creation
     if (b->titems[0])
       lane_products_tc_kernel<8><<<(unsigned)b->titems[0], kTpThreads, TpCfg<8>::SMEM, st>>>(
-          b->d_titems, b->d_lanes, b->d_subs, b->d_amaps, b->d_err);
+          b->d_titems, b->d_lanes, b->d_segs, b->d_amaps, b->d_smaps, b->d_err);
     if (b->titems[1])
       lane_products_tc_kernel<4><<<(unsigned)b->titems[1], kTpThreads, TpCfg<4>::SMEM, st>>>(
-          b->d_titems + b->titems[0], b->d_lanes, b->d_subs, b->d_amaps, b->d_err);
+          b->d_titems + b->titems[0], b->d_lanes, b->d_segs, b->d_amaps, b->d_smaps, b->d_err);
   } else {
     product_kernel<uint64_t><<<grid, kBatchThreads, 0, st>>>(p);
     product_kernel<uint32_t><<<grid, kBatchThreads, 0, st>>>(p);

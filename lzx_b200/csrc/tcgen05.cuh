@@ -37,6 +37,13 @@ LC_D uint64_t umma_desc_noswz(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   return d;
 }
 
+// Acquire of a tensor map that lies in global memory and was copied there from
+// the host: without it the thread's TMA loads may use a descriptor cached from an
+// earlier map at the same address (its box, and so the bytes that arrive, may differ).
+LC_D void tensormap_acquire(const CUtensorMap* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+}
+
 LC_D void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(

@@ -219,6 +219,37 @@ def test_batch_argument_checks(mixed_classes):
         empty.products = 7
 
 
+@pytest.mark.parametrize("cls", [0, 2, 3, 4])
+@pytest.mark.parametrize("lengths", [
+    [1], [64, 64], [65, 64, 63, 62, 1],
+    list(range(1, 41)),                       # every row its own segment, two blocks
+    [80] * 33 + [17] * 3 + [16] * 30 + [1],   # a block that ends where another segment starts
+], ids=["one", "equal", "around64", "steps", "blocks"])
+def test_batch_segments(mixed_classes, cls, lengths):
+    """Staircases whose segments (runs of ring elements with the same number of
+    active jobs) are shorter and longer than a 64-row stage: tensor-core
+    products equal to the integer form's."""
+    cl = mixed_classes[cls]
+    rng = np.random.default_rng(len(lengths))
+    jobs = []
+    for n in lengths:
+        w = torch.from_numpy(rng.integers(-128, 128, (n, cl["d"])).astype(np.int8)).cuda()
+        dt = torch.int64 if cl["moduli"][0] is None else torch.int32
+        jobs.append(CommitJob(0, int(rng.integers(1, 9)), n, w, None))
+        jobs[-1].out = torch.empty((len(cl["keys"]), jobs[-1].kappa, cl["d"]), dtype=dt, device="cuda")
+    batch = CommitBatch([cl["keys"]], jobs, graph=False)
+    got = {}
+    for mode in (CommitBatch.PRODUCTS_TENSOR, CommitBatch.PRODUCTS_INT64):
+        batch.products = mode
+        for j in jobs:
+            j.out.fill_(-1)
+        batch.run()
+        batch.check()
+        got[mode] = [j.out.cpu() for j in jobs]
+    for a, b in zip(got[CommitBatch.PRODUCTS_TENSOR], got[CommitBatch.PRODUCTS_INT64]):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("products", [CommitBatch.PRODUCTS_TENSOR, CommitBatch.PRODUCTS_INT64])
 @pytest.mark.parametrize("kappa", [1, 2, 3, 5, 7, 9, 15, 16])
 def test_batch_row_counts(mixed_classes, kappa, products):
