@@ -1033,7 +1033,14 @@ static int witness_ntt(lc_ajtai_key* key, const S* w, size_t batch, uint32_t b_p
     }
   }
   if constexpr (!std::is_same<S, uint32_t>::value) {
-    if (kind == PlanKind::Goldilocks) return witness_ntt_as<Goldilocks, S>(key, w, batch, b_pad, st);
+    if (kind == PlanKind::Goldilocks) {
+      if constexpr (std::is_same<S, uint64_t>::value) {
+        const int rc = gl_witness_ntt(key->log_n, w, batch, key->m, b_pad, reinterpret_cast<uint64_t*>(key->d_what_t),
+                                      key->d_err, st);
+        if (rc != LC_ERR_UNSUPPORTED) return rc;
+      }
+      return witness_ntt_as<Goldilocks, S>(key, w, batch, b_pad, st);
+    }
   }
   if constexpr (!std::is_same<S, uint64_t>::value) {
     if (kind == PlanKind::U32Lazy) return witness_ntt_as<ShoupLazy, S>(key, w, batch, b_pad, st);

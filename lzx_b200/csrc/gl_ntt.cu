@@ -53,14 +53,24 @@ constexpr int kGnTile = 4096;  // values per tile
 constexpr int kGnFold1 = 16, kGnFold2 = 8, kGnLoad = 4;  // warps folding pass A and pass B, loader warps
 constexpr int kGnThreads = 32 * (kGnFold1 + kGnFold2 + kGnLoad + 1);
 
-template <int LOG_N1, int LOG_N2>
+// WIT: the commitment's witness transform -- polynomials (j, b), b fastest, read
+// from w[b][j][n] and written to What_T[t][j][b_pad], zeros in the columns from
+// batch on.  Pass B's rows then run along the polynomials, so that a warp's
+// lanes store a run of one slot.  The register form does the butterflies of the
+// padding too and is bound by its multiplications: whole commitments of kappa =
+// 4 went from 1177 to 970 us (d = 128, m = 8192, 128 witnesses), from 120 to 110
+// (d = 128, m = 3001, 20) and from 1289 to 1096 (d = 256, m = 4096, 128).  Not
+// taken, as they were slower or no faster: d = 64 (952 us against 950 at m =
+// 16384, 73 against 77 at m = 4096 and 20 witnesses) and byte digits, which this
+// loader reads one by one (1131 us against 1293 at d = 128).
+template <int LOG_N1, int LOG_N2, bool WIT>
 struct GnCfg {
   static constexpr int N1 = 1 << LOG_N1, N2 = 1 << LOG_N2, N = N1 * N2;
   static constexpr int P = kGnTile / N;  // polynomials per tile
   static constexpr int RA = kGnTile / N1, RB = kGnTile / N2;  // rows of the passes
-  // operand: 16-byte K chunk c (two values) of row r at c * LB + 16 r; one pad
-  // chunk per column of chunks keeps the stores of pass B's operand off one bank
-  static constexpr int LBA = RA * 16 + 16, LBB = RB * 16 + 16;
+  // operand: 16-byte K chunk c (two values) of row r at c * LB + 16 r; the pad per
+  // column of chunks spreads a warp's stores of pass B's operand over the banks
+  static constexpr int LBA = RA * 16 + 16, LBB = RB * 16 + (WIT ? 16 * (32 / N2) : 16);
   static constexpr int VA = 64 * N1 * N1, VB = 64 * N2 * N2;  // (8N)^2 bytes
   static constexpr int OFF_VB = VA, OFF_W = OFF_VB + VB, OFF_A = OFF_W + 8 * N;
   static constexpr int OFF_B = OFF_A + N1 / 2 * LBA, OFF_BAR = OFF_B + N2 / 2 * LBB;
@@ -82,6 +92,7 @@ struct GnParams {
   unsigned long long count;  // polynomials
   uint32_t tiles;
   uint32_t* err;
+  uint32_t m, batch, b_pad;  // witness transforms
 };
 
 // Four values sum_l 2^(8l) D_l mod p, 0 <= D_l <= 256 * 255^2, as any 64-bit
@@ -102,9 +113,9 @@ LC_D void gl_fold_bytes4(const uint32_t (&d)[8][4], uint64_t (&out)[4]) {
   }
 }
 
-template <int LOG_N1, int LOG_N2>
+template <int LOG_N1, int LOG_N2, bool WIT>
 __global__ void __launch_bounds__(kGnThreads, 1) gl_ntt_kernel(const __grid_constant__ GnParams p) {
-  using C = GnCfg<LOG_N1, LOG_N2>;
+  using C = GnCfg<LOG_N1, LOG_N2, WIT>;
   constexpr int N1 = C::N1, N2 = C::N2, N = C::N;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* base =
@@ -171,7 +182,9 @@ __global__ void __launch_bounds__(kGnThreads, 1) gl_ntt_kernel(const __grid_cons
     const uint32_t row = mb * 128 + 32 * q + lane, poly = row / N2, y2 = row % N2;
     const uint64_t* w = reinterpret_cast<const uint64_t*>(base + C::OFF_W) + x0 * N2 + y2;
     const uint32_t col = tmem + ((32 * q) << 16) + mb * 8 * N1 + x0;
-    unsigned char* dst = base + C::OFF_B + (y2 >> 1) * C::LBB + (poly * N1 + x0) * 16 + (y2 & 1) * 8;
+    constexpr int XS = WIT ? 16 * C::P : 16;  // pass B's row: x1 P + poly or poly N1 + x1
+    unsigned char* dst =
+        base + C::OFF_B + (y2 >> 1) * C::LBB + (WIT ? poly * 16 : poly * N1 * 16) + x0 * XS + (y2 & 1) * 8;
     for (uint32_t k = 0; k < mine; ++k) {
       if (!wait(acc1_full, k & 1)) break;
       tc_fence_after();
@@ -194,7 +207,7 @@ __global__ void __launch_bounds__(kGnThreads, 1) gl_ntt_kernel(const __grid_cons
         if (h == 0 && k > 0) ok = wait(b_empty, (k - 1) & 1);  // the last tile's operand is read
         if (ok) {
 #pragma unroll
-          for (int u = 0; u < 4; ++u) *reinterpret_cast<uint64_t*>(dst + 16 * (4 * h + u)) = v[u];
+          for (int u = 0; u < 4; ++u) *reinterpret_cast<uint64_t*>(dst + XS * (4 * h + u)) = v[u];
         }
       }
       if (!ok) break;
@@ -207,6 +220,14 @@ __global__ void __launch_bounds__(kGnThreads, 1) gl_ntt_kernel(const __grid_cons
     const uint32_t q = warp & 3, part = (warp - kGnFold1) >> 2;
     for (uint32_t k = 0; k < mine; ++k) {
       const uint32_t tile = blockIdx.x + k * gridDim.x, np = polys(tile);
+      uint32_t j0 = 0, b0 = 0;  // ring element and witness of the tile's first polynomial
+      size_t place = 0;         // of this lane's polynomial in a slot
+      if constexpr (WIT) {
+        const unsigned long long f = (unsigned long long)tile * C::P;
+        j0 = (uint32_t)(f / p.batch), b0 = (uint32_t)(f % p.batch);
+        const uint32_t b = b0 + (32 * q + lane) % C::P;
+        place = (size_t)(j0 + b / p.batch) * p.b_pad + b % p.batch;
+      }
       if (!wait(acc2_full, k & 1)) break;
       tc_fence_after();
 #pragma unroll
@@ -224,11 +245,35 @@ __global__ void __launch_bounds__(kGnThreads, 1) gl_ntt_kernel(const __grid_cons
         }
         uint64_t v[4];
         gl_fold_bytes4(d, v);
-        const uint32_t row = mb * 128 + 32 * q + lane, poly = row / N1, x1 = row % N1;
-        if (poly < np) {
-          uint64_t* dst = p.out + ((size_t)tile * C::P + poly) * N + x1 + N1 * x0;
+        const uint32_t row = mb * 128 + 32 * q + lane;
+        if constexpr (WIT) {  // any representative: the products read bytes or reduce 160 bits
+          const uint32_t poly = row % C::P, x1 = row / C::P;
+          const size_t stride = (size_t)p.m * p.b_pad;
+          if (poly < np) {
+            uint64_t* dst = p.out + (x1 + N1 * x0) * stride + place;
 #pragma unroll
-          for (int u = 0; u < 4; ++u) dst[N1 * u] = gl_canon(v[u]);
+            for (int u = 0; u < 4; ++u) dst[N1 * u * stride] = v[u];
+          }
+        } else {
+          const uint32_t poly = row / N1, x1 = row % N1;
+          if (poly < np) {
+            uint64_t* dst = p.out + ((size_t)tile * C::P + poly) * N + x1 + N1 * x0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) dst[N1 * u] = gl_canon(v[u]);
+          }
+        }
+      }
+      if constexpr (WIT) {
+        // the zero columns of the ring elements whose first witness is in the tile,
+        // a power of two of lanes to a slot
+        const uint32_t pad = p.b_pad - p.batch, t2 = tid - 32 * kGnFold1;
+        if (pad) {
+          const uint32_t lg = pad > 16 ? 5 : 32 - __clz(pad - 1), c0 = t2 & ((1u << lg) - 1);
+          for (uint32_t j = j0 + (b0 ? 1 : 0); (unsigned long long)j * p.batch < (unsigned long long)tile * C::P + np; ++j)
+            for (uint32_t t = t2 >> lg; t < (uint32_t)N; t += (32 * kGnFold2) >> lg) {
+              uint64_t* z = p.out + ((size_t)t * p.m + j) * p.b_pad + p.batch;
+              for (uint32_t c = c0; c < pad; c += 1u << lg) z[c] = 0;
+            }
         }
       }
     }
@@ -239,6 +284,11 @@ __global__ void __launch_bounds__(kGnThreads, 1) gl_ntt_kernel(const __grid_cons
     const uint32_t t = tid - 32 * kLoadWarp;
     for (uint32_t k = 0; k < mine; ++k) {
       const uint32_t tile = blockIdx.x + k * gridDim.x, np = polys(tile);
+      uint32_t j0 = 0, b0 = 0;
+      if constexpr (WIT) {
+        const unsigned long long f = (unsigned long long)tile * C::P;
+        j0 = (uint32_t)(f / p.batch), b0 = (uint32_t)(f % p.batch);
+      }
       bool ok = true;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -247,7 +297,12 @@ __global__ void __launch_bounds__(kGnThreads, 1) gl_ntt_kernel(const __grid_cons
         for (int e = 0; e < PER; ++e) {
           const uint32_t pr = t + 32 * kGnLoad * (h * PER + e);
           const uint32_t y2 = pr % N2, c = pr / N2 % (N1 / 2), poly = pr / (N / 2);
-          const uint64_t* src = p.in + ((size_t)tile * C::P + poly) * N + 2 * c * N2 + y2;
+          size_t at = (size_t)tile * C::P + poly;
+          if constexpr (WIT) {
+            const uint32_t b = b0 + poly;
+            at = (size_t)(b % p.batch) * p.m + j0 + b / p.batch;
+          }
+          const uint64_t* src = p.in + at * N + 2 * c * N2 + y2;
           const bool in = poly < np;
           v[e][0] = in ? src[0] : 0;  // plain loads: out may be in
           v[e][1] = in ? src[N2] : 0;
@@ -403,17 +458,30 @@ int gl_ntt_prepare(uint32_t log_n) {
   return LC_OK;
 }
 
-template <int LOG_N1, int LOG_N2>
+template <int LOG_N1, int LOG_N2, bool WIT>
 static int gn_launch(GnParams& p, const unsigned char* table, bool inverse, cudaStream_t st) {
-  using C = GnCfg<LOG_N1, LOG_N2>;
-  auto kern = gl_ntt_kernel<LOG_N1, LOG_N2>;
+  using C = GnCfg<LOG_N1, LOG_N2, WIT>;
+  auto kern = gl_ntt_kernel<LOG_N1, LOG_N2, WIT>;
   static std::atomic<uint64_t> attr_done{0};
   const cudaError_t e = smem_attr_once(attr_done, kern, C::SMEM);
   if (e != cudaSuccess) return map_cuda(e);
   p.table = reinterpret_cast<const uint4*>(table + (inverse ? C::TABLE : 0));
-  p.tiles = (uint32_t)((p.count + C::P - 1) / C::P);
+  const unsigned long long tiles = (p.count + C::P - 1) / C::P;
+  if (tiles >> 32) return LC_ERR_UNSUPPORTED;
+  p.tiles = (uint32_t)tiles;
   kern<<<std::min<uint32_t>(p.tiles, (uint32_t)std::max(1, device_sm_count())), kGnThreads, C::SMEM, st>>>(p);
   return map_cuda(cudaGetLastError());
+}
+
+int gl_witness_ntt(uint32_t log_n, const uint64_t* w, size_t batch, uint32_t m, uint32_t b_pad, uint64_t* what_t,
+                   uint32_t* err, cudaStream_t st) {
+  int dev = 0;
+  if ((log_n != 7 && log_n != 8) || (batch * m) << log_n < kGnMinWitness) return LC_ERR_UNSUPPORTED;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return LC_ERR_UNSUPPORTED;
+  const unsigned char* table = g_gn_table[dev][log_n].load();
+  if (!table) return LC_ERR_UNSUPPORTED;
+  GnParams p{w, what_t, nullptr, (unsigned long long)batch * m, 0, err, m, (uint32_t)batch, b_pad};
+  return log_n == 7 ? gn_launch<4, 3, true>(p, table, false, st) : gn_launch<4, 4, true>(p, table, false, st);
 }
 
 int gl_ntt(uint32_t log_n, const void* in, void* out, size_t count, bool inverse, uint32_t* err, cudaStream_t st) {
@@ -422,13 +490,13 @@ int gl_ntt(uint32_t log_n, const void* in, void* out, size_t count, bool inverse
   if (count << log_n < kGnMinValues[log_n]) return LC_ERR_UNSUPPORTED;
   const unsigned char* table = g_gn_table[dev][log_n].load();
   if (!table) return LC_ERR_UNSUPPORTED;
-  GnParams p{static_cast<const uint64_t*>(in), static_cast<uint64_t*>(out), nullptr, count, 0, err};
+  GnParams p{static_cast<const uint64_t*>(in), static_cast<uint64_t*>(out), nullptr, count, 0, err, 0, 1, 0};
   switch (log_n) {
-    case 6: return gn_launch<3, 3>(p, table, inverse, st);
-    case 7: return gn_launch<4, 3>(p, table, inverse, st);
-    case 8: return gn_launch<4, 4>(p, table, inverse, st);
-    case 9: return gn_launch<5, 4>(p, table, inverse, st);
-    default: return gn_launch<5, 5>(p, table, inverse, st);
+    case 6: return gn_launch<3, 3, false>(p, table, inverse, st);
+    case 7: return gn_launch<4, 3, false>(p, table, inverse, st);
+    case 8: return gn_launch<4, 4, false>(p, table, inverse, st);
+    case 9: return gn_launch<5, 4, false>(p, table, inverse, st);
+    default: return gn_launch<5, 5, false>(p, table, inverse, st);
   }
 }
 

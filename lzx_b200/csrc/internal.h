@@ -189,6 +189,13 @@ int run_ntt(const lc_ntt_plan* plan, const void* in, void* out, size_t count, bo
 constexpr size_t kGnMinValues[11] = {0, 0, 0, 0, 0, 0, (size_t)1 << 21, (size_t)1 << 20, (size_t)1 << 19, 0, 0};
 int gl_ntt_prepare(uint32_t log_n);
 int gl_ntt(uint32_t log_n, const void* in, void* out, size_t count, bool inverse, uint32_t* err, cudaStream_t st);
+// The commitment's witness transform the same way, n = 128 and 256:
+// What_T[n][m][b_pad] from the residues w[batch][m][n].  LC_ERR_UNSUPPORTED below
+// kGnMinWitness values: 2^19 and 2^20 values fill the SMs with a tile or two and
+// were up to 2 us slower than the register form, 2^21 are 1 to 2 us faster.
+constexpr size_t kGnMinWitness = (size_t)1 << 21;
+int gl_witness_ntt(uint32_t log_n, const uint64_t* w, size_t batch, uint32_t m, uint32_t b_pad, uint64_t* what_t,
+                   uint32_t* err, cudaStream_t st);
 // Goldilocks, d = 64: build the rotation-limb tables from the coefficient
 // matrix [k][m][64] on the device (default stream); commit byte-digit
 // witnesses [batch][m][64] -> residues [batch][k][64] on `st`.

@@ -192,6 +192,21 @@ def test_goldilocks_other_degrees(log_d, kappa):
     assert np.array_equal(got[idx], oracle_gl_commit(A, kappa, m, W[idx], d=d))
 
 
+@pytest.mark.parametrize("log_d,m,batch", [(7, 8209, 2), (7, 821, 20), (7, 251, 67), (7, 128, 129), (8, 2749, 3),
+                                           (8, 391, 21), (8, 4096, 2), (8, 4097, 2)])
+def test_goldilocks_witness_gemm_shapes(log_d, m, batch):
+    """Witness transforms of residues as byte GEMMs over the polynomials (j, b):
+    tiles that end in the middle of a ring element or cover several, padded
+    batches, a partial last tile, residues at the end of the range."""
+    d, kappa = 1 << log_d, 2
+    A, key = gl_key(kappa, m, d=d, seed=m + batch)
+    W = synth.synth_gl(9, batch, batch * m * d).reshape(batch, m, d)
+    W[:, ::17] = P - 1
+    got = key.commit(W)
+    assert np.array_equal(key.commit(W), got)
+    assert np.array_equal(got, oracle_gl_commit(A, kappa, m, W, d=d))
+
+
 def test_goldilocks_config3_full_batch():
     """kappa=16, 2^16 witness elements, 128 int8 witnesses (the bench workload):
     every commitment of the batch checked against the oracle."""
