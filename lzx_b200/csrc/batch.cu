@@ -107,6 +107,9 @@ struct BatchParams {
   uint32_t lane_split;  // first lane of a u32 modulus
 };
 
+// rows per item of the finish launch, items per job
+constexpr uint32_t kFinishRows = 4, kFinishParts = 16 / kFinishRows;
+
 template <class A, int LOG_N, int LOG_V>
 struct BCfg {
   using G = Geo<LOG_N, LOG_V>;
@@ -127,7 +130,7 @@ struct BCfg {
   static constexpr int TWE = G::fwd_entries() > G::inv_entries() ? G::fwd_entries() : G::inv_entries();
   static constexpr size_t TWB = ((size_t)TWE * sizeof(Tw) + 15) / 16 * 16;
   static constexpr size_t SMEM1 = TWB + (size_t)PB * SS * sizeof(T) + (size_t)PB * 16 + (size_t)(PB + 2) * 16;
-  static constexpr size_t SMEM3 = TWB + (size_t)16 * SS * sizeof(T);
+  static constexpr size_t SMEM3 = TWB + (size_t)kFinishRows * SS * sizeof(T);
   static_assert(SS >= Slots<A, LOG_N, LOG_V>::S, "slot stride");
 };
 
@@ -370,9 +373,13 @@ LC_D void product_warp_item(const LaneDesc& L, const SubJob* __restrict__ subs, 
       if (j0 < nq[u]) P[(size_t)(2 * ip + ii) * L.nb + 4 * bq + u] = acc_reduce<E>(acc[ii][u], L.q);
 }
 
-// ---- launch 3: one job's chunk sums and inverse NTT
+// ---- launch 3: chunk sums and inverse NTT of kFinishRows of a job's rows
+//
+// With one CTA per job and the limb-pair sums loaded word by word it took 157 us
+// of 128 jobs' 5.2 ms: fewer CTAs than fit, each a chain of rounds of loads.  A
+// quarter of the rows is still whole 128-byte lines of the sums.
 template <class A, int LOG_N, int LOG_V>
-LC_D void finish_item(const LaneDesc& L, const SubJob* __restrict__ subs, uint32_t chunk, uint64_t b,
+LC_D void finish_item(const LaneDesc& L, const SubJob* __restrict__ subs, uint32_t chunk, uint64_t k,
                       unsigned char* smem) {
   using C = BCfg<A, LOG_N, LOG_V>;
   using T = typename A::T;
@@ -381,8 +388,12 @@ LC_D void finish_item(const LaneDesc& L, const SubJob* __restrict__ subs, uint32
   Tw* tw = reinterpret_cast<Tw*>(smem);
   T* slots = reinterpret_cast<T*>(smem + C::TWB);
   const int tid = threadIdx.x;
+  const uint64_t b = k / kFinishParts;
   const SubJob J = subs[L.sub0 + b];
   const uint32_t nch = (J.n + chunk - 1) / chunk;
+  const uint32_t i0 = (uint32_t)(k % kFinishParts) * kFinishRows;
+  if (i0 >= J.kappa) return;
+  const uint32_t rows = min(kFinishRows, J.kappa - i0);
   for (int i = tid; i < Geo<LOG_N, LOG_V>::inv_entries(); i += kBatchThreads)
     tw[i] = reinterpret_cast<const Tw*>(L.tw_inv)[i];
   if (L.tpart) {
@@ -394,17 +405,21 @@ LC_D void finish_item(const LaneDesc& L, const SubJob* __restrict__ subs, uint32
     const uint32_t blk = (uint32_t)b / kTpJobs, bl = (uint32_t)b % kTpJobs;
     const uint32_t c0 = L.tchunk0[blk], nchk = L.tchunk0[blk + 1] - c0;
     const size_t tile = (size_t)kTpJobs * LL * 128;
-    for (uint32_t e = tid; e < J.kappa * N; e += kBatchThreads) {
-      const uint32_t i = e % J.kappa, tt = e / J.kappa;
+    for (uint32_t e = tid; e < kFinishRows * N; e += kBatchThreads) {
+      const uint32_t i = e % kFinishRows, tt = e / kFinishRows;
+      if (i >= rows) continue;
       uint64_t tk[2 * LL - 1];
 #pragma unroll
       for (int k = 0; k < 2 * LL - 1; ++k) tk[k] = 0;
       for (uint32_t c = 0; c < nchk; ++c) {
-        const int32_t* D = L.tpart + ((size_t)(c0 + c) * N + tt) * tile + (size_t)bl * LL * 128 + i * LL;
+        const int32_t* D = L.tpart + ((size_t)(c0 + c) * N + tt) * tile + (size_t)bl * LL * 128 + (i0 + i) * LL;
 #pragma unroll
         for (int lw = 0; lw < LL; ++lw)
 #pragma unroll
-          for (int la = 0; la < LL; ++la) tk[la + lw] += (uint32_t)__ldg(D + (size_t)lw * 128 + la);
+          for (int la = 0; la < LL; la += 4) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(D + lw * 128 + la));
+            tk[la + lw] += v.x, tk[la + lw + 1] += v.y, tk[la + lw + 2] += v.z, tk[la + lw + 3] += v.w;
+          }
       }
       T res;
       if constexpr (LL == 8) {
@@ -430,10 +445,10 @@ LC_D void finish_item(const LaneDesc& L, const SubJob* __restrict__ subs, uint32
     }
   } else {
     const T* P = reinterpret_cast<const T*>(L.partial);
-    for (uint32_t e = tid; e < J.kappa * N; e += kBatchThreads) {
+    for (uint32_t e = tid; e < rows * N; e += kBatchThreads) {
       const uint32_t i = e / N, tt = e % N;
       T s = 0;
-      for (uint32_t c = 0; c < nch; ++c) s = add_mod(s, P[(((size_t)c * N + tt) * kIPad + i) * L.nb + b], L.q);
+      for (uint32_t c = 0; c < nch; ++c) s = add_mod(s, P[(((size_t)c * N + tt) * kIPad + i0 + i) * L.nb + b], L.q);
       slots[i * SS + tt] = s;
     }
   }
@@ -442,13 +457,13 @@ LC_D void finish_item(const LaneDesc& L, const SubJob* __restrict__ subs, uint32
   const int grp = tid / Geo<LOG_N, LOG_V>::T;
   const uint32_t lt = tid % Geo<LOG_N, LOG_V>::T;
   // whole warps: the transform synchronises its warp, so a warp with any of the
-  // job's rows runs all of its slots (at most 16, all there; the others unused)
+  // rows runs all of its slots (at most 4, all there; the others unused)
   const uint32_t wfirst = (uint32_t)(tid & ~31) / Geo<LOG_N, LOG_V>::T;
-  for (uint32_t p0 = 0; p0 < J.kappa; p0 += GROUPS)
-    if (p0 + wfirst < J.kappa) transform_slot<A, LOG_N, LOG_V, true>(slots + (p0 + grp) * SS, tw, ar, lt);
+  static_assert(GROUPS >= (int)kFinishRows && 32 / Geo<LOG_N, LOG_V>::T <= (int)kFinishRows, "one round, slots there");
+  if (wfirst < rows) transform_slot<A, LOG_N, LOG_V, true>(slots + grp * SS, tw, ar, lt);
   __syncthreads();
-  T* out = reinterpret_cast<T*>(J.out);
-  for (uint32_t e = tid; e < J.kappa * N; e += kBatchThreads) out[e] = slots[(e / N) * SS + e % N];
+  T* out = reinterpret_cast<T*>(J.out) + (size_t)i0 * N;
+  for (uint32_t e = tid; e < rows * N; e += kBatchThreads) out[e] = slots[(e / N) * SS + e % N];
   __syncthreads();
 }
 
@@ -484,7 +499,8 @@ template <int PHASE>
 __global__ void __launch_bounds__(kBatchThreads, PHASE == 0 ? 3 : 2) batch_kernel(const __grid_constant__ BatchParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ unsigned long long s_base;
-  const uint64_t total = p.total[PHASE];
+  constexpr uint32_t PARTS = PHASE == 2 ? kFinishParts : 1;  // item0 and total count jobs in the finish launch
+  const uint64_t total = p.total[PHASE] * PARTS;
   uint32_t lane = 0;
   for (;;) {
     if (threadIdx.x == 0) s_base = atomicAdd(&p.counters[PHASE], (unsigned long long)p.claim);
@@ -495,8 +511,8 @@ __global__ void __launch_bounds__(kBatchThreads, PHASE == 0 ? 3 : 2) batch_kerne
     const uint64_t end = min(base + p.claim, total);
     for (uint64_t it = base; it < end; ++it) {
       // claims only grow, so the lane index only moves forward
-      while (lane + 1 < p.nlanes && p.lanes[lane + 1].item0[PHASE] <= it) ++lane;
-      run_item<PHASE>(p, p.lanes[lane], it - p.lanes[lane].item0[PHASE], smem);
+      while (lane + 1 < p.nlanes && p.lanes[lane + 1].item0[PHASE] * PARTS <= it) ++lane;
+      run_item<PHASE>(p, p.lanes[lane], it - p.lanes[lane].item0[PHASE] * PARTS, smem);
     }
   }
 }
