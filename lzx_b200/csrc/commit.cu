@@ -813,7 +813,10 @@ __global__ void __launch_bounds__(256) sum_intt_kernel(const __grid_constant__ S
 // the four rows there and writes out[b][i][..].  The reduction and the inverse
 // transform as two launches took 9.6 + 9.2 us for 20 witnesses x 6 Goldilocks
 // rows of d = 128 and 8.8 + 4.4 for 16 x 2 Q_32 rows of d = 64, this 15.3 and 8.6
-// with 1024 threads (23 and 13 with 256: a warp's rounds of memory latency).
+// with 1024 threads (23 and 13 with 256: a warp's rounds of memory latency).  With
+// one split two slots are in flight, and the u32 sums are reduced twice per value
+// instead of six times: whole commitments of d = 256, kappa = 16, m = 300 and 128
+// int8 witnesses 204 -> 183 us (Goldilocks), 143 -> 115 (Q_32), 119 -> 100 (30 bits).
 // More splits go through slot_products_reduce_kernel, which spreads them over
 // warps.
 struct SlotFinishParams {
@@ -841,16 +844,8 @@ __global__ void __launch_bounds__(1024) slot_finish_kernel(const __grid_constant
     // lane: la half and row in the low three bits, columns c and c + 4 above
     const uint32_t seg = lane & 7, c = lane >> 3, shift = 8 * c + 32 * (seg & 1);
     const int32_t* d = p.part + (size_t)nt * tile + (bl * 8 + c) * 128 + iq * 32 + seg * 4;
-    for (uint32_t t = warp; t < (uint32_t)N; t += warps) {
-      const int32_t* dt = d + (size_t)t * p.ntiles * tile;
-      uint64_t tk[8] = {};
-#pragma unroll 2
-      for (uint32_t sp = 0; sp < p.splits; ++sp) {
-        const uint4 x = *reinterpret_cast<const uint4*>(dt + sp * step);
-        const uint4 y = *reinterpret_cast<const uint4*>(dt + sp * step + 4 * 128);
-        tk[0] += x.x, tk[1] += x.y, tk[2] += x.z, tk[3] += x.w;
-        tk[4] += y.x, tk[5] += y.y, tk[6] += y.z, tk[7] += y.w;
-      }
+    const size_t sstep = p.ntiles * tile;  // one slot
+    const auto put = [&](uint32_t t, const uint64_t (&tk)[8]) {
       unsigned __int128 v = 0;
 #pragma unroll
       for (int k = 0; k < 8; ++k) v += (unsigned __int128)tk[k] << (8 * k);
@@ -859,6 +854,35 @@ __global__ void __launch_bounds__(1024) slot_finish_kernel(const __grid_constant
 #pragma unroll
       for (int x : {1, 8, 16}) r = gl_add(r, __shfl_xor_sync(0xffffffffu, r, x));
       if (c == 0 && !(seg & 1)) slots[(seg >> 1) * SS + t] = r;
+    };
+    if (p.splits == 1) {
+      // U slots' loads in flight (warps and N are powers of two; N >= 2 warps)
+      constexpr int U = 2;
+      for (uint32_t t = warp; t < (uint32_t)N; t += U * warps) {
+        uint4 x[U], y[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int32_t* dt = d + (t + u * warps) * sstep;
+          x[u] = __ldg(reinterpret_cast<const uint4*>(dt));
+          y[u] = __ldg(reinterpret_cast<const uint4*>(dt + 4 * 128));
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          put(t + u * warps, {x[u].x, x[u].y, x[u].z, x[u].w, y[u].x, y[u].y, y[u].z, y[u].w});
+      }
+    } else {
+      for (uint32_t t = warp; t < (uint32_t)N; t += warps) {
+        const int32_t* dt = d + t * sstep;
+        uint64_t tk[8] = {};
+#pragma unroll 2
+        for (uint32_t sp = 0; sp < p.splits; ++sp) {
+          const uint4 x = *reinterpret_cast<const uint4*>(dt + sp * step);
+          const uint4 y = *reinterpret_cast<const uint4*>(dt + sp * step + 4 * 128);
+          tk[0] += x.x, tk[1] += x.y, tk[2] += x.z, tk[3] += x.w;
+          tk[4] += y.x, tk[5] += y.y, tk[6] += y.z, tk[7] += y.w;
+        }
+        put(t, tk);
+      }
     }
   } else {
     // lane: row in the low two bits, column lw, then one of two slots
@@ -866,16 +890,13 @@ __global__ void __launch_bounds__(1024) slot_finish_kernel(const __grid_constant
     const int32_t* d = p.part + (size_t)nt * tile + (bl * 4 + lw) * 128 + iq * 16 + i * 4;
     for (uint32_t t = 2 * warp + (lane >> 4); t < (uint32_t)N; t += 2 * warps) {
       const int32_t* dt = d + (size_t)t * p.ntiles * tile;
-      uint64_t tk[4] = {};
+      uint64_t v = 0;  // below 4 * 2^(24 + 31) * kSlotFinishSplits
 #pragma unroll 4
       for (uint32_t sp = 0; sp < p.splits; ++sp) {
-        const uint4 x = *reinterpret_cast<const uint4*>(dt + sp * step);
-        tk[0] += x.x, tk[1] += x.y, tk[2] += x.z, tk[3] += x.w;
+        const uint4 x = __ldg(reinterpret_cast<const uint4*>(dt + sp * step));
+        v += x.x + ((uint64_t)x.y << 8) + ((uint64_t)x.z << 16) + ((uint64_t)x.w << 24);
       }
-      uint64_t v = 0;
-#pragma unroll
-      for (int k = 3; k >= 0; --k) v = ((v << 8) + tk[k]) % p.q;
-      v = (v << (8 * lw)) % p.q;
+      v = (v % p.q) << (8 * lw);
       v += __shfl_xor_sync(0xffffffffu, v, 4);
       v += __shfl_xor_sync(0xffffffffu, v, 8);
       if (lw == 0) slots[i * SS + t] = (E)(v % p.q);
@@ -964,9 +985,9 @@ static int launch_witness_to(const lc_ajtai_key* key, const S* w, size_t batch, 
   constexpr int PP = WitnessTile<A, LOG_N, LOG_V>::polys;
   constexpr int G = WitnessTile<A, LOG_N, LOG_V>::groups;
   static_assert(G % 8 == 0, "small tile");
-  // tiny problems (fewer polynomials than full tiles for every SM): one
-  // polynomial per thread group, so the grid still spreads over the SMs
-  const bool tiny = (size_t)key->m * b_pad < (size_t)std::max(1, device_sm_count()) * PP;
+  // small problems (fewer polynomials than four full tiles for every SM): one
+  // polynomial per thread group, so several CTAs still share an SM
+  const bool tiny = (size_t)key->m * b_pad < 4 * (size_t)std::max(1, device_sm_count()) * PP;
   if (!tiny && PP >= 32 && b_pad % 32 == 0)
     return launch_witness_cfg<A, LOG_N, LOG_V, S, 128, PP < 32 ? PP : 32, PP < 32 ? 1 : PP / 32>(key, w, batch, b_pad,
                                                                                              dst, st);
@@ -1203,8 +1224,10 @@ static int launch_slot_finish(const lc_ajtai_key* key, size_t batch, const SlotP
   SlotFinishParams prm{static_cast<const int32_t*>(key->d_partial), out, key->plan->d_tw_inv, key->k, (uint32_t)batch,
                        sp.ncta, sp.ntiles, sp.splits, key->plan->q[0], key->plan->qinv[0]};
   const size_t grid = batch * ((key->k + 3) / 4);
-  // few CTAs: each takes its slots in as few rounds of memory latency as it can
-  const unsigned threads = grid <= 2 * (size_t)std::max(1, device_sm_count()) ? 1024 : 256;
+  // few CTAs: each takes its slots in as few rounds of memory latency as it can,
+  // while all of them fit the SMs at once
+  const size_t sms = (size_t)std::max(1, device_sm_count());
+  const unsigned threads = grid <= sms ? 1024 : grid <= 2 * sms ? 512 : 256;
   slot_finish_kernel<A, LOG_N, LOG_V><<<(unsigned)grid, threads, 0, st>>>(prm);
   return map_cuda(cudaGetLastError());
 }
@@ -1229,12 +1252,25 @@ static int slot_finish(const lc_ajtai_key* key, size_t batch, const SlotPartials
   else return slot_finish_as<MontCanon>(key, batch, sp, out, st);
 }
 
+// The tensor-core products write, and the finish launch reads back, 512 L bytes
+// per slot and column however few the ring elements are; the integer form writes
+// 16 L per K split.  Below one ring element per 192 slots and columns that
+// outweighs the multiply-adds (10 rows, us, tensor / integer; Goldilocks
+// d = 256: m = 24, 59 witnesses 51 / 36; m = 84, 59 65 / 61 and 64 87 / 74; m =
+// 200, 64 the same; Q_32 d = 256, m = 84, 64 60 / 46; d = 128, m = 84, 64
+// Goldilocks 53 / 49, 59 the same); from 8192 slots and columns on (d = 64, m =
+// 24: 64 witnesses padded to 128 27 / 24, 59 the same).
+static bool tensor_products(const lc_ajtai_key* key, uint32_t b_pad) {
+  const uint64_t cols = (uint64_t)key->n * b_pad;
+  return key->slot_products == LC_PRODUCTS_TENSOR && !(cols >= 8192 && (uint64_t)key->m * 192 <= cols);
+}
+
 template <class E>
 static int commit_core(lc_ajtai_key* key, size_t batch, uint32_t b_pad, void* out, cudaStream_t st) {
   const uint32_t n = key->n, m = key->m, kappa = key->k;
   const uint32_t q = key->plan->q[0];
   // the per-slot products as byte-limb GEMMs on the tensor cores
-  if (key->slot_products == LC_PRODUCTS_TENSOR) {
+  if (tensor_products(key, b_pad)) {
     SlotPartials sp{};
     int rc = tc_slot_products(key->d_ahat_t, key->a_m, key->d_what_t, (uint32_t)sizeof(E), m, n, kappa, b_pad,
                               &key->d_partial, &key->partial_bytes, &sp, key->d_err, st);
@@ -1406,9 +1442,9 @@ static int commit_any(lc_ajtai_key* key, const S* w, size_t batch, void* out, cu
   uint32_t b_pad = batch >= 64 ? (uint32_t)((batch + kBTile - 1) / kBTile * kBTile)
                                : batch >= 4 ? (uint32_t)((batch + 3) / 4 * 4) : (uint32_t)batch;
   int rc = LC_ERR_OUT_OF_MEMORY;
-  if (batch >= 4 && batch < 64 && key->slot_products == LC_PRODUCTS_TENSOR) {
-    uint32_t pow2 = (uint32_t)(32 / eb);
-    while (pow2 < batch) pow2 *= 2;
+  uint32_t pow2 = (uint32_t)(32 / eb);
+  while (pow2 < batch && pow2 < 64) pow2 *= 2;
+  if (batch >= 4 && batch < 64 && tensor_products(key, pow2)) {
     rc = grow(&key->d_what_t, &key->what_bytes, (size_t)key->n * key->m * pow2 * eb);
     if (rc == LC_OK) b_pad = pow2;
   }

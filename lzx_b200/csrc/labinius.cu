@@ -51,8 +51,7 @@ constexpr int kLbTileLeaves = kLbLeaves / kLbTiles;  // 108: equal tiles keep th
 constexpr int kLbK = 352;              // K: 2 x 5 words x 32 bits, then the two elements' last 2 bits
 constexpr int kLbElems = 64;           // ring elements per tile; MMA N = 128 rows (E then O)
 constexpr int kLbImg = 128 * kLbK;     // one byte limb of one leaf tile; also one stage of digit rows
-constexpr uint32_t kLbStoreWeight = 7;  // a tile of the kept limb takes about 7/4 of another's (measured 5.7 and 2.9 k cycles before its
-                                        // reductions were cut)
+constexpr uint32_t kLbStoreWeight = 7;  // a tile of the kept limb counts as 7/4 of another's (share of the CTAs)
 constexpr int kLbEpiWarps = 16, kLbProdWarps = 4;
 constexpr int kLbTcThreads = 32 * (kLbEpiWarps + kLbProdWarps + 1);
 constexpr int kLbOffB = 2 * kLbImg, kLbOffBar = kLbOffB + 2 * kLbImg;

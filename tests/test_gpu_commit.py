@@ -207,6 +207,19 @@ def test_goldilocks_witness_gemm_shapes(log_d, m, batch):
     assert np.array_equal(got, oracle_gl_commit(A, kappa, m, W, d=d))
 
 
+@pytest.mark.parametrize("log_d,m,batch", [(6, 42, 64), (6, 43, 64), (7, 42, 59), (7, 43, 59), (8, 85, 59), (8, 86, 59),
+                                           (8, 170, 65), (8, 171, 65), (8, 1, 33)])
+def test_goldilocks_few_ring_elements(log_d, m, batch):
+    """Both sides of the line between the integer and the tensor-core products
+    of keys with few ring elements; odd row counts."""
+    d, kappa = 1 << log_d, 5
+    A, key = gl_key(kappa, m, d=d, seed=m)
+    W = synth.synth_i8(13, batch, batch * m * d).reshape(batch, m, d)
+    got = key.commit(W)
+    idx = [0, 1, batch // 2, batch - 1]
+    assert np.array_equal(got[idx], oracle_gl_commit(A, kappa, m, W[idx], d=d))
+
+
 def test_goldilocks_config3_full_batch():
     """kappa=16, 2^16 witness elements, 128 int8 witnesses (the bench workload):
     every commitment of the batch checked against the oracle."""
