@@ -8,8 +8,9 @@
 // n_b > j take part, so a lane's transformed witnesses are stored as a
 // staircase: slot t, ring element j, job b at  what[t*Sp + Rp[j] + b],  where
 // R[j] = sum over j' < j of the number of jobs longer than j' (S = sum n_b),
-// Rp[j] the same with every row of active jobs padded to 16 bytes (so each
-// row starts 16-byte aligned) and Sp = Rp[n_max] the entries per slot.
+// Rp[j] where row j starts -- the rows of 64 ring elements (kTpRows) have the
+// length of the first, padded to 16 bytes -- and Sp = Rp[n_max] the entries per
+// slot.
 //   1. witness NTT: an item is PB consecutive staircase polynomials; their
 //      (j, b) come from a per-item start table and a short walk over R;
 //   2. product: a warp's item is (chunk of ring elements, slot t, block of 16
@@ -76,7 +77,7 @@ struct LaneDesc {
   uint32_t nchunks;
   uint64_t S;       // staircase polynomials
   const uint64_t* R;       // [n_max + 1]: jobs longer than j' summed over j' < j
-  const uint64_t* Rp;      // [n_max + 1]: the same with every row padded to 16 bytes (where row j starts)
+  const uint64_t* Rp;      // [n_max + 1]: where row j starts (row_stride)
   uint64_t Sp;             // entries per slot of `what` (16-byte rows, 16-byte slots)
   const uint32_t* item_j;  // witness items: ring element of the first polynomial
   uint32_t sub0;           // first job of the lane in the sub-job table
@@ -919,16 +920,15 @@ __global__ void __launch_bounds__(TwCfg<EW, PN>::THREADS, 1)
 // M = 128 (the key row's 16 x L bytes (i, la); u32 keys fill half and the
 // second A atom is a zero tile), N = 32 L bytes (b, lw), K = the chunk.  The
 // key rows Ahat[t][j][16] arrive by TMA (a 3-D map per lane: row bytes,
-// j < a_m, slot), and so do the witness rows: the staircase is cut into segments
-// of ring elements with the same number of active jobs (and at multiples of the
-// chunk), in which row j starts at a constant stride (16-byte aligned), so a 3-D
-// map per segment -- bytes of the active jobs, rows, slots -- loads 64 rows by
-// 128 bytes with the 128-byte swizzle of the MN-major layout the MMA reads; what
-// lies past the active jobs or the segment's rows reads as zero.  Stages start at
-// segment starts: the key rows past a segment's end meet zero witness rows there
-// and come again with the next segment.  The epilogue warps write D, one
-// [32 L columns][128 rows] int32 tile per item; the finish launch folds the
-// limb pairs over the block's chunks.
+// j < a_m, slot), and so do the witness rows: the 64 rows of a stage have the
+// stride that the first of them needs, and a segment is a run of stages with the
+// same number of active jobs there (within a chunk), so a 3-D map per segment --
+// bytes of the active jobs, rows, slots -- loads 64 rows by 128 bytes with the
+// 128-byte swizzle of the MN-major layout the MMA reads.  What lies past the
+// segment's jobs or rows reads as zero, and so do the entries of jobs that end
+// within the 64 rows: nothing writes them after the batch's creation zeroed them.
+// The epilogue warps write D, one [32 L columns][128 rows] int32 tile per item;
+// the finish launch folds the limb pairs over the block's chunks.
 //
 // Bound: HBM.  Gathering the rows with 16-byte cp.async copies (a shuffle of row
 // offsets and counts per copy) kept the shared-memory pipe 69 % busy: products
@@ -1203,6 +1203,16 @@ static void batch_free(lc_batch* b) {
   delete b;
 }
 
+// Entries from row j of `what` to the next: the jobs active at the first row of
+// j's stage, padded to 16 bytes.  With the stride of each row's own count every
+// change of the count began a segment, and with it a stage: 128 jobs of 1..256
+// ring elements (Goldilocks, d = 64) took 118 us with 237 stages, 37 with
+// these 10; 128 of 512..1024 under the CRT set at d = 256 922 us, 437.
+static uint64_t row_stride(const std::vector<uint64_t>& R, uint32_t j, uint32_t eb) {
+  const uint32_t j0 = j / kTpRows * kTpRows, pad = 16 / eb;
+  return (R[j0 + 1] - R[j0] + pad - 1) / pad * pad;
+}
+
 // Tensor-core products: per lane a TMA map of its key rows and of every segment
 // of its staircase, per 32-job block the K chunks, the items (longest first, Goldilocks lanes then u32 lanes)
 // and the partial tiles.  Leaves tensor_ok false when a lane cannot run
@@ -1230,15 +1240,14 @@ static int batch_tensor_setup(lc_batch* b) {
             CU_TENSOR_MAP_INTERLEAVE_NONE, aw == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return LC_OK;
-    // segments: constant count of active jobs, cut at multiples of the chunk
+    // segments: stages with the same number of active jobs at their first row
     const std::vector<uint64_t>& R = b->R[l];
     std::vector<uint32_t> chunk_seg;  // first segment of every chunk
-    const uint32_t pad = 16 / eb;
     uint64_t row0 = 0;  // where the segment's first row starts, in entries
     for (uint32_t j = 0; j < L.n_max;) {
-      const uint64_t cnt = R[j + 1] - R[j], stride = (cnt + pad - 1) / pad * pad;
-      uint32_t e = j + 1;
-      while (e < L.n_max && e % kTpChunk && R[e + 1] - R[e] == cnt) ++e;
+      const uint64_t cnt = R[j + 1] - R[j], stride = row_stride(R, j, eb);
+      uint32_t e = std::min(L.n_max, j + kTpRows);
+      while (e < L.n_max && e % kTpChunk && R[e + 1] - R[e] == cnt) e = std::min(L.n_max, e + kTpRows);
       if (j % kTpChunk == 0) chunk_seg.push_back((uint32_t)segs.size());
       const cuuint64_t sdims[3] = {cnt * eb, e - j, d};
       const cuuint64_t sstr[2] = {stride * eb, L.Sp * eb};
@@ -1263,8 +1272,7 @@ static int batch_tensor_setup(lc_batch* b) {
       tchunk0.push_back(acc);
       for (uint32_t c = 0; c < chunks; ++c) {
         const uint32_t j1 = std::min(nfirst, (c + 1) * kTpChunk);
-        uint32_t nst = 0;  // nfirst and the chunk's end are segment ends
-        for (size_t g = chunk_seg[c]; g < segs.size() && segs[g].j0 < j1; ++g) nst += (segs[g].len + kTpRows - 1) / kTpRows;
+        const uint32_t nst = (j1 - c * kTpChunk + kTpRows - 1) / kTpRows;  // segments start at multiples of kTpRows
         for (uint32_t t = 0; t < d; ++t)
           items[eb == 8 ? 0 : 1].push_back({nst, TpItem{(uint32_t)l, t, blk, c, chunk_seg[c], nst}});
       }
@@ -1622,14 +1630,11 @@ LC_API int lc_batch_create(const lc_commit_class* classes, uint32_t num_classes,
         }
         R[L.n_max] = acc;
         L.S = acc;
-        // the same offsets with each row of active jobs padded to 16 bytes, so
-        // that every row of `what` starts 16-byte aligned
-        const uint64_t pad = 16 / eb;
         std::vector<uint64_t> Rp(L.n_max + 1);
         uint64_t accp = 0;
         for (uint32_t j = 0; j < L.n_max; ++j) {
           Rp[j] = accp;
-          accp += (R[j + 1] - R[j] + pad - 1) / pad * pad;
+          accp += row_stride(R, j, (uint32_t)eb);
         }
         Rp[L.n_max] = accp;
         L.Sp = accp;
@@ -1667,6 +1672,7 @@ LC_API int lc_batch_create(const lc_commit_class* classes, uint32_t num_classes,
     return LC_ERR_OUT_OF_MEMORY;
   }
   cudaMemset(b->d_err, 0, 4);
+  cudaMemset(b->d_what, 0, what_bytes);  // the copies below wait for it
   if (!subs.empty()) cudaMemcpy(b->d_subs, subs.data(), subs.size() * sizeof(SubJob), cudaMemcpyHostToDevice);
   if (!Rall.empty()) cudaMemcpy(b->d_R, Rall.data(), Rall.size() * 8, cudaMemcpyHostToDevice);
   if (!itemj_all.empty())

@@ -267,3 +267,35 @@ def test_batch_row_counts(mixed_classes, kappa, products):
     batch.check()
     for j in jobs:
         assert torch.equal(j.out, one_by_one(mixed_classes, j)), (j.cls, kappa)
+
+
+def best_ms(fn, reps=5, blocks=5):
+    """Shortest of ``blocks`` timed runs of ``reps`` calls each."""
+    fn()
+    best = float("inf")
+    for _ in range(blocks):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(reps):
+            fn()
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b) / reps)
+    return best
+
+
+@pytest.mark.parametrize("log_d,gl", [(6, True), (8, False)], ids=["gl64", "crt256"])
+def test_uneven_lengths_cost_no_stages(log_d, gl):
+    """128 jobs of 2, 4, .. 256 ring elements are half the work of 128 jobs of 256:
+    they may not take longer (the products' stages follow the longest job of a
+    block, not how often the number of active jobs changes)."""
+    cl = gl_class(log_d, 256, 5) if gl else u32_class(CRT_SET_30BIT, log_d, 256, 5)
+    d, dt = 1 << log_d, torch.int64 if gl else torch.int32
+    w = torch.randint(-128, 128, (256, d), dtype=torch.int8, device="cuda")
+    ms = {}
+    for name, lengths in (("uneven", range(2, 257, 2)), ("even", [256] * 128)):
+        jobs = [CommitJob(0, 16, n, w, torch.empty((len(cl["keys"]), 16, d), dtype=dt, device="cuda")) for n in lengths]
+        batch = CommitBatch([cl["keys"]], jobs)
+        ms[name] = best_ms(batch.run)
+        batch.check()
+    assert ms["uneven"] <= 1.2 * ms["even"], ms
