@@ -1,0 +1,18 @@
+// blocks.h -- device memory of keys: freed blocks are kept for the next key.
+#pragma once
+
+#include <stddef.h>
+
+namespace lc {
+
+// block_alloc hands out a kept block of the same (rounded) size that no queued
+// work uses, or driver memory.  `idle` tells block_free that nothing queued uses
+// the block any more; the others wait in the list for block_settle, which
+// synchronises the current device when it has such blocks (for calls that are
+// synchronous anyway).
+int block_alloc(void** p, size_t bytes);
+void block_free(void* p, size_t bytes, int device, bool idle);
+void block_settle();
+void block_users(int delta);  // live plans and keys: the last one frees what is kept
+
+}  // namespace lc

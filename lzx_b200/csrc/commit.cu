@@ -1673,7 +1673,7 @@ int key_create_from(const lc_ntt_plan* plan, uint32_t k, uint32_t m, const void*
   // one synchronisation: the kernels' errors, and nothing reads the matrix any more
   const cudaError_t e = cudaStreamSynchronize(nullptr);
   if (!rc) rc = map_cuda(e);
-  block_free(tmp, bytes, key->device);
+  block_free(tmp, bytes, key->device, e == cudaSuccess);  // used on this stream only
   if (rc) {
     lc_ajtai_key_destroy(key);
     return rc;
@@ -1701,6 +1701,7 @@ LC_API int lc_ajtai_key_create_ex(const lc_ntt_plan* plan, uint32_t k, uint32_t 
   const size_t bytes = (size_t)k * m * ((size_t)1 << plan->log_n) * eb;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return lc::map_cuda(cudaGetLastError());
+  lc::block_settle();
   // aligned memory of this device is read in place; a host matrix, another
   // device's or an unaligned one is copied first
   if (matrix_on_device && ((uintptr_t)matrix & 15) == 0) {
@@ -1716,7 +1717,8 @@ LC_API int lc_ajtai_key_create_ex(const lc_ntt_plan* plan, uint32_t k, uint32_t 
   rc = lc::map_cuda(
       cudaMemcpy(tmp, matrix, bytes, matrix_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
   if (!rc) rc = lc::key_create_from(plan, k, m, tmp, flags, out);
-  lc::block_free(tmp, bytes, dev);  // synchronous above: nothing queued reads it
+  // used on the default stream only, which the creation waits for
+  lc::block_free(tmp, bytes, dev, !rc || cudaStreamSynchronize(nullptr) == cudaSuccess);
   return rc;
 }
 
@@ -1724,19 +1726,7 @@ LC_API void lc_ajtai_key_destroy(lc_ajtai_key* key) {
   if (!key) return;
   for (void* p : {key->d_what_t, key->d_partial, key->d_chat, key->d_wtmp, (void*)key->d_grid, key->d_in, key->d_out})
     if (p) cudaFree(p);
-  if (key->d_block) {
-    // commits of this key may still run on any stream of its device
-    int cur = key->device;
-    cudaGetDevice(&cur);
-    if (cur != key->device) cudaSetDevice(key->device);
-    if (cudaDeviceSynchronize() == cudaSuccess)
-      block_free(key->d_block, key->block_bytes, key->device);
-    else {
-      cudaGetLastError();
-      cudaFree(key->d_block);
-    }
-    if (cur != key->device) cudaSetDevice(cur);
-  }
+  block_free(key->d_block, key->block_bytes, key->device, false);  // its commits may still run on any stream
   if (key->host_stream) cudaStreamDestroy(key->host_stream);
   if (key->h_flags) cudaFreeHost(key->h_flags);
   if (key->h_stage_in) cudaFreeHost(key->h_stage_in);

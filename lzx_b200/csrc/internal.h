@@ -7,6 +7,7 @@
 #include <atomic>
 
 #include "../../include/lattice_cuda.h"
+#include "blocks.h"
 
 namespace lc {
 
@@ -169,11 +170,6 @@ int key_create_from(const lc_ntt_plan* plan, uint32_t k, uint32_t m, const void*
 // A plan for the current device with `plan`'s moduli: its tables are shared when
 // they live on that device.  `d_err` (device, zeroed) is its error word then.
 int plan_share(const lc_ntt_plan* plan, uint32_t* d_err, lc_ntt_plan** out);
-// Device blocks of keys (lattice_cuda.cu): a few freed ones are kept for the
-// next key.  block_free wants a block that no queued work uses any more.
-int block_alloc(void** p, size_t bytes);
-void block_free(void* p, size_t bytes, int device);
-void block_users(int delta);  // live plans and keys: the last one frees what is kept
 int map_cuda(cudaError_t e);
 int run_ntt(const lc_ntt_plan* plan, const void* in, void* out, size_t count, bool inverse,
             cudaStream_t s);

@@ -244,13 +244,14 @@ LC_API int lc_ajtai_key_from_seed(const lc_ntt_plan* plan, uint32_t k, uint32_t 
   void* mat = nullptr;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return map_cuda(cudaGetLastError());
+  block_settle();
   rc = block_alloc(&mat, count * n * 4);
   if (rc) return rc;
   static const uint8_t dom[7] = {'a', 'j', 't', 'a', 'i', '-', 'A'};
   rc = uniform_from_seed(plan, dom, 7, seed, 32, 0, count, static_cast<uint32_t*>(mat), nullptr);
   if (!rc) rc = key_create_from(plan, k, m, mat, 0, out);  // synchronous
-  else cudaStreamSynchronize(nullptr);
-  block_free(mat, count * n * 4, dev);
+  const bool idle = !rc || cudaStreamSynchronize(nullptr) == cudaSuccess;  // used on this stream only
+  block_free(mat, count * n * 4, dev, idle);
   return rc;
 }
 

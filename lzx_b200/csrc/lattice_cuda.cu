@@ -123,79 +123,6 @@ int device_sm_count() {
   return g_num_sms;
 }
 
-// ---------------------------------------------------------------- key blocks
-//
-// Making a key costs a cudaMalloc and destroying it a cudaFree, each a driver
-// call of 100 us and more that also serialises with the device's other work; a
-// verifier that derives its key from the seed on every call paid both several
-// times per call (from_seed + one commit, k = 2, m = 2000: 940 us).
-// Freed blocks of up to 32 MiB are kept for the next key, at most 64 MiB per
-// device; they go back to the driver when an allocation fails and when the last
-// plan and key of the process is destroyed.  A block enters the list only when
-// the device is idle (lc_ajtai_key_destroy), so its next user may use any stream.
-constexpr size_t kBlockKeepMax = (size_t)32 << 20, kBlockKeepTotal = (size_t)64 << 20;
-
-struct KeptBlock {
-  void* p;
-  size_t bytes;
-  int device;
-};
-static std::mutex g_block_mu;
-static std::vector<KeptBlock> g_blocks;
-static long g_block_users = 0;
-
-static size_t block_size(size_t bytes) {  // what may be kept has at most 1/8 unused
-  if (bytes > kBlockKeepMax) return bytes;
-  size_t step = 512;
-  while (step * 16 < bytes) step *= 2;
-  return (bytes + step - 1) / step * step;
-}
-
-// frees the kept blocks (of every device); g_block_mu held
-static void block_drain() {
-  for (const KeptBlock& b : g_blocks) cudaFree(b.p);
-  g_blocks.clear();
-}
-
-int block_alloc(void** p, size_t bytes) {
-  const size_t size = block_size(bytes);
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return map_cuda(cudaGetLastError());
-  std::lock_guard<std::mutex> lk(g_block_mu);
-  for (size_t i = 0; i < g_blocks.size(); ++i)
-    if (g_blocks[i].bytes == size && g_blocks[i].device == dev) {
-      *p = g_blocks[i].p;
-      g_blocks.erase(g_blocks.begin() + (long)i);
-      return LC_OK;
-    }
-  if (cudaMalloc(p, size) == cudaSuccess) return LC_OK;
-  cudaGetLastError();
-  block_drain();
-  if (cudaMalloc(p, size) == cudaSuccess) return LC_OK;
-  cudaGetLastError();
-  *p = nullptr;
-  return LC_ERR_OUT_OF_MEMORY;
-}
-
-void block_free(void* p, size_t bytes, int device) {
-  if (!p) return;
-  const size_t size = block_size(bytes);
-  std::lock_guard<std::mutex> lk(g_block_mu);
-  size_t kept = size;
-  for (const KeptBlock& b : g_blocks)
-    if (b.device == device) kept += b.bytes;
-  if (size <= kBlockKeepMax && kept <= kBlockKeepTotal)
-    g_blocks.push_back({p, size, device});
-  else
-    cudaFree(p);
-}
-
-void block_users(int delta) {
-  std::lock_guard<std::mutex> lk(g_block_mu);
-  g_block_users += delta;
-  if (g_block_users == 0) block_drain();
-}
-
 int map_cuda(cudaError_t e) {
   if (e == cudaSuccess) return LC_OK;
   cudaGetLastError();

@@ -1,0 +1,124 @@
+"""The kept device blocks of keys (lzx_b200/csrc/blocks.cu) against a fake CUDA runtime, on the CPU.
+
+The source is compiled with the host compiler against a stand-in
+``cuda_runtime.h`` whose allocator hands out numbers, counts the driver calls
+and fails on request.
+"""
+import os
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+RUNTIME = r"""
+#pragma once
+#include <stddef.h>
+enum cudaError_t { cudaSuccess = 0, cudaErrorMemoryAllocation = 2, cudaErrorOther = 900 };
+struct Fake {
+  long mallocs = 0, frees = 0, syncs = 0;
+  int device = 0;
+  size_t live = 0, limit = (size_t)1 << 40;
+  bool sync_fails = false;
+};
+extern Fake fake;
+cudaError_t cudaMalloc(void** p, size_t bytes);
+cudaError_t cudaFree(void* p);
+cudaError_t cudaGetDevice(int* d);
+cudaError_t cudaGetLastError();
+cudaError_t cudaDeviceSynchronize();
+"""
+
+FAKE = r"""
+#include <cuda_runtime.h>
+#include <cstdio>
+#include <cstdlib>
+#include <map>
+#include <vector>
+#include "blocks.h"
+#include "lattice_cuda.h"
+Fake fake;
+static std::map<void*, size_t> sizes;
+static char* next_p = reinterpret_cast<char*>(4096);
+cudaError_t cudaMalloc(void** p, size_t bytes) {
+  ++fake.mallocs;
+  if (fake.live + bytes > fake.limit) return cudaErrorMemoryAllocation;
+  *p = next_p;
+  next_p += (bytes + 511) / 512 * 512;
+  sizes[*p] = bytes;
+  fake.live += bytes;
+  return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) {
+  ++fake.frees;
+  fake.live -= sizes.at(p);  // throws for a block that is not there
+  sizes.erase(p);
+  return cudaSuccess;
+}
+cudaError_t cudaGetDevice(int* d) { *d = fake.device; return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() { ++fake.syncs; return fake.sync_fails ? cudaErrorOther : cudaSuccess; }
+#define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); std::exit(1); } } while (0)
+using namespace lc;
+constexpr size_t MiB = 1 << 20;
+int main() {
+  block_users(1);
+  BODY
+  block_users(-1);
+  CHECK(fake.live == 0 && sizes.empty());
+  return 0;
+}
+"""
+
+
+def run(tmp_path, body):
+    (tmp_path / "cuda_runtime.h").write_text(RUNTIME)
+    (tmp_path / "main.cpp").write_text(FAKE.replace("BODY", body))
+    src = os.path.join(ROOT, "lzx_b200", "csrc")
+    exe = str(tmp_path / "blocks")
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-I", str(tmp_path), "-I", src,
+                    "-I", os.path.join(ROOT, "include"), "-o", exe, str(tmp_path / "main.cpp"),
+                    "-x", "c++", os.path.join(src, "blocks.cu")], check=True, capture_output=True, text=True)
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+BODIES = {
+    # a block that queued work may use is not synchronised for when it is freed, nor
+    # handed out before the device was synchronised
+    "busy": """
+  void *a, *b, *c;
+  CHECK(block_alloc(&a, MiB) == LC_OK);
+  block_free(a, MiB, 0, false);
+  CHECK(fake.syncs == 0);
+  CHECK(block_alloc(&b, MiB) == LC_OK && b != a && fake.mallocs == 2 && fake.syncs == 0);
+  block_settle();
+  CHECK(fake.syncs == 1);
+  block_settle();
+  CHECK(fake.syncs == 1);
+  CHECK(block_alloc(&c, MiB) == LC_OK && c == a && fake.mallocs == 2);
+  block_free(b, MiB, 0, true);
+  CHECK(block_alloc(&b, MiB) == LC_OK && fake.mallocs == 2 && fake.syncs == 1);
+  block_free(b, MiB, 0, true);
+  block_free(c, MiB, 0, true);""",
+    # a failed synchronisation hands nothing out; another device's blocks stay as they are
+    "device": """
+  void *a, *b;
+  CHECK(block_alloc(&a, MiB) == LC_OK);
+  block_free(a, MiB, 0, false);
+  fake.sync_fails = true;
+  block_settle();
+  CHECK(block_alloc(&b, MiB) == LC_OK && b != a);
+  block_free(b, MiB, 0, true);
+  fake.sync_fails = false;
+  fake.device = 1;
+  block_settle();
+  CHECK(fake.syncs == 1);
+  CHECK(block_alloc(&b, MiB) == LC_OK && fake.mallocs == 3);
+  block_free(b, MiB, 1, true);""",
+}
+
+
+@pytest.mark.parametrize("name", list(BODIES))
+def test_blocks(tmp_path, name):
+    run(tmp_path, BODIES[name])

@@ -220,6 +220,52 @@ def test_goldilocks_few_ring_elements(log_d, m, batch):
     assert np.array_equal(got[idx], oracle_gl_commit(A, kappa, m, W[idx], d=d))
 
 
+@pytest.mark.parametrize("batch", [1, 8])
+def test_key_destroyed_during_capture(batch):
+    """A key that goes while a stream captures (in the mode that allows frees)
+    does not end the capture."""
+    kappa, m, d = 4, 100, 64
+    A, key = gl_key(kappa, m, seed=6)
+    other = gl_key(kappa, m, seed=7)[1]
+    W = synth.synth_i8(15, batch, batch * m * d).reshape(batch, m, d)
+    dev = torch.from_numpy(W).cuda()
+    out = torch.empty((batch, kappa, d), dtype=torch.int64, device="cuda")
+    key.commit(dev, out)  # scratch is there before the capture
+    other.commit(dev)
+    out.zero_()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="relaxed"):
+        key.commit(dev, out)
+        del other
+    g.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy().view(np.uint64), oracle_gl_commit(A, kappa, m, W))
+
+
+def test_key_destroyed_while_its_commit_runs():
+    """The next key of the same size may not take the memory of a destroyed one
+    whose commitments still run on another stream."""
+    kappa, m, d, batch = 16, 2000, 64, 256
+    W = synth.synth_i8(16, 0, batch * m * d).reshape(batch, m, d)
+    dev = torch.from_numpy(W).cuda()
+    outs, mats = [], []
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    for seed in range(6):
+        A, key = gl_key(kappa, m, seed=20 + seed)
+        mats.append(A)
+        with torch.cuda.stream(streams[seed % 2]):
+            for _ in range(8):
+                out = key.commit(dev)
+            outs.append(out)
+        del key
+    torch.cuda.synchronize()
+    idx = [0, batch - 1]
+    for A, out in zip(mats, outs):
+        assert np.array_equal(out[idx].cpu().numpy().view(np.uint64), oracle_gl_commit(A, kappa, m, W[idx]))
+
+
 def test_goldilocks_config3_full_batch():
     """kappa=16, 2^16 witness elements, 128 int8 witnesses (the bench workload):
     every commitment of the batch checked against the oracle."""
