@@ -8,9 +8,9 @@
 // n_b > j take part, so a lane's transformed witnesses are stored as a
 // staircase: slot t, ring element j, job b at  what[t*Sp + Rp[j] + b],  where
 // R[j] = sum over j' < j of the number of jobs longer than j' (S = sum n_b),
-// Rp[j] where row j starts -- the rows of 64 ring elements (kTpRows) have the
-// length of the first, padded to 16 bytes -- and Sp = Rp[n_max] the entries per
-// slot.
+// Rp[j] where row j starts -- rows have the length of their active jobs, or of
+// those of the first of their 64 (row_group), padded to 16 bytes -- and Sp =
+// Rp[n_max] the entries per slot.
 //   1. witness NTT: an item is PB consecutive staircase polynomials; their
 //      (j, b) come from a per-item start table and a short walk over R;
 //   2. product: a warp's item is (chunk of ring elements, slot t, block of 16
@@ -920,13 +920,14 @@ __global__ void __launch_bounds__(TwCfg<EW, PN>::THREADS, 1)
 // M = 128 (the key row's 16 x L bytes (i, la); u32 keys fill half and the
 // second A atom is a zero tile), N = 32 L bytes (b, lw), K = the chunk.  The
 // key rows Ahat[t][j][16] arrive by TMA (a 3-D map per lane: row bytes,
-// j < a_m, slot), and so do the witness rows: the 64 rows of a stage have the
-// stride that the first of them needs, and a segment is a run of stages with the
-// same number of active jobs there (within a chunk), so a 3-D map per segment --
-// bytes of the active jobs, rows, slots -- loads 64 rows by 128 bytes with the
-// 128-byte swizzle of the MN-major layout the MMA reads.  What lies past the
-// segment's jobs or rows reads as zero, and so do the entries of jobs that end
-// within the 64 rows: nothing writes them after the batch's creation zeroed them.
+// j < a_m, slot), and so do the witness rows: a segment is a run of rows of one
+// length (row_group, within a chunk), so a 3-D map per segment -- bytes of the
+// active jobs, rows, slots -- loads 64 rows by 128 bytes with the 128-byte swizzle
+// of the MN-major layout the MMA reads.  What lies past the segment's jobs or rows
+// reads as zero, and so do the entries of jobs that end within 64 rows of one
+// length: nothing writes them after the batch's creation zeroed them.  Stages
+// start at segment starts: the key rows past a segment's end meet zero witness
+// rows and come again with the next segment.
 // The epilogue warps write D, one [32 L columns][128 rows] int32 tile per item;
 // the finish launch folds the limb pairs over the block's chunks.
 //
@@ -1144,6 +1145,7 @@ static bool lane_geometry(PlanKind kind, uint32_t log_n, size_t& s1, size_t& s3,
 struct lc_batch {
   std::vector<lc::LaneDesc> lanes;     // host copies (device pointers inside)
   std::vector<std::vector<uint64_t>> R;  // staircase offsets per lane (host)
+  std::vector<uint32_t> group;           // rows of one length per lane (row_group)
   uint64_t* d_citem = nullptr;
   uint8_t* d_cblk = nullptr;
   std::vector<uint64_t> lane_elem;     // element bytes per lane
@@ -1203,13 +1205,31 @@ static void batch_free(lc_batch* b) {
   delete b;
 }
 
-// Entries from row j of `what` to the next: the jobs active at the first row of
-// j's stage, padded to 16 bytes.  With the stride of each row's own count every
-// change of the count began a segment, and with it a stage: 128 jobs of 1..256
-// ring elements (Goldilocks, d = 64) took 118 us with 237 stages, 37 with
-// these 10; 128 of 512..1024 under the CRT set at d = 256 922 us, 437.
-static uint64_t row_stride(const std::vector<uint64_t>& R, uint32_t j, uint32_t eb) {
-  const uint32_t j0 = j / kTpRows * kTpRows, pad = 16 / eb;
+// Where the row length of `what` may change.  With rows of their own active jobs
+// every change of that number ends a segment, and with it a stage of 64 rows
+// (kTpRows): 128 jobs of 1..256 ring elements (Goldilocks, d = 64) took 118 us
+// with 237 stages.  With one length per 64 rows they take 37 with 10; 128 jobs
+// of 512..1024 under the CRT set at d = 256 922 us, 437.  Lanes whose segments
+// cost at most an eighth more stages keep rows of their own length: 20, 32 and 80
+// jobs to 2^16, 2^15 and 2^16 took 1.30, 1.40 and 2.91 ms so, and 1.36, 1.49 and
+// 3.04 with one length per 64 (aligned row starts: shifting the 64s by 27 rows
+// changed the last two to 1.37 and 2.90); 128 jobs to 2^12, a sixth more stages,
+// 0.65 and 0.62.
+static uint32_t row_group(const std::vector<uint64_t>& R) {
+  const uint64_t n = R.size() - 1;
+  uint64_t stages = 0;
+  for (uint64_t j = 0; j < n;) {
+    uint64_t e = j + 1;
+    while (e < n && e % kTpChunk && R[e + 1] - R[e] == R[j + 1] - R[j]) ++e;
+    stages += (e - j + kTpRows - 1) / kTpRows;
+    j = e;
+  }
+  return 8 * stages <= 9 * ((n + kTpRows - 1) / kTpRows) ? 1 : kTpRows;
+}
+
+// Entries from row j to the next.
+static uint64_t row_stride(const std::vector<uint64_t>& R, uint32_t j, uint32_t group, uint32_t eb) {
+  const uint32_t j0 = j / group * group, pad = 16 / eb;
   return (R[j0 + 1] - R[j0] + pad - 1) / pad * pad;
 }
 
@@ -1240,14 +1260,15 @@ static int batch_tensor_setup(lc_batch* b) {
             CU_TENSOR_MAP_INTERLEAVE_NONE, aw == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return LC_OK;
-    // segments: stages with the same number of active jobs at their first row
+    // segments: groups of rows with the same number of active jobs at their first
     const std::vector<uint64_t>& R = b->R[l];
+    const uint32_t group = b->group[l];
     std::vector<uint32_t> chunk_seg;  // first segment of every chunk
     uint64_t row0 = 0;  // where the segment's first row starts, in entries
     for (uint32_t j = 0; j < L.n_max;) {
-      const uint64_t cnt = R[j + 1] - R[j], stride = row_stride(R, j, eb);
-      uint32_t e = std::min(L.n_max, j + kTpRows);
-      while (e < L.n_max && e % kTpChunk && R[e + 1] - R[e] == cnt) e = std::min(L.n_max, e + kTpRows);
+      const uint64_t cnt = R[j + 1] - R[j], stride = row_stride(R, j, group, eb);
+      uint32_t e = j + 1;
+      while (e < L.n_max && e % kTpChunk && (e % group || R[e + 1] - R[e] == cnt)) ++e;
       if (j % kTpChunk == 0) chunk_seg.push_back((uint32_t)segs.size());
       const cuuint64_t sdims[3] = {cnt * eb, e - j, d};
       const cuuint64_t sstr[2] = {stride * eb, L.Sp * eb};
@@ -1272,7 +1293,9 @@ static int batch_tensor_setup(lc_batch* b) {
       tchunk0.push_back(acc);
       for (uint32_t c = 0; c < chunks; ++c) {
         const uint32_t j1 = std::min(nfirst, (c + 1) * kTpChunk);
-        const uint32_t nst = (j1 - c * kTpChunk + kTpRows - 1) / kTpRows;  // segments start at multiples of kTpRows
+        uint32_t nst = 0;
+        for (size_t g = chunk_seg[c]; g < segs.size() && segs[g].j0 < j1; ++g)
+          nst += (std::min(segs[g].len, j1 - segs[g].j0) + kTpRows - 1) / kTpRows;
         for (uint32_t t = 0; t < d; ++t)
           items[eb == 8 ? 0 : 1].push_back({nst, TpItem{(uint32_t)l, t, blk, c, chunk_seg[c], nst}});
       }
@@ -1632,9 +1655,10 @@ LC_API int lc_batch_create(const lc_commit_class* classes, uint32_t num_classes,
         L.S = acc;
         std::vector<uint64_t> Rp(L.n_max + 1);
         uint64_t accp = 0;
+        b->group.push_back(row_group(R));
         for (uint32_t j = 0; j < L.n_max; ++j) {
           Rp[j] = accp;
-          accp += row_stride(R, j, (uint32_t)eb);
+          accp += row_stride(R, j, b->group.back(), (uint32_t)eb);
         }
         Rp[L.n_max] = accp;
         L.Sp = accp;

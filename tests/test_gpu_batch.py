@@ -250,6 +250,27 @@ def test_batch_segments(mixed_classes, cls, lengths):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("cls", [0, 3])
+@pytest.mark.parametrize("lengths", [[290, 171, 108], [128, 128, 65], [300] * 32 + [235] * 4, list(range(300, 200, -3))],
+                         ids=["odd", "stage", "blocks", "dense"])
+def test_batch_row_lengths(mixed_classes, cls, lengths):
+    """Few long jobs (rows as long as their own active jobs) and many different
+    ones (one length per 64 rows): every job equals its own commitment."""
+    cl = mixed_classes[cls]
+    rng = np.random.default_rng(len(lengths))
+    dt = torch.int64 if cl["moduli"][0] is None else torch.int32
+    jobs = []
+    for n in lengths:
+        w = torch.from_numpy(rng.integers(-128, 128, (n, cl["d"])).astype(np.int8)).cuda()
+        jobs.append(CommitJob(cls, 8, n, w, torch.empty((len(cl["keys"]), 8, cl["d"]), dtype=dt, device="cuda")))
+    batch = CommitBatch([c["keys"] for c in mixed_classes], jobs, graph=False)
+    for _ in range(2):  # the second run on used buffers
+        batch.run()
+        batch.check()
+        for j in jobs:
+            assert torch.equal(j.out, one_by_one(mixed_classes, j)), j.n
+
+
 @pytest.mark.parametrize("products", [CommitBatch.PRODUCTS_TENSOR, CommitBatch.PRODUCTS_INT64])
 @pytest.mark.parametrize("kappa", [1, 2, 3, 5, 7, 9, 15, 16])
 def test_batch_row_counts(mixed_classes, kappa, products):
