@@ -1254,15 +1254,21 @@ static int slot_finish(const lc_ajtai_key* key, size_t batch, const SlotPartials
 
 // The tensor-core products write, and the finish launch reads back, 512 L bytes
 // per slot and column however few the ring elements are; the integer form writes
-// 16 L per K split.  Below one ring element per 192 slots and columns that
-// outweighs the multiply-adds (10 rows, us, tensor / integer; Goldilocks
-// d = 256: m = 24, 59 witnesses 51 / 36; m = 84, 59 65 / 61 and 64 87 / 74; m =
-// 200, 64 the same; Q_32 d = 256, m = 84, 64 60 / 46; d = 128, m = 84, 64
-// Goldilocks 53 / 49, 59 the same); from 8192 slots and columns on (d = 64, m =
-// 24: 64 witnesses padded to 128 27 / 24, 59 the same).
+// 16 L per K split and its multiply-adds grow with m.  So the two meet at an m of
+// their own once the columns fill the SMs, higher for more rows and for narrow
+// elements (us, tensor / integer, int8 digits): Goldilocks d = 256, 1024
+// witnesses, 16 rows m = 128 779 / 729, 170 878 / 935, 2 rows m = 84 506 / 454,
+// 128 605 / 665; d = 64, 4096 witnesses, 10 rows m = 128 517 / 491, 170 552 / 631;
+// Q_32 d = 128, 1024 witnesses, 10 rows m = 256 291 / 283, 400 375 / 414, 2 rows m =
+// 170 202 / 197, 256 247 / 270.  Fewer columns leave the integer form with less to
+// split: one ring element per 192 slots and columns (10 rows; Goldilocks d = 256:
+// m = 24, 59 witnesses 51 / 36; m = 84, 59 65 / 61 and 64 87 / 74; Q_32 d = 256,
+// m = 84, 64 60 / 46; d = 128, m = 84, 64 Goldilocks 53 / 49, 59 the same), from
+// 8192 slots and columns on (d = 64, m = 24: 64 witnesses padded to 128 27 / 24,
+// 59 the same).
 static bool tensor_products(const lc_ajtai_key* key, uint32_t b_pad) {
-  const uint64_t cols = (uint64_t)key->n * b_pad;
-  return key->slot_products == LC_PRODUCTS_TENSOR && !(cols >= 8192 && (uint64_t)key->m * 192 <= cols);
+  const uint64_t cols = (uint64_t)key->n * b_pad, few = (85 + 4 * (uint64_t)key->k) * (key->wide ? 1 : 2);
+  return key->slot_products == LC_PRODUCTS_TENSOR && !(cols >= 8192 && key->m <= std::min(cols / 192, few));
 }
 
 template <class E>

@@ -266,6 +266,40 @@ def test_key_destroyed_while_its_commit_runs():
         assert np.array_equal(out[idx].cpu().numpy().view(np.uint64), oracle_gl_commit(A, kappa, m, W[idx]))
 
 
+@pytest.mark.parametrize("log_d,kappa,m,batch", [(8, 5, 105, 129), (8, 5, 106, 129), (6, 5, 105, 513), (6, 5, 106, 513),
+                                                 (7, 16, 149, 257), (7, 16, 150, 257)])
+def test_goldilocks_few_ring_elements_many_columns(log_d, kappa, m, batch):
+    """Both sides of the line where many columns fill the SMs with either form."""
+    d = 1 << log_d
+    A, key = gl_key(kappa, m, d=d, seed=m)
+    W = synth.synth_i8(14, batch, batch * m * d).reshape(batch, m, d)
+    got = key.commit(W)
+    idx = [0, 1, batch // 2, batch - 1]
+    assert np.array_equal(got[idx], oracle_gl_commit(A, kappa, m, W[idx], d=d))
+
+
+def test_large_batches_take_the_faster_products():
+    """512 witnesses of 600 ring elements, d = 256: far above the ring elements
+    where the integer products stop being faster, however many columns there are."""
+    kappa, m, d, batch = 16, 600, 256, 512
+    key = gl_key(kappa, m, d=d, seed=1)[1]
+    w = torch.randint(-128, 128, (batch, m, d), dtype=torch.int8, device="cuda")
+    ms, outs = {}, {}
+    for mode in (GoldilocksAjtaiKey.PRODUCTS_INT64, GoldilocksAjtaiKey.PRODUCTS_TENSOR):
+        key.slot_products = mode
+        key.commit(w)
+        ms[mode] = float("inf")
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            outs[mode] = key.commit(w)
+            b.record()
+            b.synchronize()
+            ms[mode] = min(ms[mode], a.elapsed_time(b))
+    assert torch.equal(outs[GoldilocksAjtaiKey.PRODUCTS_INT64], outs[GoldilocksAjtaiKey.PRODUCTS_TENSOR])
+    assert ms[GoldilocksAjtaiKey.PRODUCTS_TENSOR] < 0.8 * ms[GoldilocksAjtaiKey.PRODUCTS_INT64], ms
+
+
 def test_goldilocks_config3_full_batch():
     """kappa=16, 2^16 witness elements, 128 int8 witnesses (the bench workload):
     every commitment of the batch checked against the oracle."""
