@@ -128,3 +128,36 @@ def test_word_fold_is_congruent_and_in_range():
     for d in cases:
         d = [int(x) for x in d]
         assert fold_words(d) % P == sum(x << (8 * l) for l, x in enumerate(d)) % P, d
+
+
+def test_word_fold_corrects_rarely():
+    """``gl_fold_limbs8`` looks at the top bits of lB and of the high word: they
+    differ for every sum that wraps, seldom otherwise, and not for zeros or the
+    transforms of small constants."""
+    rng = np.random.default_rng(14)
+
+    def words(d):
+        p = [d[2 * i] + 256 * d[2 * i + 1] for i in range(4)]
+        a, b = 65536 * p[1] + p[0], 65536 * p[3] + p[2]
+        hb, lb = b >> 32, b & 0xFFFFFFFF
+        s = ((a - hb) >> 32) + hb
+        hi = (lb + s) & 0xFFFFFFFF
+        return lb + s != hi, (hi ^ lb) >> 31 == 1  # wraps, looked at
+
+    assert words([0] * 8) == (False, False)
+    for c in range(128):
+        assert words([c] + [0] * 7) == (False, False)
+    lim, taken = 64 * 128 * 255, 0
+    small = rng.integers(-3, 4, size=(20000, 8))
+    small[:, :4] = rng.integers(-lim, lim + 1, size=(20000, 4))
+    wraps = 0
+    for d in small.tolist():
+        w, t = words(d)
+        assert t or not w
+        wraps += w
+    assert wraps  # the case is there
+    for d in rng.integers(-lim, lim + 1, size=(20000, 8)).tolist():
+        w, t = words(d)
+        assert t or not w
+        taken += t
+    assert taken < 20

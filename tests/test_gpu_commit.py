@@ -300,6 +300,45 @@ def test_large_batches_take_the_faster_products():
     assert ms[GoldilocksAjtaiKey.PRODUCTS_TENSOR] < 0.8 * ms[GoldilocksAjtaiKey.PRODUCTS_INT64], ms
 
 
+@pytest.mark.parametrize("batch,m,signed", [(65, 515, True), (127, 512, False), (129, 300, True), (255, 257, False),
+                                            (128, 513, False)])
+def test_goldilocks_witness_tiles_of_part_batches(batch, m, signed):
+    """d = 64 digits on the tensor cores: a last tile of fewer than 128 witnesses
+    after full ones and alone, extreme digits."""
+    kappa, d = 2, 64
+    A, key = gl_key(kappa, m, seed=m)
+    W = synth.synth_i8(17, batch, batch * m * d).reshape(batch, m, d)
+    W[:, ::7] = -128
+    if not signed:
+        W = W.view(np.uint8)
+    got = key.commit(torch.from_numpy(W).cuda()).cpu().numpy().view(np.uint64)
+    assert np.array_equal(got, oracle_gl_commit(A, kappa, m, W if signed else W.astype(np.uint64)))
+
+
+@pytest.mark.parametrize("kind", ["part", "zeros"])
+def test_zero_witnesses_cost_no_more(kind):
+    """127 witnesses, and 128 of which a quarter of the ring elements are zero, are
+    less work than 128 full ones, and may not take longer."""
+    kappa, m, d = 1, 32768, 64
+    key = gl_key(kappa, m, seed=1)[1]
+    w = torch.randint(-128, 128, (128, m, d), dtype=torch.int8, device="cuda")
+    other = w[:127] if kind == "part" else w.clone()
+    if kind == "zeros":
+        other[::4] = 0
+    ms = []
+    for x in (w, other):
+        key.commit(x)
+        ms.append(float("inf"))
+        for _ in range(10):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            key.commit(x)
+            b.record()
+            b.synchronize()
+            ms[-1] = min(ms[-1], a.elapsed_time(b))
+    assert ms[1] <= 1.05 * ms[0], ms
+
+
 def test_goldilocks_config3_full_batch():
     """kappa=16, 2^16 witness elements, 128 int8 witnesses (the bench workload):
     every commitment of the batch checked against the oracle."""
