@@ -128,7 +128,23 @@ __global__ void __launch_bounds__(NT)
   const uint32_t j0 = blockIdx.x * JB;
   const uint32_t b0 = blockIdx.y * BB;
   for (int i = threadIdx.x; i < G::fwd_entries(); i += NT) tw[i] = twg[i];
-  if (sizeof(S) == 1 && (reinterpret_cast<uintptr_t>(w) & 3) == 0) {
+  if (sizeof(S) == 1 && sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(w) & 15) == 0) {
+    // sixteen digits per load; four at a time, as below, take 90 us instead of 68
+    // (d = 128, 300 ring elements of 803 witnesses) and 501 instead of 452 (d = 64,
+    // 8000 of 300), but 161 instead of 170 for 8-byte values (d = 128, 700 of 256)
+    constexpr int CH = N / 16;
+    for (int e = threadIdx.x; e < PP * CH; e += NT) {
+      const int pp = e / CH, k = e % CH;
+      const int jj = pp / BB, b = pp % BB;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (b0 + b < batch && j0 + jj < m)
+        v = *reinterpret_cast<const uint4*>(w + ((size_t)(b0 + b) * m + j0 + jj) * N + (size_t)k * 16);
+      const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+      T* dst = slots + pp * SS + 16 * k;
+#pragma unroll
+      for (int u = 0; u < 16; ++u) dst[u] = to_residue<T, S>((S)(x[u / 4] >> (8 * (u % 4))), q);
+    }
+  } else if (sizeof(S) == 1 && (reinterpret_cast<uintptr_t>(w) & 3) == 0) {
     // four digits per load; lane l stores digit (u + l / 8) mod 4 in step u, so
     // that a warp's 32 stores (stride 4) fall on 32 banks
     const uint32_t rot = threadIdx.x >> 3;

@@ -11,6 +11,7 @@ import numpy as np
 import pytest
 
 import oracle
+from lzx_b200.batch import U32AjtaiKey
 from lzx_b200 import (AjtaiCommitment, AjtaiError, AjtaiParams, AjtaiPublicKey, GoldilocksAjtaiKey,
                       Modulus32, RingConfig, RingElement, _lib, sample_small_secret, synth)
 
@@ -337,6 +338,27 @@ def test_zero_witnesses_cost_no_more(kind):
             b.synchronize()
             ms[-1] = min(ms[-1], a.elapsed_time(b))
     assert ms[1] <= 1.05 * ms[0], ms
+
+
+@pytest.mark.parametrize("offset", [0, 4, 1])
+@pytest.mark.parametrize("log_d,m,batch", [(6, 700, 70), (7, 257, 20), (8, 90, 9)])
+def test_u32_digit_loads(log_d, m, batch, offset):
+    """Digits of 32-bit rings by 16-byte, 4-byte and single loads (the base's alignment)."""
+    kappa, d = 3, 1 << log_d
+    q = Modulus32.Q_32.q
+    A = synth.synth_mod32(3, 1, q, kappa * m * d)
+    key = U32AjtaiKey(Modulus32.Q_32, log_d, kappa, m, A.reshape(kappa, m, d))
+    W = synth.synth_i8(18, batch, batch * m * d).reshape(batch, m, d)
+    buf = torch.empty(W.size + 16, dtype=torch.int8, device="cuda")
+    w = buf[offset:offset + W.size].view(batch, m, d)
+    w.copy_(torch.from_numpy(W))
+    assert w.data_ptr() % 16 == offset
+    got = key.commit(w).cpu().numpy().view(np.uint32)
+    t = q32_tables(log_d)
+    a_ntt = t.forward_batch(A.reshape(-1, d))
+    for b in (0, batch - 1):
+        s = (W[b].astype(np.int64) % q).astype(np.uint32)
+        assert np.array_equal(got[b], oracle.ajtai32_commit(t, a_ntt, kappa, m, s))
 
 
 def test_goldilocks_config3_full_batch():
