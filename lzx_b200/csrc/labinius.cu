@@ -24,6 +24,8 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <map>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <vector>
@@ -65,7 +67,6 @@ struct LbLimb {
   uint32_t q, quad;
   uint32_t z6, z6s, om, oms;
   uint32_t tw[kLbTw], tws[kLbTw], tw2[kLbTw], tw2s[kLbTw];  // zeta, zeta^2 per (level, subring)
-  uint32_t leaf[kLbQSlots];                                // quadratic leaves: psi'^QUAD_SLOT_EXP[j]
   uint32_t dtw[4][kLbN162];                                // decomposition factors
   uint32_t i_root, inv2;
   // per leaf of the tensor-core form: its node g_j, slots (first | second << 16) and w_j
@@ -81,6 +82,11 @@ struct LbMaps {
 
 __constant__ LbMaps c_lb_maps;
 
+constexpr int kLbMaxLimbs = 7;
+// one prime's tables on the device: its constants, then its transform matrices
+// [tile][byte limb][128 x 352]
+constexpr size_t kLbOffImg = (sizeof(LbLimb) + 255) / 256 * 256;
+
 }  // namespace lc
 
 struct lc_lb_key {
@@ -89,11 +95,10 @@ struct lc_lb_key {
   std::vector<uint16_t> primes;
   std::vector<int16_t> a_host;  // centered rows [limbs][nr][648]
   uint32_t* d_a = nullptr;      // canonical rows by leaf [limbs][nr][324]: first slot | second << 16
-  lc::LbLimb* d_limb = nullptr;
-  uint8_t* d_img = nullptr;     // transform matrices [limbs][tile][byte limb][128 x 352]
+  const lc::LbLimb* limb[lc::kLbMaxLimbs] = {};  // the primes' tables (device), shared by keys
   uint32_t* d_sums = nullptr;   // column sums [limbs][r][648], zero between calls
   size_t sums_bytes = 0;
-  uint32_t* d_err = nullptr;
+  uint32_t* d_err = nullptr;    // after the rows
   uint64_t* d_in = nullptr;  // host-API staging
   size_t in_bytes = 0;
   void* d_out = nullptr;
@@ -208,7 +213,6 @@ static void build_limb(uint32_t q, LbLimb& L) {
   }
   L.inv2 = (uint32_t)lb_pow(2, q - 2, q);
   if (quad) {
-    for (int j = 0; j < kLbQSlots; ++j) L.leaf[j] = (uint32_t)lb_pow(psi, sub_exp(true, 6, j), q);
     for (int s = 0; s < kLbN162; ++s)  // inv2 * psi'^{-v}, ring.rs:248-262
       L.dtw[0][s] = (uint32_t)((uint64_t)L.inv2 * lb_pow(psi, (kLbCondQ - pow3[s]) % kLbCondQ, q) % q);
   } else {
@@ -344,9 +348,9 @@ LC_D void lb_transform(uint32_t* v, const LbTw& T, const LbLimb& L, uint32_t lan
 // 0 or 2^s, so the matrix entry of coefficient y there is g^y 2^-s mod q.
 // Element h of a parity has the words 5h .. 5h + 4 and holds the coefficients
 // y = 2 m + h (m its bit); K step 10 has both elements' bits 160 and 161.
-__global__ void __launch_bounds__(256) lb_image_kernel(const LbLimb* limbs, uint8_t* img) {
+__global__ void __launch_bounds__(256) lb_image_kernel(const LbLimb* limb, uint8_t* img) {
   const uint32_t e = blockIdx.x * 256 + threadIdx.x;  // position in one byte limb's image
-  const LbLimb& L = limbs[blockIdx.z];
+  const LbLimb& L = *limb;
   const uint32_t q = L.q, kpos = e / 2048 * 16 + e % 16, row = e / 16 % 128;
   const uint32_t wd = kpos / 32, s = kpos / 4 % 8, b = kpos % 4;
   const uint32_t h = wd < 10 ? wd / 5 : b, m = wd < 10 ? 32 * (wd % 5) + 8 * b + s : 160 + s;
@@ -360,7 +364,7 @@ __global__ void __launch_bounds__(256) lb_image_kernel(const LbLimb* limbs, uint
     }
     for (uint32_t t = 0; t < s; ++t) v = (v & 1 ? v + q : v) / 2;
   }
-  uint8_t* dst = img + ((size_t)blockIdx.z * kLbTiles + blockIdx.y) * 2 * kLbImg + e;
+  uint8_t* dst = img + (size_t)blockIdx.y * 2 * kLbImg + e;
   dst[0] = (uint8_t)v;
   dst[kLbImg] = (uint8_t)(v >> 8);
 }
@@ -368,8 +372,7 @@ __global__ void __launch_bounds__(256) lb_image_kernel(const LbLimb* limbs, uint
 struct LbCommitParams {
   const uint64_t* witness;  // [r * nr][12]
   const uint32_t* a;        // [limbs][nr][324] leaf pairs
-  const LbLimb* limbs;
-  const uint8_t* img;
+  const LbLimb* limb[kLbMaxLimbs];
   uint32_t* sums;           // [limbs][r][648]
   uint32_t* batches;        // [r * nr][648] (limb 0) or null
   uint32_t* err;
@@ -599,7 +602,7 @@ __global__ void __launch_bounds__(kLbTcThreads, 1) lb_commit_kernel(const __grid
   const uint32_t rest = first ? 0 : blockIdx.x - p.runs0;
   const uint32_t lt = blockIdx.y, k = first ? 0 : 1 + rest / p.runs, per = first ? p.per0 : p.per;
   const uint32_t t0 = (first ? blockIdx.x : rest % p.runs) * per, t1 = min(p.tiles, t0 + per);
-  const LbLimb& L = p.limbs[k];
+  const LbLimb& L = *p.limb[k];
   if (tid == 0) {
     mbar_init(a_full, 1);
     for (int s = 0; s < 2; ++s) {
@@ -680,7 +683,7 @@ __global__ void __launch_bounds__(kLbTcThreads, 1) lb_commit_kernel(const __grid
       if (lane == 0) mbar_arrive(&b_full[it & 1]);
     }
   } else if (lane == 0) {
-    const uint8_t* src = p.img + ((size_t)k * kLbTiles + lt) * 2 * kLbImg;
+    const uint8_t* src = reinterpret_cast<const uint8_t*>(&L) + kLbOffImg + (size_t)lt * 2 * kLbImg;
     mbar_arrive_expect_tx(a_full, 2 * kLbImg);
     bulk_g2s(base, src, kLbImg, a_full);
     bulk_g2s(base + kLbImg, src + kLbImg, kLbImg, a_full);
@@ -722,7 +725,7 @@ LC_D int16_t lb_center(uint32_t r, uint32_t q) { return r > (q - 1) / 2 ? (int16
 
 struct LbFinishParams {
   uint32_t* sums;     // [limbs][r][648], read and zeroed for the next call
-  const LbLimb* limbs;
+  const LbLimb* limb[kLbMaxLimbs];
   uint32_t* raw;      // [limbs][r][648]
   int16_t* matrix;    // [4][r][limbs][162]
   uint32_t r, nlimbs;
@@ -731,7 +734,7 @@ struct LbFinishParams {
 __global__ void __launch_bounds__(256) lb_finish_kernel(const __grid_constant__ LbFinishParams p) {
   __shared__ uint32_t y[kLbN];
   const uint32_t c = blockIdx.x, k = blockIdx.y;
-  const LbLimb& L = p.limbs[k];
+  const LbLimb& L = *p.limb[k];
   const uint32_t q = L.q;
   uint32_t* sums = p.sums + ((size_t)k * p.r + c) * kLbN;
   for (int u = threadIdx.x; u < kLbN; u += blockDim.x) {
@@ -811,31 +814,83 @@ struct LbRng {
   uint32_t below(uint32_t n) { return (uint32_t)(((next() >> 32) * n) >> 32); }
 };
 
-static int lb_key_finish(lc_lb_key* key, const std::vector<LbLimb>& tabs) {
-  // canonical rows on the device, one word per leaf
-  std::vector<uint32_t> canon((size_t)key->limbs * key->nr * kLbLeaves);
-  for (uint32_t k = 0; k < key->limbs; ++k) {
-    const int32_t q = key->primes[k];
-    const uint32_t* ps = tabs[k].pair_slot;
-    for (size_t i = 0; i < key->nr; ++i) {
-      const int16_t* row = key->a_host.data() + ((size_t)k * key->nr + i) * kLbN;
-      uint32_t* out = canon.data() + ((size_t)k * key->nr + i) * kLbLeaves;
-      for (int j = 0; j < kLbLeaves; ++j) {
-        const int32_t x = row[ps[j] & 0xFFFF] % q, y = row[ps[j] >> 16] % q;
-        out[j] = (uint32_t)(x < 0 ? x + q : x) | (uint32_t)(y < 0 ? y + q : y) << 16;
-      }
-    }
+// The tables of a prime (host) and their copy on the current device.  They depend on
+// the prime alone, so they are made once (seven primes, 0.28 MB each per device) and
+// kept: built for every key they made a key of 32 elements and one to three limbs
+// take 0.21, 0.35 and 0.51 ms, 0.09, 0.13 and 0.18 so.
+static std::mutex g_lb_mu;
+static std::map<uint32_t, LbLimb> g_lb_tabs;                           // by prime
+static std::map<std::pair<int, uint32_t>, const LbLimb*> g_lb_device;  // by device and prime
+
+static int lb_prime(uint32_t q, const LbLimb** tab, const LbLimb** dev_tab) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return map_cuda(cudaGetLastError());
+  std::lock_guard<std::mutex> lk(g_lb_mu);
+  auto t = g_lb_tabs.find(q);
+  if (t == g_lb_tabs.end()) {
+    t = g_lb_tabs.emplace(q, LbLimb{}).first;
+    build_limb(q, t->second);
+    build_pairs(q, t->second);
   }
-  if (cudaMalloc(&key->d_a, canon.size() * 4) != cudaSuccess) {
+  *tab = &t->second;  // nodes of the map stay where they are
+  const auto d = g_lb_device.find({dev, q});
+  if (d != g_lb_device.end()) {
+    *dev_tab = d->second;
+    return LC_OK;
+  }
+  uint8_t* p = nullptr;
+  if (cudaMalloc(&p, kLbOffImg + (size_t)kLbTiles * 2 * kLbImg) != cudaSuccess) {
     cudaGetLastError();
     return LC_ERR_OUT_OF_MEMORY;
   }
-  return map_cuda(cudaMemcpy(key->d_a, canon.data(), canon.size() * 4, cudaMemcpyHostToDevice));
+  cudaError_t e = cudaMemcpy(p, &t->second, sizeof(LbLimb), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    lb_image_kernel<<<dim3(kLbImg / 256, kLbTiles), 256>>>(reinterpret_cast<const LbLimb*>(p), p + kLbOffImg);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // any stream may use it from here on
+  if (e != cudaSuccess) {
+    cudaFree(p);
+    return map_cuda(e);
+  }
+  *dev_tab = g_lb_device[{dev, q}] = reinterpret_cast<const LbLimb*>(p);
+  return LC_OK;
 }
 
-static int lb_key_alloc(size_t len_f162, const uint16_t* primes, uint32_t limbs, std::vector<LbLimb>& tabs,
+// Canonical rows on the device, one word per leaf, and the error word.
+static int lb_key_finish(lc_lb_key* key, const std::vector<const LbLimb*>& tabs) {
+  const size_t words = (size_t)key->limbs * key->nr * kLbLeaves;
+  std::unique_ptr<uint32_t[]> canon(new (std::nothrow) uint32_t[words + 4]);
+  if (!canon) return LC_ERR_OUT_OF_MEMORY;
+  std::fill_n(canon.get() + words, 4, 0u);
+  for (uint32_t k = 0; k < key->limbs; ++k) {
+    const int32_t q = key->primes[k];
+    const uint32_t* ps = tabs[k]->pair_slot;
+    const auto residue = [q](int32_t x) -> uint32_t {
+      x += (x >> 31) & q;
+      if ((uint32_t)x >= (uint32_t)q) {  // not a centered residue
+        x %= q;
+        x += (x >> 31) & q;
+      }
+      return (uint32_t)x;
+    };
+    for (size_t i = 0; i < key->nr; ++i) {
+      const int16_t* row = key->a_host.data() + ((size_t)k * key->nr + i) * kLbN;
+      uint32_t* out = canon.get() + ((size_t)k * key->nr + i) * kLbLeaves;
+      for (int j = 0; j < kLbLeaves; ++j) out[j] = residue(row[ps[j] & 0xFFFF]) | residue(row[ps[j] >> 16]) << 16;
+    }
+  }
+  if (cudaMalloc(&key->d_a, (words + 4) * 4) != cudaSuccess) {
+    cudaGetLastError();
+    return LC_ERR_OUT_OF_MEMORY;
+  }
+  key->d_err = key->d_a + words;
+  return map_cuda(cudaMemcpy(key->d_a, canon.get(), (words + 4) * 4, cudaMemcpyHostToDevice));
+}
+
+static int lb_key_alloc(size_t len_f162, const uint16_t* primes, uint32_t limbs, std::vector<const LbLimb*>& tabs,
                         lc_lb_key** out) {
-  if (!out || !primes || limbs == 0 || limbs > 7) return LC_ERR_INVALID_ARGUMENT;
+  if (!out || !primes || limbs == 0 || limbs > (uint32_t)kLbMaxLimbs) return LC_ERR_INVALID_ARGUMENT;
   *out = nullptr;
   // key.rs:96-100: len_f162 > 0 and a multiple of 4; no limb listed twice (:102-106)
   if (len_f162 == 0 || len_f162 % 4 || len_f162 / 4 > (1u << 16)) return LC_ERR_INVALID_ARGUMENT;  // nr <= 2^16 keeps the u64 sums exact
@@ -854,26 +909,7 @@ static int lb_key_alloc(size_t len_f162, const uint16_t* primes, uint32_t limbs,
   key->limbs = limbs;
   key->primes.assign(primes, primes + limbs);
   tabs.resize(limbs);
-  // transform matrices, then the error word (zero)
-  const size_t per = (size_t)kLbTiles * 2 * kLbImg;
-  for (uint32_t k = 0; k < limbs; ++k) {
-    build_limb(primes[k], tabs[k]);
-    build_pairs(primes[k], tabs[k]);
-  }
-  if (cudaMalloc(&key->d_limb, sizeof(LbLimb) * limbs) != cudaSuccess ||
-      cudaMalloc(&key->d_img, limbs * per + 16) != cudaSuccess) {
-    cudaGetLastError();
-    lc_lb_key_destroy(key);
-    return LC_ERR_OUT_OF_MEMORY;
-  }
-  key->d_err = reinterpret_cast<uint32_t*>(key->d_img + limbs * per);
-  rc = map_cuda(cudaMemcpy(key->d_limb, tabs.data(), sizeof(LbLimb) * limbs, cudaMemcpyHostToDevice));
-  if (!rc) {
-    lb_image_kernel<<<dim3(kLbImg / 256, kLbTiles, limbs), 256>>>(key->d_limb, key->d_img);
-    rc = map_cuda(cudaGetLastError());
-  }
-  if (!rc) rc = map_cuda(cudaMemset(key->d_err, 0, 4));  // after the kernel, on the same stream
-  if (!rc) rc = map_cuda(cudaStreamSynchronize(nullptr));
+  for (uint32_t k = 0; k < limbs && !rc; ++k) rc = lb_prime(primes[k], &tabs[k], &key->limb[k]);
   if (rc) {
     lc_lb_key_destroy(key);
     return rc;
@@ -904,7 +940,7 @@ LC_API int lc_lb_key_create(size_t len_f162, const uint16_t* primes, uint32_t li
   using namespace lc;
   if (!a) return LC_ERR_INVALID_ARGUMENT;
   lc_lb_key* key = nullptr;
-  std::vector<LbLimb> tabs;
+  std::vector<const LbLimb*> tabs;
   int rc = lb_key_alloc(len_f162, primes, limbs, tabs, &key);
   if (rc) return rc;
   key->a_host.assign(a, a + (size_t)limbs * key->nr * kLbN);
@@ -924,7 +960,7 @@ LC_API int lc_lb_key_random(size_t len_f162, uint64_t seed, const uint16_t* prim
                             lc_lb_key** out) {
   using namespace lc;
   lc_lb_key* key = nullptr;
-  std::vector<LbLimb> tabs;
+  std::vector<const LbLimb*> tabs;
   int rc = lb_key_alloc(len_f162, primes, limbs, tabs, &key);
   if (rc) return rc;
   const size_t per = key->nr * kLbN;
@@ -941,7 +977,7 @@ LC_API int lc_lb_key_random(size_t len_f162, uint64_t seed, const uint16_t* prim
     LbRng rng(seed ^ (0x9E3779B9ull * (uint64_t)(k + 1)));
     for (size_t e = 0; e < per; ++e) coeffs[e] = rng.below(q);
     rc = map_cuda(cudaMemcpy(d_buf, coeffs.data(), per * 4, cudaMemcpyHostToDevice));
-    if (!rc) rc = lb_ntt_run(key->d_limb + k, d_buf, d_buf + per, key->nr, nullptr);
+    if (!rc) rc = lb_ntt_run(key->limb[k], d_buf, d_buf + per, key->nr, nullptr);
     if (!rc) rc = map_cuda(cudaMemcpy(t.data(), d_buf + per, per * 4, cudaMemcpyDeviceToHost));
     const int32_t half = (int32_t)((q - 1) / 2);
     for (size_t e = 0; e < per && !rc; ++e)
@@ -960,8 +996,6 @@ LC_API int lc_lb_key_random(size_t len_f162, uint64_t seed, const uint16_t* prim
 LC_API void lc_lb_key_destroy(lc_lb_key* key) {
   if (!key) return;
   cudaFree(key->d_a);
-  cudaFree(key->d_limb);
-  cudaFree(key->d_img);
   cudaFree(key->d_sums);
   cudaFree(key->d_in);
   cudaFree(key->d_out);
@@ -981,7 +1015,7 @@ LC_API int lc_lb_ntt(const lc_lb_key* key, uint32_t limb, const uint32_t* in, ui
                      lc_stream stream) {
   using namespace lc;
   if (!key || limb >= key->limbs || ((!in || !out) && count)) return LC_ERR_INVALID_ARGUMENT;
-  return lb_ntt_run(key->d_limb + limb, in, out, count, (cudaStream_t)stream);
+  return lb_ntt_run(key->limb[limb], in, out, count, (cudaStream_t)stream);
 }
 
 LC_API int lc_lb_commit(lc_lb_key* key, const uint64_t* witness, uint32_t r, uint32_t* raw, int16_t* matrix,
@@ -1003,8 +1037,7 @@ LC_API int lc_lb_commit(lc_lb_key* key, const uint64_t* witness, uint32_t r, uin
   LbCommitParams p{};
   p.witness = witness;
   p.a = key->d_a;
-  p.limbs = key->d_limb;
-  p.img = key->d_img;
+  std::copy(key->limb, key->limb + kLbMaxLimbs, p.limb);
   p.sums = key->d_sums;
   p.batches = batches;
   p.err = key->d_err;
@@ -1025,7 +1058,8 @@ LC_API int lc_lb_commit(lc_lb_key* key, const uint64_t* witness, uint32_t r, uin
   lb_commit_kernel<<<dim3(p.runs0 + p.runs * (key->limbs - 1), kLbTiles), kLbTcThreads, kLbSmem, st>>>(p);
   int rc = map_cuda(cudaGetLastError());
   if (rc) return rc;
-  LbFinishParams f{key->d_sums, key->d_limb, raw, matrix, r, key->limbs};
+  LbFinishParams f{key->d_sums, {}, raw, matrix, r, key->limbs};
+  std::copy(key->limb, key->limb + kLbMaxLimbs, f.limb);
   lb_finish_kernel<<<dim3(r, key->limbs), 256, 0, st>>>(f);
   return map_cuda(cudaGetLastError());
 }

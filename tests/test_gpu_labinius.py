@@ -129,3 +129,36 @@ def test_argument_errors():
         key.commit(w, 3)  # r must be a power of two >= 2
     with pytest.raises(_lib.LatticeCudaError):
         key.commit(w[:8], 1)
+
+
+def test_keys_share_the_primes_tables():
+    """The transform matrices depend on the prime alone: a key does not hold its own."""
+    limbs = [Modulus.Q3889_FS_S, Modulus.Q2917_Q_S, Modulus.Q9721_FS_S]
+    keys = [CommitmentKey.random(32, 1, limbs[0], limbs[1:])]
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    keys += [CommitmentKey.random(32, seed, limbs[0], limbs[1:]) for seed in range(2, 66)]
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] < 8 << 20  # 64 keys; 0.8 MB of tables each
+    w = random_witness(4 * 32, 3)
+    primes = [m.prime() for m in limbs]
+    for key in (keys[0], keys[-1]):
+        raw, mat, bat = lb.commit(key.a, primes, 32, w, 4)
+        cm, aux = key.commit(w, 4)
+        assert np.array_equal(aux.raw, raw) and np.array_equal(cm.value, mat) and np.array_equal(aux.batches, bat)
+
+
+def test_rows_that_are_no_centered_residues():
+    """Key rows are taken mod q whatever int16 they are."""
+    limbs = [Modulus.Q3889_FS_S, Modulus.Q2917_Q_S]
+    rng = np.random.default_rng(8)
+    a = rng.integers(-(1 << 15), 1 << 15, size=(2, 8, 648)).astype(np.int16)
+    a[0, 0, :4] = [-(1 << 15), (1 << 15) - 1, 3889, -3889]
+    centered = np.empty_like(a)
+    for k, m in enumerate(limbs):
+        q = m.prime()
+        c = a[k].astype(np.int64) % q
+        centered[k] = np.where(c > (q - 1) // 2, c - q, c)
+    w = random_witness(2 * 32, 9)
+    got, want = (CommitmentKey.from_rows(32, limbs, x).commit(w, 2) for x in (a, centered))
+    assert np.array_equal(got[1].raw, want[1].raw) and np.array_equal(got[0].value, want[0].value)
