@@ -9,7 +9,8 @@
 // Karatsuba (u0 + u1 X)(v0 + v1 X) mod (X^2 - gamma) between two transforms.
 //
 // GPU layout: polynomials are contiguous [count][n] u64 residues.  T = n/V
-// lanes own one polynomial, V = min(16, n) values each, in registers.  Phase 0
+// lanes own one polynomial, V = min(16, n) values each (fewer for few polynomials,
+// q50_log_v_few), in registers.  Phase 0
 // holds elements t + T r: the levels whose pairs are at least T apart.  The
 // values change hands once, through a padded copy in the warp's shared memory,
 // and phase 1 holds V consecutive elements: the remaining levels and the
@@ -49,6 +50,10 @@ struct Q50Const {
 // of the forward levels, of the inverse levels, then the leaf gammas.
 constexpr int kQ50P1 = 48, kQ50Tab = 2 * kQ50P1 + 64;
 
+// log2 of the values per lane: 16 where there are as many, and for few polynomials
+constexpr int q50_log_v(int log_n) { return log_n < 4 ? log_n : 4; }
+constexpr int q50_log_v_few(int log_n) { return (log_n + 1) / 2; }
+
 }  // namespace lc
 
 struct lc_quad50_plan {
@@ -58,7 +63,7 @@ struct lc_quad50_plan {
   // phase-0 constants: level d's block i at 2^d - 1 + i; the inverse's entry 0
   // and ninv carry the factor 2^-(levels)
   lc::Q50Const fwd0[15] = {}, inv0[15] = {}, ninv = {};
-  lc::Q50Const* d_tab = nullptr;
+  lc::Q50Const* d_tab = nullptr;  // tables of the two forms
   lc::HostPipeline staging;
 };
 
@@ -114,10 +119,11 @@ LC_D double q50_red(double x, double q, double qinv) {  // |x| < 2^53 to [-q/2, 
   return __fma_rn(-c, q, x);
 }
 
-template <int LOG_N>
+template <int LOG_N, int LV>
 struct Q50Geo {
   static constexpr int N = 1 << LOG_N;
-  static constexpr int LOG_V = LOG_N < 4 ? LOG_N : 4, V = 1 << LOG_V;
+  static constexpr int LOG_V = LV, V = 1 << LOG_V;
+  static_assert(LOG_V <= LOG_N && LOG_N <= 2 * LOG_V, "two phases");
   static constexpr int LOG_T = LOG_N - LOG_V, T = 1 << LOG_T;  // lanes per polynomial
   static constexpr int PW = 32 / T;                            // polynomials per warp
   static constexpr int WE = PW * N;                            // elements per warp (32 V)
@@ -135,9 +141,9 @@ struct Q50Geo {
 };
 
 // phase 0 of the forward transform: v[r] = element t + T r
-template <int LOG_N>
-LC_D void q50_forward0(double (&v)[Q50Geo<LOG_N>::V], const Q50Params& p) {
-  using Q = Q50Geo<LOG_N>;
+template <int LOG_N, int LV>
+LC_D void q50_forward0(double (&v)[Q50Geo<LOG_N, LV>::V], const Q50Params& p) {
+  using Q = Q50Geo<LOG_N, LV>;
 #pragma unroll
   for (int b = LOG_N - 1; b >= Q::LOW0; --b) {
     const int d = LOG_N - 1 - b, hr = 1 << (b - Q::LOG_T);
@@ -152,9 +158,9 @@ LC_D void q50_forward0(double (&v)[Q50Geo<LOG_N>::V], const Q50Params& p) {
 }
 
 // phase 1: v[r] = element V t + r
-template <int LOG_N, int B>
-LC_D void q50_forward1(double (&v)[Q50Geo<LOG_N>::V], const Q50Const* tab, uint32_t t, double q) {
-  using Q = Q50Geo<LOG_N>;
+template <int LOG_N, int LV, int B>
+LC_D void q50_forward1(double (&v)[Q50Geo<LOG_N, LV>::V], const Q50Const* tab, uint32_t t, double q) {
+  using Q = Q50Geo<LOG_N, LV>;
   if constexpr (B >= 1) {
     constexpr int hr = 1 << B;
 #pragma unroll
@@ -164,7 +170,7 @@ LC_D void q50_forward1(double (&v)[Q50Geo<LOG_N>::V], const Q50Const* tab, uint3
       v[r + hr] = __dadd_rn(v[r], -x);
       v[r] = __dadd_rn(v[r], x);
     }
-    q50_forward1<LOG_N, B - 1>(v, tab, t, q);
+    q50_forward1<LOG_N, LV, B - 1>(v, tab, t, q);
   }
 }
 
@@ -188,22 +194,22 @@ LC_D void q50_inv_pair(double& lo, double& hi, Q50Const w, const Q50Params& p) {
     lo = Q50Inv<LOG_N, B>::kReduce ? q50_red(s, p.q, p.qinv) : s;
 }
 
-template <int LOG_N, int B>
-LC_D void q50_inverse1(double (&v)[Q50Geo<LOG_N>::V], const Q50Const* tab, uint32_t t, const Q50Params& p) {
-  using Q = Q50Geo<LOG_N>;
+template <int LOG_N, int LV, int B>
+LC_D void q50_inverse1(double (&v)[Q50Geo<LOG_N, LV>::V], const Q50Const* tab, uint32_t t, const Q50Params& p) {
+  using Q = Q50Geo<LOG_N, LV>;
   if constexpr (B < Q::LOW0) {
 #pragma unroll
     for (int r = 0; r < Q::V; ++r) {
       if (r & (1 << B)) continue;
       q50_inv_pair<LOG_N, B>(v[r], v[r + (1 << B)], tab[kQ50P1 + Q::p1_off(B) + (r >> (B + 1)) * Q::T + t], p);
     }
-    q50_inverse1<LOG_N, B + 1>(v, tab, t, p);
+    q50_inverse1<LOG_N, LV, B + 1>(v, tab, t, p);
   }
 }
 
-template <int LOG_N, int B>
-LC_D void q50_inverse0(double (&v)[Q50Geo<LOG_N>::V], const Q50Params& p) {
-  using Q = Q50Geo<LOG_N>;
+template <int LOG_N, int LV, int B>
+LC_D void q50_inverse0(double (&v)[Q50Geo<LOG_N, LV>::V], const Q50Params& p) {
+  using Q = Q50Geo<LOG_N, LV>;
   if constexpr (B < LOG_N) {
     constexpr int d = LOG_N - 1 - B, hr = 1 << (B - Q::LOG_T);
 #pragma unroll
@@ -211,15 +217,15 @@ LC_D void q50_inverse0(double (&v)[Q50Geo<LOG_N>::V], const Q50Params& p) {
       if (r & hr) continue;
       q50_inv_pair<LOG_N, B>(v[r], v[r + hr], p.inv0[(1 << d) - 1 + (r >> (B + 1 - Q::LOG_T))], p);
     }
-    q50_inverse0<LOG_N, B + 1>(v, p);
+    q50_inverse0<LOG_N, LV, B + 1>(v, p);
   }
 }
 
 // u <- u (*) v slotwise, (u0 + u1 X)(v0 + v1 X) mod (X^2 - gamma_p): at most 2q
-template <int LOG_N>
-LC_D void q50_slotwise(double (&u)[Q50Geo<LOG_N>::V], double (&v)[Q50Geo<LOG_N>::V], const Q50Const* tab, uint32_t t,
+template <int LOG_N, int LV>
+LC_D void q50_slotwise(double (&u)[Q50Geo<LOG_N, LV>::V], double (&v)[Q50Geo<LOG_N, LV>::V], const Q50Const* tab, uint32_t t,
                        const Q50Params& p) {
-  using Q = Q50Geo<LOG_N>;
+  using Q = Q50Geo<LOG_N, LV>;
 #pragma unroll
   for (int s = 0; s < Q::V / 2; ++s) {
     const double u0 = q50_red(u[2 * s], p.q, p.qinv), u1 = q50_red(u[2 * s + 1], p.q, p.qinv);
@@ -239,17 +245,46 @@ LC_D void q50_slotwise(double (&u)[Q50Geo<LOG_N>::V], double (&v)[Q50Geo<LOG_N>:
 // next task into registers instead of L2 spills (1.23 ms), no prefetch: 1.17 ms.
 constexpr int kQ50Warps = 4, kQ50Ctas = 4;
 
-template <int LOG_N, int OP>
+template <int LOG_N, int LV, int OP>
 __global__ void __launch_bounds__(kQ50Warps * 32, kQ50Ctas) quad50_kernel(const __grid_constant__ Q50Params p) {
-  using Q = Q50Geo<LOG_N>;
+  using Q = Q50Geo<LOG_N, LV>;
   constexpr int V = Q::V, T = Q::T;
   constexpr bool TWO = OP == kQ50Slot || OP == kQ50Mul;
   // which layout the operands arrive and the results leave in: 0 = t + T r, 1 = V t + r
   constexpr bool IN0 = OP == kQ50Fwd || OP == kQ50Mul, OUT0 = OP == kQ50Inv_ || OP == kQ50Mul;
   __shared__ Q50Const s_tab[kQ50Tab];
   __shared__ double s_x[kQ50Warps][Q::SLOT];
-  for (int e = threadIdx.x; e < kQ50Tab; e += blockDim.x) s_tab[e] = p.tab[e];
-  __syncthreads();
+  // With fewer values per lane the tables are on their way while the first task's
+  // operands are loaded; at 16 there are no registers for that (2^20 products at n =
+  // 128 1107 us instead of 1070).
+  constexpr bool EARLY = V < 16;
+  constexpr int TAB = (kQ50Tab + kQ50Warps * 32 - 1) / (kQ50Warps * 32);
+  Q50Const pre[EARLY ? TAB : 1];
+  bool waiting = EARLY;
+  if constexpr (EARLY) {
+#pragma unroll
+    for (int e = 0; e < TAB; ++e) {
+      const int at = e * kQ50Warps * 32 + (int)threadIdx.x;
+      pre[e] = at < kQ50Tab ? p.tab[at] : Q50Const{};
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < TAB; ++e)
+      if (e * kQ50Warps * 32 + (int)threadIdx.x < kQ50Tab)
+        s_tab[e * kQ50Warps * 32 + threadIdx.x] = p.tab[e * kQ50Warps * 32 + threadIdx.x];
+    __syncthreads();
+  }
+  auto tables = [&]() {
+    waiting = false;
+    if constexpr (EARLY) {
+#pragma unroll
+      for (int e = 0; e < TAB; ++e) {
+        const int at = e * kQ50Warps * 32 + (int)threadIdx.x;
+        if (at < kQ50Tab) s_tab[at] = pre[e];
+      }
+      __syncthreads();
+    }
+  };
   const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const uint32_t t = lane % T, poly = lane / T;
   const size_t total = p.count * Q::N;
@@ -295,30 +330,31 @@ __global__ void __launch_bounds__(kQ50Warps * 32, kQ50Ctas) quad50_kernel(const 
     double u[V], v[V];
     load(p.a, u);
     if (TWO) load(p.b, v);
+    if (waiting) tables();
     if (OP == kQ50Fwd || OP == kQ50Mul) {
-      q50_forward0<LOG_N>(u, p);
+      q50_forward0<LOG_N, LV>(u, p);
       if (T > 1) {
         put(u, true);
         get(u, false);
       }
-      q50_forward1<LOG_N, Q::LOW0 - 1>(u, s_tab, t, p.q);
+      q50_forward1<LOG_N, LV, Q::LOW0 - 1>(u, s_tab, t, p.q);
     }
     if (OP == kQ50Mul) {
-      q50_forward0<LOG_N>(v, p);
+      q50_forward0<LOG_N, LV>(v, p);
       if (T > 1) {
         put(v, true);
         get(v, false);
       }
-      q50_forward1<LOG_N, Q::LOW0 - 1>(v, s_tab, t, p.q);
+      q50_forward1<LOG_N, LV, Q::LOW0 - 1>(v, s_tab, t, p.q);
     }
-    if (TWO) q50_slotwise<LOG_N>(u, v, s_tab, t, p);
+    if (TWO) q50_slotwise<LOG_N, LV>(u, v, s_tab, t, p);
     if (OP == kQ50Inv_ || OP == kQ50Mul) {
-      q50_inverse1<LOG_N, 1>(u, s_tab, t, p);
+      q50_inverse1<LOG_N, LV, 1>(u, s_tab, t, p);
       if (T > 1) {
         put(u, false);
         get(u, true);
       }
-      q50_inverse0<LOG_N, Q::LOW0>(u, p);
+      q50_inverse0<LOG_N, LV, Q::LOW0>(u, p);
     }
     if (OP == kQ50Fwd || OP == kQ50Slot || LOG_N == 1) {  // the last inverse level leaves 0.6q by itself
 #pragma unroll
@@ -338,20 +374,40 @@ __global__ void __launch_bounds__(kQ50Warps * 32, kQ50Ctas) quad50_kernel(const 
       __syncwarp();
     }
   }
+  if (waiting) tables();  // a warp without a task: the block's barrier
 }
 
-template <int LOG_N, int OP>
-static int q50_launch(const lc_quad50_plan* plan, const uint64_t* a, const uint64_t* b, uint64_t* out,
-                      size_t count, cudaStream_t st) {
-  using Q = Q50Geo<LOG_N>;
-  Q50Params p{a, b, out, count, (double)plan->q, 1.0 / (double)plan->q, plan->q, plan->d_tab, {}, {}, plan->ninv};
+template <int LOG_N, int LV, int OP>
+static int q50_launch_as(const lc_quad50_plan* plan, const uint64_t* a, const uint64_t* b, uint64_t* out, size_t count,
+                         cudaStream_t st) {
+  using Q = Q50Geo<LOG_N, LV>;
+  const Q50Const* tab = plan->d_tab + (LV == q50_log_v(LOG_N) ? 0 : kQ50Tab);
+  Q50Params p{a, b, out, count, (double)plan->q, 1.0 / (double)plan->q, plan->q, tab, {}, {}, plan->ninv};
   std::copy(plan->fwd0, plan->fwd0 + 15, p.fwd0);
   std::copy(plan->inv0, plan->inv0 + 15, p.inv0);
   const size_t tasks = (count + Q::PW - 1) / Q::PW;
   const size_t want = (tasks + kQ50Warps - 1) / kQ50Warps;
   const size_t cap = (size_t)std::max(1, device_sm_count()) * kQ50Ctas;
-  quad50_kernel<LOG_N, OP><<<(unsigned)std::min(want, cap), kQ50Warps * 32, 0, st>>>(p);
+  quad50_kernel<LOG_N, LV, OP><<<(unsigned)std::min(want, cap), kQ50Warps * 32, 0, st>>>(p);
   return map_cuda(cudaGetLastError());
+}
+
+// Few polynomials are a matter of one lane's chain of operations: up to
+// kQ50FewValues values per SM they take the fewest values per lane that two phases
+// allow (n = 128 has no other split).  Products, us in a graph, 16 values per lane /
+// fewer / one butterfly per lane and level through shared memory, which this kernel
+// replaced: 148 of n = 16 4.76 / 2.40 / 2.75, n = 32 5.34 / 3.13 / 3.03, n = 64 5.66 /
+// 2.81 / 3.27; 9472 of n = 64, past the line, 7.3 / 6.2 / 10.3.  Forward transforms:
+// 148 of n = 64 3.54 / 2.24 / 2.11, and of n = 128 3.26 against 2.64.
+constexpr size_t kQ50FewValues = 2048;
+
+template <int LOG_N, int OP>
+static int q50_launch(const lc_quad50_plan* plan, const uint64_t* a, const uint64_t* b, uint64_t* out,
+                      size_t count, cudaStream_t st) {
+  if constexpr (q50_log_v_few(LOG_N) < q50_log_v(LOG_N))
+    if (count << LOG_N <= kQ50FewValues * (size_t)std::max(1, device_sm_count()))
+      return q50_launch_as<LOG_N, q50_log_v_few(LOG_N), OP>(plan, a, b, out, count, st);
+  return q50_launch_as<LOG_N, q50_log_v(LOG_N), OP>(plan, a, b, out, count, st);
 }
 
 template <int OP>
@@ -429,41 +485,46 @@ LC_API int lc_quad50_plan_create(uint64_t q, uint32_t two_adicity, uint64_t gene
     return Q50Const{c, c / (double)q};
   };
   const uint64_t ninv = hpow(hpow(2, log_n - 1, q), q - 2, q);  // the levels' factors 1/2
-  const int log_v = std::min(4, (int)log_n), log_t = (int)log_n - log_v, v = 1 << log_v, t = 1 << log_t;
-  Q50Const tab[kQ50Tab] = {};
+  Q50Const tabs[2 * kQ50Tab] = {};
   p->ninv = constant(ninv);
-  int p1 = 0;
-  for (uint32_t d = 0; d + 1 < log_n; ++d) {  // :272-289
-    const int b = (int)log_n - 1 - (int)d;    // pair bit
-    for (uint32_t i = 0; i < (1u << d); ++i) {
-      const uint64_t e = ((2 * (uint64_t)rev_bits(i, d) + 1) << (5 - d)) % 128;
-      const uint64_t w = hpow(zeta, e, q), wi = hpow(w, q - 2, q);
-      if (b >= std::max(1, log_t)) {
-        p->fwd0[(1u << d) - 1 + i] = constant(w);
-        p->inv0[(1u << d) - 1 + i] = constant(d == 0 ? hmul(wi, ninv, q) : wi);
-      } else {  // block i = lane t's j-th, stored [j][t]
-        const int per = v >> (b + 1), at = p1 + (int)(i % per) * t + (int)(i / per);
-        tab[at] = constant(w);
-        tab[kQ50P1 + at] = constant(wi);
+  for (int few = 0; few < 2; ++few) {
+    Q50Const* tab = tabs + few * kQ50Tab;
+    const int log_v = few ? q50_log_v_few((int)log_n) : q50_log_v((int)log_n), log_t = (int)log_n - log_v;
+    const int v = 1 << log_v, t = 1 << log_t;
+    int p1 = 0;
+    for (uint32_t d = 0; d + 1 < log_n; ++d) {  // :272-289
+      const int b = (int)log_n - 1 - (int)d;    // pair bit
+      for (uint32_t i = 0; i < (1u << d); ++i) {
+        const uint64_t e = ((2 * (uint64_t)rev_bits(i, d) + 1) << (5 - d)) % 128;
+        const uint64_t w = hpow(zeta, e, q), wi = hpow(w, q - 2, q);
+        if (b >= std::max(1, log_t)) {  // the first form's entries are the second's too
+          if (few) continue;
+          p->fwd0[(1u << d) - 1 + i] = constant(w);
+          p->inv0[(1u << d) - 1 + i] = constant(d == 0 ? hmul(wi, ninv, q) : wi);
+        } else {  // block i = lane t's j-th, stored [j][t]
+          const int per = v >> (b + 1), at = p1 + (int)(i % per) * t + (int)(i / per);
+          tab[at] = constant(w);
+          tab[kQ50P1 + at] = constant(wi);
+        }
       }
+      if (b < std::max(1, log_t)) p1 += (v >> (b + 1)) * t;
     }
-    if (b < std::max(1, log_t)) p1 += (v >> (b + 1)) * t;
-  }
-  for (uint32_t s = 0; s < (1u << (log_n - 1)); ++s) {  // :291-296
-    const uint64_t e = ((2 * (uint64_t)rev_bits(s, log_n - 1) + 1) << (7 - log_n)) % 128;
-    p->gamma[s] = hpow(zeta, e, q);
-    tab[2 * kQ50P1 + (int)(s % (v / 2)) * t + (int)(s / (v / 2))] = constant(p->gamma[s]);
+    for (uint32_t s = 0; s < (1u << (log_n - 1)); ++s) {  // :291-296
+      const uint64_t e = ((2 * (uint64_t)rev_bits(s, log_n - 1) + 1) << (7 - log_n)) % 128;
+      p->gamma[s] = hpow(zeta, e, q);
+      tab[2 * kQ50P1 + (int)(s % (v / 2)) * t + (int)(s / (v / 2))] = constant(p->gamma[s]);
+    }
   }
   if (device_sm_count() <= 0) {
     delete p;
     return LC_ERR_NO_DEVICE;
   }
-  if (cudaMalloc(&p->d_tab, sizeof(tab)) != cudaSuccess) {
+  if (cudaMalloc(&p->d_tab, sizeof(tabs)) != cudaSuccess) {
     cudaGetLastError();
     delete p;
     return LC_ERR_OUT_OF_MEMORY;
   }
-  cudaError_t e = cudaMemcpy(p->d_tab, tab, sizeof(tab), cudaMemcpyHostToDevice);
+  cudaError_t e = cudaMemcpy(p->d_tab, tabs, sizeof(tabs), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(p->d_tab);
     delete p;

@@ -143,3 +143,20 @@ def test_errors():
     with pytest.raises(Mod50Error) as e:
         ring.mul(np.array([1, 2, 3], dtype=np.uint64), np.array([1, 2, 3], dtype=np.uint64))
     assert e.value.kind == Mod50Error.LengthMismatch
+
+
+@pytest.mark.parametrize("log_n", [3, 4, 5, 6])
+def test_both_forms_agree(log_n):
+    """Few polynomials take fewer values per lane than many: the same results on
+    both sides of the line, partly filled warps included."""
+    n = 1 << log_n
+    t = QuadSlotTables(Modulus50.Q_50, log_n)
+    q = Modulus50.Q_50.q
+    line = 2048 * torch.cuda.get_device_properties(0).multi_processor_count >> log_n
+    g = torch.Generator(device="cuda").manual_seed(log_n)
+    a, b = (torch.randint(0, q, (line + 3, n), dtype=torch.int64, device="cuda", generator=g) for _ in range(2))
+    a[0], b[0] = q - 1, q - 1
+    for f in (lambda x, y: t.forward(x), lambda x, y: t.inverse(x), t.slotwise_mul, t.mul):
+        many = f(a, b)  # above the line
+        for count in (1, 31, line):
+            assert torch.equal(f(a[:count].contiguous(), b[:count].contiguous()), many[:count]), count
