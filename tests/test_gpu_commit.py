@@ -361,6 +361,17 @@ def test_u32_digit_loads(log_d, m, batch, offset):
         assert np.array_equal(got[b], oracle.ajtai32_commit(t, a_ntt, kappa, m, s))
 
 
+def test_more_witness_tiles_than_a_grid_dimension():
+    """2 100 000 witnesses of one ring element: 65 625 tiles of 32 columns."""
+    kappa, m, d, batch = 1, 1, 64, 2_100_000
+    A = synth.synth_mod32(4, 1, Modulus32.Q_32.q, kappa * m * d)
+    key = U32AjtaiKey(Modulus32.Q_32, 6, kappa, m, A.reshape(kappa, m, d))
+    w = torch.randint(-128, 128, (batch, m, d), dtype=torch.int8, device="cuda")
+    got = key.commit(w)
+    for lo in (0, 65535 * 32 - 100, batch - 200):
+        assert torch.equal(got[lo:lo + 200], key.commit(w[lo:lo + 200].contiguous())), lo
+
+
 def test_goldilocks_config3_full_batch():
     """kappa=16, 2^16 witness elements, 128 int8 witnesses (the bench workload):
     every commitment of the batch checked against the oracle."""
