@@ -5,8 +5,8 @@
 // verifier that derives its key from the seed on every call paid both several
 // times per call (from_seed + one commit, k = 2, m = 2000: 940 us).
 // Freed blocks of up to 32 MiB are kept for the next key, at most 64 MiB per
-// device; they go back to the driver when an allocation fails and when the last
-// plan and key of the process is destroyed.
+// device, the newest; they go back to the driver when an allocation fails and when
+// the last plan and key of the process is destroyed.
 //
 // A key may be destroyed while its commits still run, on any stream.  Its block
 // is handed out again only after a synchronisation of the device, and that is
@@ -76,14 +76,26 @@ int block_alloc(void** p, size_t bytes) {
 void block_free(void* p, size_t bytes, int device, bool idle) {
   if (!p) return;
   const size_t size = block_size(bytes);
+  if (size > kBlockKeepMax) {
+    cudaFree(p);
+    return;
+  }
   std::lock_guard<std::mutex> lk(g_block_mu);
-  size_t kept = size;
+  g_blocks.push_back({p, size, device, idle});
+  size_t kept = 0;
   for (const KeptBlock& b : g_blocks)
     if (b.device == device) kept += b.bytes;
-  if (size <= kBlockKeepMax && kept <= kBlockKeepTotal)
-    g_blocks.push_back({p, size, device, idle});
-  else
-    cudaFree(p);
+  // the oldest make room: a list full of sizes that no key asks for any more would
+  // leave every later key to the driver
+  for (size_t i = 0; kept > kBlockKeepTotal;) {
+    if (g_blocks[i].device != device) {
+      ++i;
+      continue;
+    }
+    kept -= g_blocks[i].bytes;
+    cudaFree(g_blocks[i].p);
+    g_blocks.erase(g_blocks.begin() + (long)i);
+  }
 }
 
 void block_settle() {

@@ -116,6 +116,20 @@ BODIES = {
   CHECK(fake.syncs == 1);
   CHECK(block_alloc(&b, MiB) == LC_OK && fake.mallocs == 3);
   block_free(b, MiB, 1, true);""",
+    # a full list makes room: the oldest blocks go back, the newest are there for the next key
+    "evict": """
+  void *a[5], *b;
+  for (int i = 0; i < 5; ++i) CHECK(block_alloc(&a[i], (16 + 2 * i) * MiB) == LC_OK);
+  for (int i = 0; i < 5; ++i) block_free(a[i], (16 + 2 * i) * MiB, 0, true);  // 100 MiB, of which 64 are kept
+  CHECK(fake.frees == 3 && fake.live == 46 * MiB);
+  CHECK(block_alloc(&b, 24 * MiB) == LC_OK && b == a[4] && fake.mallocs == 5);
+  block_free(b, 24 * MiB, 0, true);
+  CHECK(block_alloc(&b, 16 * MiB) == LC_OK && fake.mallocs == 6);
+  block_free(b, 16 * MiB, 0, true);
+  CHECK(block_alloc(&b, 40 * MiB) == LC_OK);  // too large to keep: the list stays
+  long frees = fake.frees;
+  block_free(b, 40 * MiB, 0, true);
+  CHECK(fake.frees == frees + 1);""",
 }
 
 
