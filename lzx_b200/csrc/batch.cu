@@ -1309,12 +1309,12 @@ static int batch_tensor_setup(lc_batch* b) {
   std::vector<TpItem> flat;
   for (auto& v : items)
     for (auto& x : v) flat.push_back(x.second);
-  if (cudaMalloc(&b->d_amaps, nl * sizeof(CUtensorMap)) != cudaSuccess ||
-      cudaMalloc(&b->d_smaps, std::max<size_t>(1, smaps.size()) * sizeof(CUtensorMap)) != cudaSuccess ||
-      cudaMalloc(&b->d_segs, std::max<size_t>(1, segs.size()) * sizeof(TpSeg)) != cudaSuccess ||
-      cudaMalloc(&b->d_tchunk0, tchunk0.size() * 4) != cudaSuccess ||
-      cudaMalloc(&b->d_titems, std::max<size_t>(1, flat.size()) * sizeof(TpItem)) != cudaSuccess ||
-      cudaMalloc(&b->d_tpart, std::max<size_t>(256, part_elems * 4)) != cudaSuccess) {
+  if (lc::dev_malloc(&b->d_amaps, nl * sizeof(CUtensorMap)) != cudaSuccess ||
+      lc::dev_malloc(&b->d_smaps, std::max<size_t>(1, smaps.size()) * sizeof(CUtensorMap)) != cudaSuccess ||
+      lc::dev_malloc(&b->d_segs, std::max<size_t>(1, segs.size()) * sizeof(TpSeg)) != cudaSuccess ||
+      lc::dev_malloc(&b->d_tchunk0, tchunk0.size() * 4) != cudaSuccess ||
+      lc::dev_malloc(&b->d_titems, std::max<size_t>(1, flat.size()) * sizeof(TpItem)) != cudaSuccess ||
+      lc::dev_malloc(&b->d_tpart, std::max<size_t>(256, part_elems * 4)) != cudaSuccess) {
     cudaGetLastError();
     return LC_ERR_OUT_OF_MEMORY;
   }
@@ -1398,7 +1398,7 @@ static int batch_tw_setup(lc_batch* b, const std::vector<uint32_t>& plan_gen) {
     if (!img) {
       std::vector<uint8_t> h;
       tw_image(gl ? kGlP : L.q, gl ? 7 : plan_gen[l], L.log_n, limbs, h);
-      if (cudaMalloc(&img, h.size()) != cudaSuccess) {
+      if (lc::dev_malloc(&img, h.size()) != cudaSuccess) {
         cudaGetLastError();
         return LC_ERR_OUT_OF_MEMORY;
       }
@@ -1422,8 +1422,8 @@ static int batch_tw_setup(lc_batch* b, const std::vector<uint32_t>& plan_gen) {
     b->lane_tw[l] = 1;
   }
   if (items.empty()) return LC_OK;
-  if (cudaMalloc(&b->d_vmaps, nl * sizeof(CUtensorMap)) != cudaSuccess ||
-      cudaMalloc(&b->d_twitems, items.size() * sizeof(TwItem)) != cudaSuccess) {
+  if (lc::dev_malloc(&b->d_vmaps, nl * sizeof(CUtensorMap)) != cudaSuccess ||
+      lc::dev_malloc(&b->d_twitems, items.size() * sizeof(TwItem)) != cudaSuccess) {
     cudaGetLastError();
     return LC_ERR_OUT_OF_MEMORY;
   }
@@ -1470,8 +1470,8 @@ static int batch_layout(lc_batch* b) {
   if (b->d_cblk) cudaFree(b->d_cblk);
   b->d_citem = nullptr;
   b->d_cblk = nullptr;
-  if (cudaMalloc(&b->d_citem, std::max<size_t>(1, citem.size()) * 8) != cudaSuccess ||
-      cudaMalloc(&b->d_cblk, std::max<size_t>(1, cblk.size())) != cudaSuccess) {
+  if (lc::dev_malloc(&b->d_citem, std::max<size_t>(1, citem.size()) * 8) != cudaSuccess ||
+      lc::dev_malloc(&b->d_cblk, std::max<size_t>(1, cblk.size())) != cudaSuccess) {
     cudaGetLastError();
     return LC_ERR_OUT_OF_MEMORY;
   }
@@ -1683,14 +1683,14 @@ LC_API int lc_batch_create(const lc_commit_class* classes, uint32_t num_classes,
   }
   // ---- device buffers
   const size_t nl = std::max<size_t>(1, b->lanes.size());
-  if (cudaMalloc(&b->d_lanes, nl * sizeof(LaneDesc)) != cudaSuccess ||
-      cudaMalloc(&b->d_subs, std::max<size_t>(1, subs.size()) * sizeof(SubJob)) != cudaSuccess ||
-      cudaMalloc(&b->d_R, (Rall.size() + 2) * 8) != cudaSuccess ||  // + slack for 16-byte copy rounding
-      cudaMalloc(&b->d_itemj, std::max<size_t>(1, itemj_all.size()) * 4) != cudaSuccess ||
-      cudaMalloc(&b->d_what, what_bytes + 256) != cudaSuccess ||  // + slack for 16-byte copy rounding
-      cudaMalloc(&b->d_partial, std::max<size_t>(256, partial_bytes)) != cudaSuccess ||
-      cudaMalloc(&b->d_counters, 4 * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc(&b->d_err, 4) != cudaSuccess) {
+  if (lc::dev_malloc(&b->d_lanes, nl * sizeof(LaneDesc)) != cudaSuccess ||
+      lc::dev_malloc(&b->d_subs, std::max<size_t>(1, subs.size()) * sizeof(SubJob)) != cudaSuccess ||
+      lc::dev_malloc(&b->d_R, (Rall.size() + 2) * 8) != cudaSuccess ||  // + slack for 16-byte copy rounding
+      lc::dev_malloc(&b->d_itemj, std::max<size_t>(1, itemj_all.size()) * 4) != cudaSuccess ||
+      lc::dev_malloc(&b->d_what, what_bytes + 256) != cudaSuccess ||  // + slack for 16-byte copy rounding
+      lc::dev_malloc(&b->d_partial, std::max<size_t>(256, partial_bytes)) != cudaSuccess ||
+      lc::dev_malloc(&b->d_counters, 4 * sizeof(unsigned long long)) != cudaSuccess ||
+      lc::dev_malloc(&b->d_err, 4) != cudaSuccess) {
     cudaGetLastError();
     batch_free(b);
     return LC_ERR_OUT_OF_MEMORY;

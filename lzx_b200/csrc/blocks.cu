@@ -5,8 +5,8 @@
 // verifier that derives its key from the seed on every call paid both several
 // times per call (from_seed + one commit, k = 2, m = 2000: 940 us).
 // Freed blocks of up to 32 MiB are kept for the next key, at most 64 MiB per
-// device, the newest; they go back to the driver when an allocation fails and when
-// the last plan and key of the process is destroyed.
+// device, the newest; they go back to the driver when an allocation of this library fails
+// and when the last plan and key of the process is destroyed.
 //
 // A key may be destroyed while its commits still run, on any stream.  Its block
 // is handed out again only after a synchronisation of the device, and that is
@@ -49,6 +49,16 @@ static void block_drain() {
   g_blocks.clear();
 }
 
+cudaError_t dev_malloc(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  std::lock_guard<std::mutex> lk(g_block_mu);
+  if (g_blocks.empty()) return e;
+  cudaGetLastError();
+  block_drain();
+  return cudaMalloc(p, bytes);
+}
+
 int block_alloc(void** p, size_t bytes) {
   const size_t size = block_size(bytes);
   int dev = 0;
@@ -57,17 +67,16 @@ int block_alloc(void** p, size_t bytes) {
     cudaGetLastError();
     return LC_ERR_CUDA;
   }
-  std::lock_guard<std::mutex> lk(g_block_mu);
-  for (size_t i = 0; i < g_blocks.size(); ++i)
-    if (g_blocks[i].bytes == size && g_blocks[i].device == dev && g_blocks[i].idle) {
-      *p = g_blocks[i].p;
-      g_blocks.erase(g_blocks.begin() + (long)i);
-      return LC_OK;
-    }
-  if (cudaMalloc(p, size) == cudaSuccess) return LC_OK;
-  cudaGetLastError();
-  block_drain();
-  if (cudaMalloc(p, size) == cudaSuccess) return LC_OK;
+  {
+    std::lock_guard<std::mutex> lk(g_block_mu);
+    for (size_t i = 0; i < g_blocks.size(); ++i)
+      if (g_blocks[i].bytes == size && g_blocks[i].device == dev && g_blocks[i].idle) {
+        *p = g_blocks[i].p;
+        g_blocks.erase(g_blocks.begin() + (long)i);
+        return LC_OK;
+      }
+  }
+  if (dev_malloc(p, size) == cudaSuccess) return LC_OK;
   cudaGetLastError();
   *p = nullptr;
   return LC_ERR_OUT_OF_MEMORY;

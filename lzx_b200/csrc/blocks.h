@@ -1,9 +1,18 @@
 // blocks.h -- device memory of keys: freed blocks are kept for the next key.
 #pragma once
 
+#include <cuda_runtime.h>
 #include <stddef.h>
 
 namespace lc {
+
+// cudaMalloc for everything this library allocates: when the driver has no more, the
+// kept blocks go back to it first.
+cudaError_t dev_malloc(void** p, size_t bytes);
+template <class T>
+cudaError_t dev_malloc(T** p, size_t bytes) {
+  return dev_malloc(reinterpret_cast<void**>(p), bytes);
+}
 
 // block_alloc hands out a kept block of the same (rounded) size that no queued
 // work uses, or driver memory.  `idle` tells block_free that nothing queued uses

@@ -946,7 +946,7 @@ static int grow(void** p, size_t* have, size_t need) {
   if (*p) cudaFree(*p);
   *p = nullptr;
   *have = 0;
-  if (cudaMalloc(p, need) != cudaSuccess) {
+  if (lc::dev_malloc(p, need) != cudaSuccess) {
     cudaGetLastError();
     return LC_ERR_OUT_OF_MEMORY;
   }
@@ -1101,7 +1101,7 @@ static int launch_mac_intt(lc_ajtai_key* key, size_t batch, uint32_t b_pad, uint
   cudaError_t e = smem_attr_once(attr_done, kern, C::SMEM);
   if (e != cudaSuccess) return map_cuda(e);
   if (!key->d_grid) {
-    if (cudaMalloc(&key->d_grid, 256) != cudaSuccess) {
+    if (lc::dev_malloc(&key->d_grid, 256) != cudaSuccess) {
       cudaGetLastError();
       return LC_ERR_OUT_OF_MEMORY;
     }
@@ -1307,7 +1307,8 @@ static int commit_core(lc_ajtai_key* key, size_t batch, uint32_t b_pad, void* ou
         rc = tc_slot_reduce(key->d_partial, sp, (uint32_t)sizeof(E), q, n, kappa, batch, key->d_chat, st);
       return rc ? rc : run_ntt(key->plan, key->d_chat, out, (size_t)batch * kappa, true, st);
     }
-    if (rc != LC_ERR_UNSUPPORTED) return rc;
+    // without memory for the limb sums the integer form's smaller partial sums may do
+    if (rc != LC_ERR_UNSUPPORTED && rc != LC_ERR_OUT_OF_MEMORY) return rc;
   }
   const bool tiled = b_pad % kBTile == 0;
   const bool quad = !tiled && b_pad % 4 == 0;

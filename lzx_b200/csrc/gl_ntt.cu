@@ -434,7 +434,7 @@ int gl_ntt_prepare(uint32_t log_n) {
   gn_split(log_n, &l1, &l2);
   const uint32_t bytes = (64u << (2 * l1)) + (64u << (2 * l2)) + (8u << log_n);
   unsigned char* d = nullptr;
-  if (cudaMalloc(&d, 2 * (size_t)bytes) != cudaSuccess) {
+  if (lc::dev_malloc(&d, 2 * (size_t)bytes) != cudaSuccess) {
     cudaGetLastError();
     return LC_ERR_OUT_OF_MEMORY;
   }

@@ -40,7 +40,7 @@ struct HostPipeline {
     }
     bytes = 0;
     for (int i = 0; i < kSlots; ++i) {
-      if (cudaMalloc(&buf[i], need) != cudaSuccess) {
+      if (lc::dev_malloc(&buf[i], need) != cudaSuccess) {
         cudaGetLastError();
         return LC_ERR_OUT_OF_MEMORY;
       }

@@ -839,7 +839,7 @@ static int lb_prime(uint32_t q, const LbLimb** tab, const LbLimb** dev_tab) {
     return LC_OK;
   }
   uint8_t* p = nullptr;
-  if (cudaMalloc(&p, kLbOffImg + (size_t)kLbTiles * 2 * kLbImg) != cudaSuccess) {
+  if (lc::dev_malloc(&p, kLbOffImg + (size_t)kLbTiles * 2 * kLbImg) != cudaSuccess) {
     cudaGetLastError();
     return LC_ERR_OUT_OF_MEMORY;
   }
@@ -880,7 +880,7 @@ static int lb_key_finish(lc_lb_key* key, const std::vector<const LbLimb*>& tabs)
       for (int j = 0; j < kLbLeaves; ++j) out[j] = residue(row[ps[j] & 0xFFFF]) | residue(row[ps[j] >> 16]) << 16;
     }
   }
-  if (cudaMalloc(&key->d_a, (words + 4) * 4) != cudaSuccess) {
+  if (lc::dev_malloc(&key->d_a, (words + 4) * 4) != cudaSuccess) {
     cudaGetLastError();
     return LC_ERR_OUT_OF_MEMORY;
   }
@@ -923,7 +923,7 @@ static int grow(void** p, size_t* have, size_t need) {
   if (*p) cudaFree(*p);
   *p = nullptr;
   *have = 0;
-  if (cudaMalloc(p, need) != cudaSuccess) {
+  if (lc::dev_malloc(p, need) != cudaSuccess) {
     cudaGetLastError();
     return LC_ERR_OUT_OF_MEMORY;
   }
@@ -966,7 +966,7 @@ LC_API int lc_lb_key_random(size_t len_f162, uint64_t seed, const uint16_t* prim
   const size_t per = key->nr * kLbN;
   std::vector<uint32_t> coeffs(per), t(per);
   uint32_t* d_buf = nullptr;
-  if (cudaMalloc(&d_buf, per * 4 * 2) != cudaSuccess) {
+  if (lc::dev_malloc(&d_buf, per * 4 * 2) != cudaSuccess) {
     cudaGetLastError();
     lc_lb_key_destroy(key);
     return LC_ERR_OUT_OF_MEMORY;

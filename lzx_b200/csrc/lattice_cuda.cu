@@ -386,7 +386,7 @@ static int finish_plan(lc_ntt_plan* plan, const std::vector<uint64_t>& fwd_raw_a
   if (!plan->tables) return LC_ERR_OUT_OF_MEMORY;
   block_users(1);
   uint64_t* block = nullptr;
-  if (cudaGetDevice(&plan->tables->device) != cudaSuccess || cudaMalloc(&block, img.size() * 8) != cudaSuccess) {
+  if (cudaGetDevice(&plan->tables->device) != cudaSuccess || lc::dev_malloc(&block, img.size() * 8) != cudaSuccess) {
     cudaGetLastError();
     return LC_ERR_OUT_OF_MEMORY;
   }

@@ -110,7 +110,7 @@ static int partial_tables(lc_ntt_plan* plan) {
     for (uint32_t k = 0; k < n / 2; ++k, x = x * omega % q) row[n + k] = (uint32_t)x;
   }
   void* d = nullptr;
-  if (cudaMalloc(&d, t.size() * 4) != cudaSuccess) {
+  if (lc::dev_malloc(&d, t.size() * 4) != cudaSuccess) {
     cudaGetLastError();
     return LC_ERR_OUT_OF_MEMORY;
   }

@@ -326,9 +326,9 @@ LC_API int lc_fold_pipeline_create(lc_ajtai_key* key, const lc_ntt_plan* crt_pla
   f->kappa = k;
   f->use_graph = use_graph;
   const size_t coeffs = (size_t)m * 64;
-  if (cudaMalloc(&f->z, coeffs * 8) != cudaSuccess || cudaMalloc(&f->digits, coeffs * 8) != cudaSuccess ||
-      cudaMalloc(&f->commits, (size_t)8 * k * 64 * 8) != cudaSuccess ||
-      cudaMalloc(&f->crt_out, coeffs * nm * 4) != cudaSuccess ||
+  if (lc::dev_malloc(&f->z, coeffs * 8) != cudaSuccess || lc::dev_malloc(&f->digits, coeffs * 8) != cudaSuccess ||
+      lc::dev_malloc(&f->commits, (size_t)8 * k * 64 * 8) != cudaSuccess ||
+      lc::dev_malloc(&f->crt_out, coeffs * nm * 4) != cudaSuccess ||
       cudaStreamCreateWithFlags(&f->side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&f->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&f->ev_join, cudaEventDisableTiming) != cudaSuccess) {

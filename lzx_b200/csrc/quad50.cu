@@ -519,7 +519,7 @@ LC_API int lc_quad50_plan_create(uint64_t q, uint32_t two_adicity, uint64_t gene
     delete p;
     return LC_ERR_NO_DEVICE;
   }
-  if (cudaMalloc(&p->d_tab, sizeof(tabs)) != cudaSuccess) {
+  if (lc::dev_malloc(&p->d_tab, sizeof(tabs)) != cudaSuccess) {
     cudaGetLastError();
     delete p;
     return LC_ERR_OUT_OF_MEMORY;

@@ -563,7 +563,7 @@ int tc_tables_create(const uint64_t* matrix_dev, uint32_t k, uint32_t m, lc_tc_t
   t->m_pad = (m + 1) & ~1u;
   t->groups = (k + 3) / 4;
   const size_t bytes = (size_t)t->groups * 4 * t->m_pad * 8 * kTcFRow;
-  if (cudaMalloc(&t->fkey, bytes) != cudaSuccess) {
+  if (lc::dev_malloc(&t->fkey, bytes) != cudaSuccess) {
     cudaGetLastError();
     delete t;
     return LC_ERR_OUT_OF_MEMORY;
@@ -600,7 +600,7 @@ int tc_commit(lc_tc_tables* t, const void* w, bool s8, size_t batch, uint64_t* o
     if (t->partial) cudaFree(t->partial);
     t->partial = nullptr;
     t->partial_bytes = 0;
-    if (cudaMalloc(&t->partial, pbytes) != cudaSuccess) {
+    if (lc::dev_malloc(&t->partial, pbytes) != cudaSuccess) {
       cudaGetLastError();
       return LC_ERR_OUT_OF_MEMORY;
     }
@@ -672,7 +672,7 @@ int tc_ntt_prepare() {
   std::vector<uint8_t> img;
   tn_build_image(img);
   uint4* d = nullptr;
-  if (cudaMalloc(&d, img.size()) != cudaSuccess) {
+  if (lc::dev_malloc(&d, img.size()) != cudaSuccess) {
     cudaGetLastError();
     return LC_ERR_OUT_OF_MEMORY;
   }
@@ -1058,7 +1058,7 @@ int tc_slot_products(const void* ahat_t, uint32_t a_m, const void* what_t, uint3
     if (*part) cudaFree(*part);
     *part = nullptr;
     *part_bytes = 0;
-    if (cudaMalloc(part, need) != cudaSuccess) {
+    if (lc::dev_malloc(part, need) != cudaSuccess) {
       cudaGetLastError();
       return LC_ERR_OUT_OF_MEMORY;
     }

@@ -130,7 +130,28 @@ BODIES = {
   long frees = fake.frees;
   block_free(b, 40 * MiB, 0, true);
   CHECK(fake.frees == frees + 1);""",
+    # an allocation that the driver refuses takes the kept blocks back first
+    "drain": """
+  void *a, *b;
+  int* c = nullptr;
+  CHECK(block_alloc(&a, 30 * MiB) == LC_OK && block_alloc(&b, 30 * MiB) == LC_OK);
+  block_free(a, 30 * MiB, 0, true);
+  block_free(b, 30 * MiB, 0, false);
+  fake.limit = 64 * MiB;
+  CHECK(dev_malloc(&c, 40 * MiB) == cudaSuccess && c && fake.live == 40 * MiB && fake.frees == 2);
+  void* d;
+  CHECK(dev_malloc(&d, 40 * MiB) == cudaErrorMemoryAllocation && fake.frees == 2);
+  CHECK(block_alloc(&d, 40 * MiB) == LC_ERR_OUT_OF_MEMORY && d == nullptr);
+  cudaFree(c);""",
 }
+
+
+def test_every_allocation_can_take_the_kept_blocks_back():
+    src = os.path.join(ROOT, "lzx_b200", "csrc")
+    for f in sorted(os.listdir(src)):
+        if f != "blocks.cu":
+            with open(os.path.join(src, f)) as fh:
+                assert "cudaMalloc(" not in fh.read(), f
 
 
 @pytest.mark.parametrize("name", list(BODIES))
