@@ -1,4 +1,4 @@
-// blocks.cu -- device blocks of keys.
+// blocks.cu -- device blocks of keys and of their scratch.
 //
 // Making a key costs a cudaMalloc and destroying it a cudaFree, each a driver
 // call of 100 us and more that also serialises with the device's other work; a
@@ -105,6 +105,21 @@ void block_free(void* p, size_t bytes, int device, bool idle) {
     cudaFree(g_blocks[i].p);
     g_blocks.erase(g_blocks.begin() + (long)i);
   }
+}
+
+int block_grow(void** p, size_t* have, size_t need) {
+  if (need <= *have) return LC_OK;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return LC_ERR_CUDA;
+  }
+  block_free(*p, *have, dev, false);  // queued work may use it
+  *p = nullptr;
+  *have = 0;
+  const int rc = block_alloc(p, need);
+  if (!rc) *have = need;
+  return rc;
 }
 
 void block_settle() {

@@ -22,6 +22,9 @@ cudaError_t dev_malloc(T** p, size_t bytes) {
 int block_alloc(void** p, size_t bytes);
 void block_free(void* p, size_t bytes, int device, bool idle);
 void block_settle();
+// A key's scratch: a block of at least `need` bytes in *p (its size in *have); a
+// smaller one there is freed.
+int block_grow(void** p, size_t* have, size_t need);
 void block_users(int delta);  // live plans and keys: the last one frees what is kept
 
 }  // namespace lc

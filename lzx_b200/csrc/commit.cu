@@ -941,19 +941,6 @@ using namespace lc;
 
 namespace lc {
 
-static int grow(void** p, size_t* have, size_t need) {
-  if (need <= *have) return LC_OK;
-  if (*p) cudaFree(*p);
-  *p = nullptr;
-  *have = 0;
-  if (lc::dev_malloc(p, need) != cudaSuccess) {
-    cudaGetLastError();
-    return LC_ERR_OUT_OF_MEMORY;
-  }
-  *have = need;
-  return LC_OK;
-}
-
 static uint32_t choose_splits(uint32_t n, uint32_t btiles, uint32_t m) {
   const int sms = device_sm_count();
   const uint32_t target = (uint32_t)std::max(1, sms * 3);  // about three CTAs per SM
@@ -1035,7 +1022,7 @@ template <class E, class S>
 static int witness_ntt_generic(lc_ajtai_key* key, const S* w, size_t batch, uint32_t b_pad,
                                cudaStream_t st) {
   const size_t count = batch * key->m * key->n;
-  int rc = grow(&key->d_wtmp, &key->wtmp_bytes, count * sizeof(E));
+  int rc = block_grow(&key->d_wtmp, &key->wtmp_bytes, count * sizeof(E));
   if (rc) return rc;
   E* tmp = reinterpret_cast<E*>(key->d_wtmp);
   const unsigned blocks = (unsigned)std::min<size_t>((count + 255) / 256, 65535);
@@ -1121,7 +1108,7 @@ static int launch_mac_intt(lc_ajtai_key* key, size_t batch, uint32_t b_pad, uint
     const size_t want = (4 * resident + per_split - 1) / per_split;
     splits = (uint32_t)std::max<size_t>(
         splits, std::min<size_t>(want, std::max<uint32_t>(1, key->m / 64)));
-    const int rc = grow(&key->d_partial, &key->partial_bytes, (size_t)splits * n * kIPad * b_pad * sizeof(E));
+    const int rc = block_grow(&key->d_partial, &key->partial_bytes, (size_t)splits * n * kIPad * b_pad * sizeof(E));
     if (rc) return rc;
   }
   size_t work1;
@@ -1302,7 +1289,7 @@ static int commit_core(lc_ajtai_key* key, size_t batch, uint32_t b_pad, void* ou
     if (rc == LC_OK) {
       rc = slot_finish<E>(key, batch, sp, out, st);
       if (rc != LC_ERR_UNSUPPORTED) return rc;
-      rc = grow(&key->d_chat, &key->chat_bytes, (size_t)batch * kappa * n * sizeof(E));
+      rc = block_grow(&key->d_chat, &key->chat_bytes, (size_t)batch * kappa * n * sizeof(E));
       if (!rc)
         rc = tc_slot_reduce(key->d_partial, sp, (uint32_t)sizeof(E), q, n, kappa, batch, key->d_chat, st);
       return rc ? rc : run_ntt(key->plan, key->d_chat, out, (size_t)batch * kappa, true, st);
@@ -1323,9 +1310,9 @@ static int commit_core(lc_ajtai_key* key, size_t batch, uint32_t b_pad, void* ou
       tiled ? choose_splits(n, btiles, m)
             : (uint32_t)std::max<size_t>(
                   1, std::min<size_t>(std::max<size_t>(1, m / 32), want / std::max<size_t>(1, outs)));
-  int rc = grow(&key->d_partial, &key->partial_bytes, (size_t)splits * n * kIPad * b_pad * sizeof(E));
+  int rc = block_grow(&key->d_partial, &key->partial_bytes, (size_t)splits * n * kIPad * b_pad * sizeof(E));
   if (rc) return rc;
-  rc = grow(&key->d_chat, &key->chat_bytes, (size_t)batch * kappa * n * sizeof(E));
+  rc = block_grow(&key->d_chat, &key->chat_bytes, (size_t)batch * kappa * n * sizeof(E));
   if (rc) return rc;
   // the products, their split sums and the inverse transforms in one launch:
   // by default for the smallest batches (at most 3 witnesses), where it
@@ -1471,10 +1458,10 @@ static int commit_any(lc_ajtai_key* key, const S* w, size_t batch, void* out, cu
   uint32_t pow2 = (uint32_t)(32 / eb);
   while (pow2 < batch && pow2 < 64) pow2 *= 2;
   if (batch >= 4 && batch < 64 && tensor_products(key, pow2)) {
-    rc = grow(&key->d_what_t, &key->what_bytes, (size_t)key->n * key->m * pow2 * eb);
+    rc = block_grow(&key->d_what_t, &key->what_bytes, (size_t)key->n * key->m * pow2 * eb);
     if (rc == LC_OK) b_pad = pow2;
   }
-  if (rc) rc = grow(&key->d_what_t, &key->what_bytes, (size_t)key->n * key->m * b_pad * eb);
+  if (rc) rc = block_grow(&key->d_what_t, &key->what_bytes, (size_t)key->n * key->m * b_pad * eb);
   if (rc) return rc;
   rc = witness_ntt<S>(key, w, batch, b_pad, st);
   if (rc) return rc;
@@ -1750,9 +1737,15 @@ LC_API int lc_ajtai_key_create_ex(const lc_ntt_plan* plan, uint32_t k, uint32_t 
 
 LC_API void lc_ajtai_key_destroy(lc_ajtai_key* key) {
   if (!key) return;
-  for (void* p : {key->d_what_t, key->d_partial, key->d_chat, key->d_wtmp, (void*)key->d_grid, key->d_in, key->d_out})
-    if (p) cudaFree(p);
-  block_free(key->d_block, key->block_bytes, key->device, false);  // its commits may still run on any stream
+  // its commits may still run on any stream
+  block_free(key->d_what_t, key->what_bytes, key->device, false);
+  block_free(key->d_partial, key->partial_bytes, key->device, false);
+  block_free(key->d_chat, key->chat_bytes, key->device, false);
+  block_free(key->d_wtmp, key->wtmp_bytes, key->device, false);
+  block_free(key->d_in, key->in_bytes, key->device, false);
+  block_free(key->d_out, key->out_bytes, key->device, false);
+  block_free(key->d_block, key->block_bytes, key->device, false);
+  if (key->d_grid) cudaFree(key->d_grid);
   if (key->host_stream) cudaStreamDestroy(key->host_stream);
   if (key->h_flags) cudaFreeHost(key->h_flags);
   if (key->h_stage_in) cudaFreeHost(key->h_stage_in);
@@ -1904,8 +1897,8 @@ static int commit_host(lc_ajtai_key* key, const void* s, size_t in_elem, size_t 
   const size_t eb = key->wide ? 8 : 4;
   const size_t in_bytes = batch * key->m * key->n * in_elem;
   const size_t out_bytes = batch * key->k * key->n * eb;
-  int rc = grow(&key->d_in, &key->in_bytes, in_bytes);
-  if (!rc) rc = grow(&key->d_out, &key->out_bytes, out_bytes);
+  int rc = block_grow(&key->d_in, &key->in_bytes, in_bytes);
+  if (!rc) rc = block_grow(&key->d_out, &key->out_bytes, out_bytes);
   if (rc) return rc;
   if (!key->host_stream && cudaStreamCreateWithFlags(&key->host_stream, cudaStreamNonBlocking) != cudaSuccess)
     return map_cuda(cudaGetLastError());

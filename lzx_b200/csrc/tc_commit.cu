@@ -1054,16 +1054,8 @@ int tc_slot_products(const void* ahat_t, uint32_t a_m, const void* what_t, uint3
   const uint32_t splits = (m + jper - 1) / jper;
   if (ntiles > 65535 || splits > kSpMaxSplits) return LC_ERR_UNSUPPORTED;  // grid y; the reduction's sums
   const size_t need = (size_t)splits * n * ntiles * ncta * 128 * sizeof(int32_t);
-  if (need > *part_bytes) {
-    if (*part) cudaFree(*part);
-    *part = nullptr;
-    *part_bytes = 0;
-    if (lc::dev_malloc(part, need) != cudaSuccess) {
-      cudaGetLastError();
-      return LC_ERR_OUT_OF_MEMORY;
-    }
-    *part_bytes = need;
-  }
+  const int grown = block_grow(part, part_bytes, need);
+  if (grown) return grown;
   // A: bytes (i, la) of Ahat_T[t][j][16]; B: bytes (b, lw) of What_T[t][j][b_pad]
   const uint32_t aw = 16 * elem_bytes;
   CUtensorMap amap, wmap;

@@ -143,6 +143,23 @@ BODIES = {
   CHECK(dev_malloc(&d, 40 * MiB) == cudaErrorMemoryAllocation && fake.frees == 2);
   CHECK(block_alloc(&d, 40 * MiB) == LC_ERR_OUT_OF_MEMORY && d == nullptr);
   cudaFree(c);""",
+    # the scratch of a key goes to the next one, after a synchronisation
+    "scratch": """
+  void *a = nullptr, *b = nullptr;
+  size_t have_a = 0, have_b = 0;
+  CHECK(block_grow(&a, &have_a, 3 * MiB) == LC_OK && have_a == 3 * MiB);
+  void* was = a;
+  CHECK(block_grow(&a, &have_a, 2 * MiB) == LC_OK && a == was && have_a == 3 * MiB);
+  CHECK(block_grow(&a, &have_a, 5 * MiB) == LC_OK && a != was && have_a == 5 * MiB && fake.frees == 0 && fake.syncs == 0);
+  CHECK(block_grow(&b, &have_b, 3 * MiB) == LC_OK && b != was && fake.mallocs == 3);
+  block_free(b, have_b, 0, false);
+  block_settle();
+  b = nullptr;
+  have_b = 0;
+  CHECK(block_grow(&b, &have_b, 3 * MiB) == LC_OK && fake.mallocs == 3);
+  fake.limit = 8 * MiB;
+  CHECK(block_grow(&b, &have_b, 20 * MiB) == LC_ERR_OUT_OF_MEMORY && !b && have_b == 0);
+  block_free(a, have_a, 0, true);""",
 }
 
 
