@@ -142,16 +142,17 @@ LC_D void cp_async_wait() {
 // exact in int64 (below 2^47.1).  With hB:lB = B (hB signed) and X = A - hB,
 //   A + 2^32 B == X + 2^32 (hB + lB)   (2^64 == 2^32 - 1),
 // so the low word is X's and the high word s + lB with s = hi(X) + hB, |s| < 2^17.
-// That sum leaves [0, 2^32) by k = 1 or -1 only when it passes an end, and as |s|
-// is small the top bits of lB and of the sum's low word differ then; they also do
-// when it passes 2^31 (2^-14 of the outputs together).  Then k (2^32 - 1) is added,
-// which stays inside [0, 2^64).  Zero outputs (zero ring elements, the columns past
-// the batch) need nothing: with the test "the low word lies within 2^18 of an end"
-// they took the correction, a fifth of tc_ntt_kernel's time.
+// That sum leaves [0, 2^32) by k = 1 or -1 only when its low word lies within
+// 2^18 of the ends (2^-13 of the outputs); then k (2^32 - 1) is added, which
+// stays inside [0, 2^64).  Zeros (zero ring elements, the columns past the batch)
+// lie there too and need nothing, which the top bits of lB and of the low word
+// tell: they differ for every sum that passes an end.  Correcting zeros with the
+// rest took tc_ntt_kernel a fifth longer; asking for the top bits at once 1 % (852
+// -> 861 us at 128 witnesses of 2^16 ring elements).
 LC_D void gl_fold_limbs8(const uint32_t (&d)[8][8], uint64_t (&out)[8]) {
   uint32_t hi[8], lo[8];
   int32_t s[8];
-  uint32_t edge = 0;
+  bool edge = false;
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
     const int32_t p01 = (int32_t)d[0][u] + (int32_t)d[1][u] * 256;
@@ -165,11 +166,15 @@ LC_D void gl_fold_limbs8(const uint32_t (&d)[8][8], uint64_t (&out)[8]) {
     s[u] = (int32_t)(X >> 32) + hB;
     lo[u] = (uint32_t)X;
     hi[u] = (uint32_t)B + (uint32_t)s[u];
-    edge |= hi[u] ^ (uint32_t)B;
+    edge |= hi[u] + 0x40000u < 0x80000u;
   }
 #pragma unroll
   for (int u = 0; u < 8; ++u) out[u] = (uint64_t)hi[u] << 32 | lo[u];
-  if ((int32_t)edge < 0) {
+  if (edge) {
+    uint32_t passed = 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) passed |= hi[u] ^ (hi[u] - (uint32_t)s[u]);
+    if ((int32_t)passed >= 0) return;
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const int k = s[u] >= 0 ? (int)(hi[u] < (uint32_t)s[u]) : -(int)(hi[u] >= (uint32_t)s[u]);
