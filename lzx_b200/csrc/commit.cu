@@ -126,8 +126,7 @@ __global__ void __launch_bounds__(NT)
   Tw* tw = reinterpret_cast<Tw*>(smem_raw);
   T* slots = reinterpret_cast<T*>(smem_raw + ((G::fwd_entries() * sizeof(Tw) + 15) / 16 * 16));
   const uint32_t j0 = blockIdx.x * JB;
-  const uint32_t b0 = (blockIdx.z * gridDim.y + blockIdx.y) * BB;
-  if (b0 >= b_pad) return;
+  const uint32_t b0 = blockIdx.y * BB;
   for (int i = threadIdx.x; i < G::fwd_entries(); i += NT) tw[i] = twg[i];
   if (sizeof(S) == 1 && sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(w) & 15) == 0) {
     // sixteen digits per load; four at a time, as below, take 90 us instead of 68
@@ -960,13 +959,16 @@ static int launch_witness_cfg(const lc_ajtai_key* key, const S* w, size_t batch,
   auto kern = witness_ntt_kernel<A, S, LOG_N, LOG_V, NT, BB, JB>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return map_cuda(e);
-  // column tiles in y, and in z past its 65535
-  const unsigned tiles = (b_pad + BB - 1) / BB, rows = (tiles + 65534) / 65535;
-  dim3 grid((key->m + JB - 1) / JB, (tiles + rows - 1) / rows, rows);
   const lc_ntt_plan* plan = key->plan;
-  kern<<<grid, NT, smem, st>>>(w, dst, key->m, (uint32_t)batch, b_pad,
-                               reinterpret_cast<const typename A::Tw*>(plan->d_tw_fwd), plan->q[0],
-                               plan->qinv[0]);
+  // column tiles in y, 65535 to a launch (more only of batches above a million,
+  // whose padding BB divides; a third grid dimension took the kernel 2 of 26 us)
+  const uint32_t tiles = (b_pad + BB - 1) / BB;
+  for (uint32_t t0 = 0; t0 < tiles; t0 += 65535) {
+    const size_t b0 = (size_t)t0 * BB, left = batch > b0 ? batch - b0 : 0;
+    kern<<<dim3((key->m + JB - 1) / JB, std::min(tiles - t0, 65535u)), NT, smem, st>>>(
+        left ? w + b0 * key->m * G::N : w, dst + b0, key->m, (uint32_t)left, b_pad,
+        reinterpret_cast<const typename A::Tw*>(plan->d_tw_fwd), plan->q[0], plan->qinv[0]);
+  }
   return map_cuda(cudaGetLastError());
 }
 
