@@ -579,8 +579,8 @@ LC_D void lb_epilogue(const LbCommitParams& p, const LbLimb& L, uint32_t k, uint
 //
 // As butterflies in shared memory the transform was issue-bound: 427 us for
 // 2^16 elements and two limbs with the base limb's transform kept.  Here a tile
-// is 22 MMAs, and the epilogue is what is left: 106 us (tensor pipe 34 %, issue
-// 51 %), against 27 us for the bytes of the kept transform.  A limb whose
+// is 22 MMAs, and the epilogue is what is left: 106 us (tensor pipe 29 %, issue
+// 44 %), against 27 us for the bytes of the kept transform.  A limb whose
 // transform is not kept skips the reductions per element, so the kept one gets
 // more of the blocks (kLbStoreWeight; equal shares took 138 us).
 __global__ void __launch_bounds__(kLbTcThreads, 1) lb_commit_kernel(const __grid_constant__ LbCommitParams p) {
@@ -931,6 +931,19 @@ static int grow(void** p, size_t* have, size_t need) {
   return LC_OK;
 }
 
+// Zeros that are there when the call returns.  On the caller's stream the memset
+// would only be recorded while that stream captures, and calls outside of the graph
+// would find whatever the memory held.
+static int zero_now(void* p, size_t bytes) {
+  cudaStream_t s = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return map_cuda(e);
+  e = cudaMemsetAsync(p, 0, bytes, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaStreamDestroy(s);
+  return map_cuda(e);
+}
+
 }  // namespace lc
 
 extern "C" {
@@ -1028,8 +1041,11 @@ LC_API int lc_lb_commit(lc_lb_key* key, const uint64_t* witness, uint32_t r, uin
   const size_t sums = (size_t)key->limbs * r * kLbN * 4;
   if (sums > key->sums_bytes) {
     int rc = grow((void**)&key->d_sums, &key->sums_bytes, sums);
-    if (!rc) rc = map_cuda(cudaMemsetAsync(key->d_sums, 0, sums, st));
-    if (rc) return rc;
+    if (!rc) rc = zero_now(key->d_sums, sums);
+    if (rc) {
+      key->sums_bytes = 0;  // not zero: allocated again by the next call
+      return rc;
+    }
   }
   static std::atomic<uint64_t> attr_done{0};
   cudaError_t e = smem_attr_once(attr_done, lb_commit_kernel, kLbSmem);

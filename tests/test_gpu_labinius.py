@@ -162,3 +162,29 @@ def test_rows_that_are_no_centered_residues():
     w = random_witness(2 * 32, 9)
     got, want = (CommitmentKey.from_rows(32, limbs, x).commit(w, 2) for x in (a, centered))
     assert np.array_equal(got[1].raw, want[1].raw) and np.array_equal(got[0].value, want[0].value)
+
+
+def test_first_commit_recorded_not_run():
+    """A key whose first commitment is captured into a graph gives right results
+    outside of it, before the graph runs and after."""
+    limbs = [Modulus.Q3889_FS_S, Modulus.Q2917_Q_S]
+    key = CommitmentKey.random(64, 11, limbs[0], limbs[1:])
+    w = random_witness(16 * 64, 12)
+    raw, mat, _ = lb.commit(key.a, [m.prime() for m in limbs], 64, w, 16)
+    dev = torch.from_numpy(w.view(np.int64)).cuda()
+    other = CommitmentKey.random(64, 13, limbs[0], limbs[1:])
+    other.commit(dev, 16)  # the launches are set up
+    # memory of about the sums' size that is not zero: the rows of keys that go
+    spoilers = [CommitmentKey.random(128, seed, limbs[0], limbs[1:]) for seed in range(24)]
+    del spoilers
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="relaxed"):
+        recorded = key.commit(dev, 16)
+    for _ in range(2):
+        cm, aux = key.commit(dev, 16)
+        assert np.array_equal(np.asarray(aux.raw.cpu()).view(np.uint32), raw)
+        assert np.array_equal(np.asarray(cm.value.cpu()), mat)
+        g.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(np.asarray(recorded[1].raw.cpu()).view(np.uint32), raw)
