@@ -270,7 +270,7 @@ LC_API int lc_ajtai_key_get_fused(const lc_ajtai_key *key);
  * witness transforms, int32 sums of at most 32768 ring elements, limbs
  * recombined and reduced mod q -- whenever a witness row of the transforms
  * (limbs x padded batch) is 32, 64, 128, 256 or a multiple of 512 bytes (other
- * paddings, and keys of few ring elements for the columns, use the integer form); LC_PRODUCTS_INT64 with 160-bit integer
+ * paddings, and keys of few ring elements, use the integer form); LC_PRODUCTS_INT64 with 160-bit integer
  * multiply-accumulates on the CUDA cores.  Identical results.
  * lc_ajtai_key_get_slot_products returns the mode (-1 for a null key). */
 #define LC_PRODUCTS_INT64 0

@@ -626,7 +626,8 @@ LC_D uint32_t tw_fold(const uint32_t* x, uint32_t q, uint32_t c, int64_t off) {
 // value congruent mod p, not necessarily canonical (the products read any
 // 64-bit representative): S = A + hi(B) (2^32 - 1), |S| < 2^48.02; U = S +
 // 2^32 lo(B) = R + k 2^64 with R = U mod 2^64, k = carry - [S < 0], and the
-// value R + k (2^32 - 1) stays inside [0, 2^64) (the reasoning of tn_fold).
+// value R + k (2^32 - 1) stays inside [0, 2^64): k = 1 only when R < 2^49, k = -1
+// only when R > 2^64 - 2^49.
 LC_D uint64_t tw_fold_gl(const uint32_t* x) {
   int64_t A = (int32_t)x[0], B = (int32_t)x[4];
   A += (int64_t)(int32_t)x[1] * 256;

@@ -353,7 +353,7 @@ __global__ void tc_reduce_kernel(const int64_t* __restrict__ partial, uint64_t* 
 // (the natural-order negacyclic NTT, out[t] = w(psi^(2t+1))).  With the
 // residues V split into 8 byte limbs, D_l[r][t] = sum_c W[r][c] V_l[t][c] is
 // exact in int32 (64 * 128 * 255 < 2^21, u8 digits 64 * 255 * 255 < 2^22) and
-// What = sum_l 2^(8l) D_l (mod p) (gl_fold_limbs).  An M = 128 tile holds R consecutive ring
+// What = sum_l 2^(8l) D_l (mod p) (gl_fold_limbs8).  An M = 128 tile holds R consecutive ring
 // elements x BB witnesses (R * BB = 128; rows ordered witness fastest, one
 // 64-byte ring element each, read by a 3-D TMA view of w[b][j][64] -- x the
 // digit, y the witness, z the ring element -- with the 64-byte swizzle).  A

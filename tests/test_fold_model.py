@@ -1,7 +1,7 @@
 """CPU models of the limb folds and residue steps of the tensor-core and CRT kernels.
 
-The tensor-core witness transforms (lzx_b200/csrc/tc_commit.cu ``tn_fold``,
-lzx_b200/csrc/batch.cu ``tw_fold_gl``) turn eight signed limb sums D_l into
+The batch's tensor-core witness transforms (lzx_b200/csrc/batch.cu
+``tw_fold_gl``) turn eight signed limb sums D_l into
 one 64-bit value congruent to sum_l 2^(8l) D_l mod p (p = 2^64 - 2^32 + 1),
 not necessarily canonical: S = A + hi(B) (2^32 - 1) with A, B the sums of
 limbs 0-3 and 4-7, R = (S + 2^32 lo(B)) mod 2^64 and the result
